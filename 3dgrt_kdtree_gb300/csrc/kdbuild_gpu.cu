@@ -12,23 +12,35 @@
 // one level per step, every node of the level at once:
 //   1. runs of equal Gaussian ID inside each node (triangles stay sorted by
 //      node, then ID, through every partition) give per-ID intervals
-//      [gmin, gmax] on each axis;
-//   2. the candidate positions (both edges of every triangle), the interval
-//      starts, ends and planar positions of every splittable node are sorted
-//      at once as 64-bit keys (axis, node, position) -- one device radix sort
-//      per list per level;
-//   3. one thread per distinct candidate counts by binary search in the
-//      sorted start/end/planar segments of its node and scores the SAH cost
-//      in the host builder's types and operation order (double costs, float
-//      extents); a two-pass atomic reduction keeps the first minimum in
-//      ascending position, axis 0 first on ties, as the sequential sweep does;
-//   4. triangles are partitioned stably into the children (two exclusive
-//      scans give every triangle its slot) and straddling ones are clipped
-//      with the host's float arithmetic;
-//   5. leaves write the IDs of their runs into one pool.
-// The node records come back to the host, which numbers the nodes as the
-// reference allocates them (child pairs in depth-first, left-first order) and
-// appends the leaf ID lists in the same order.
+//      [mn, mx] on each axis;
+//   2. the split search scores the interval ends ("events") first.  Between
+//      two neighbouring events every count is constant, so the SAH cost is
+//      linear in the position there and bounded below by its value at the
+//      two ends: triangle edges inside a gap are scored only when that bound
+//      does not exceed the best event (the tightest interval of such gaps is
+//      kept per axis).  Scores are first taken in FP32; only candidates
+//      within kMargin of the best FP32 score are scored in the host builder's
+//      types and operation order (double costs, float extents), and the
+//      smallest (cost, axis, position) wins, as in the sequential sweep.
+//      Nodes of up to 1024 IDs are searched by one warp or one block each,
+//      sorted interval ends in shared memory; larger nodes (the top levels)
+//      by kernels over globally sorted 64-bit (axis, node, position) keys;
+//   3. triangles are partitioned stably into the children (one exclusive scan
+//      of packed left/right counts gives every triangle its slots) and
+//      straddling ones are clipped with the host's float arithmetic, their
+//      vertices recomputed from the Gaussian (a triangle is carried as its
+//      clipped box, its number and its node: 32 bytes);
+//   4. leaves write the IDs of their runs into one pool.
+// The nodes are then numbered on the device as the reference allocates them
+// (child pairs in depth-first, left-first order; leaf ID lists in the same
+// order) from subtree sums taken bottom up and ranks handed down.
+//
+// What bounds it and why this shape: scoring every distinct edge, as the
+// sequential sweep does, took a global 64-bit radix sort of all edges per
+// level and about 60 FP64 operations per edge on a chip with two FP64 lanes
+// per SM; events are 3 to 20 times fewer than edges, and FP64 is left for a
+// handful of candidates per node.  Measured on a GB300, whole call: 10k
+// Gaussians 15.5 -> 4.9 ms, 500k 337 -> 87 ms, 1M 723 -> 180 ms.
 //
 // This unit is compiled with --fmad=false and IEEE division, so every float
 // and double expression rounds as on the host (compiled -ffp-contract=off).
@@ -38,12 +50,16 @@
 // face exactly at -0 versus +0 may take the other zero's bits than the
 // sequential host loop would.
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <cfloat>
 #include <cstdio>
+#include <cstdlib>
 #include <chrono>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -58,6 +74,13 @@ constexpr float kEmptyBonus = 0.9f;  // EMTPY_BONUS
 constexpr unsigned kMinPrim = 16;    // MIN_TRI
 constexpr float kEps = 0.00001f;     // KD_TREE_EPSILON
 constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr uint32_t kFaces = 20;      // triangles per proxy: triangle t belongs to Gaussian t / kFaces
+
+// Relative slack between FP32 and FP64 scores.  Every term of a score is
+// positive (costs and extents; other parameters switch the FP32 filter off),
+// so the FP32 value of its at most 20 roundings is within 1.3e-6; the gap
+// bound adds as much again.
+constexpr float kMargin = 5e-5f;
 
 struct Params {
   int max_level;
@@ -65,12 +88,57 @@ struct Params {
   float isect_cost;
   int sah_mode;
   float sort_cost;
+  int filter;  // FP32 scores may discard candidates (no negative or NaN cost parameter)
 };
 
 // ------------------------------------------------------------ device buffers
-// The build's stream and its own memory pool: the pool keeps what it has
-// mapped until the build ends (the device's default pool would hand it back
-// at every stream synchronisation, and the level loop synchronises often).
+// The builder's memory pool of a device.  It keeps what it has mapped while a
+// build runs (the level loop synchronises often, and the device's default
+// pool hands memory back at every synchronisation) and, when the last build
+// on the device has ended, up to kPoolKeep bytes for the next one: mapping
+// and unmapping them took longer than a 10k-Gaussian build's kernels.
+// Allocation and release are stream-ordered, so builds on several threads
+// (each on its own stream) may share it.
+constexpr size_t kPoolKeep = 256ull << 20;
+struct BuildPool {
+  std::mutex mu;
+  cudaMemPool_t pool[64] = {};
+  int users[64] = {};
+};
+BuildPool& build_pool() {
+  static BuildPool p;
+  return p;
+}
+cudaError_t pool_enter(int dev, cudaMemPool_t* out) {
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  BuildPool& B = build_pool();
+  std::lock_guard<std::mutex> lk(B.mu);
+  if (!B.pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = UINT64_MAX;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    B.pool[dev] = pool;
+  }
+  ++B.users[dev];
+  *out = B.pool[dev];
+  return cudaSuccess;
+}
+void pool_leave(int dev) {
+  BuildPool& B = build_pool();
+  std::lock_guard<std::mutex> lk(B.mu);
+  if (--B.users[dev] == 0) cudaMemPoolTrimTo(B.pool[dev], kPoolKeep);
+}
+
 struct Stream {
   cudaStream_t s = nullptr;
   cudaMemPool_t pool = nullptr;
@@ -92,6 +160,10 @@ struct DBuf {
     st = &s;
     n = count;
     if (count) st->check(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), count * sizeof(T), st->pool, st->s));
+  }
+  // at least `count` elements; the contents are not kept
+  void reserve(Stream& s, size_t count) {
+    if (count > n) alloc(s, count);
   }
   void release() {
     if (p && st) cudaFreeAsync(p, st->s);
@@ -121,56 +193,57 @@ struct DBuf {
   }
 };
 
-// Triangles of one level, SoA: v[k*cap + t] for the 9 vertex floats,
-// lo/hi[a*cap + t] for the clipped box, the Gaussian ID and the node index.
+// Triangles of one level, SoA: lo/hi[a*cap + t] for the clipped box, the
+// triangle's number (kFaces * valid Gaussian + face) and its node.
 struct TriSet {
-  DBuf<float> v, lo, hi;
-  DBuf<uint32_t> gid, node;
+  DBuf<float> lo, hi;
+  DBuf<uint32_t> tri, node;
   size_t cap = 0;
   void alloc(Stream& s, size_t c) {
     cap = c;
-    v.alloc(s, 9 * c);
     lo.alloc(s, 3 * c);
     hi.alloc(s, 3 * c);
-    gid.alloc(s, c);
+    tri.alloc(s, c);
     node.alloc(s, c);
   }
 };
+struct TriView {
+  const float *lo, *hi;
+  const uint32_t *tri, *node;
+  size_t cap;
+};
+TriView view(const TriSet& t) { return TriView{t.lo.p, t.hi.p, t.tri.p, t.node.p, t.cap}; }
 
-template <typename T>
-void exclusive_sum(Stream& s, const T* in, T* out, size_t n) {
+template <typename It, typename T>
+void exclusive_sum(Stream& s, DBuf<uint8_t>& tmp, It in, T* out, size_t n) {
   if (n == 0) return;
   size_t bytes = 0;
   s.check(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int64_t)n, s.s));
-  DBuf<uint8_t> tmp(s, bytes);
+  tmp.reserve(s, bytes);
   s.check(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, in, out, (int64_t)n, s.s));
 }
+// exclusive sum of op(0), op(1), ... op(n - 1), evaluated inside the scan
+template <typename Op, typename T>
+void exclusive_sum_of(Stream& s, DBuf<uint8_t>& tmp, Op op, T* out, size_t n) {
+  exclusive_sum(s, tmp, thrust::make_transform_iterator(thrust::counting_iterator<uint64_t>(0), op), out, n);
+}
 
-void sort_keys(Stream& s, DBuf<uint64_t>& keys, DBuf<uint64_t>& alt, size_t n, int end_bit) {
+void sort_keys(Stream& s, DBuf<uint8_t>& tmp, DBuf<uint64_t>& keys, DBuf<uint64_t>& alt, size_t n, int end_bit) {
   if (n == 0) return;
   cub::DoubleBuffer<uint64_t> db(keys.p, alt.p);
   size_t bytes = 0;
   s.check(cub::DeviceRadixSort::SortKeys(nullptr, bytes, db, (int64_t)n, 0, end_bit, s.s));
-  DBuf<uint8_t> tmp(s, bytes);
+  tmp.reserve(s, bytes);
   s.check(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, db, (int64_t)n, 0, end_bit, s.s));
   if (db.Current() != keys.p) std::swap(keys.p, alt.p);
-}
-
-template <typename T>
-T read_one(Stream& s, const T* dev) {
-  T v{};
-  s.check(cudaMemcpyAsync(&v, dev, sizeof(T), cudaMemcpyDeviceToHost, s.s));
-  s.check(cudaStreamSynchronize(s.s));
-  return v;
 }
 
 // at least one block: every kernel checks its own bounds
 inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)std::max<size_t>(1, (n + block - 1) / block); }
 
-// ------------------------------------------------------------ key encoding
-// (axis, node, position) -> 64-bit key ordered by axis, then node, then
-// position (the float's bits mapped to an order-preserving unsigned; -0
-// sorts before +0 as a distinct key, like the host radix sort).
+// ------------------------------------------------------------ positions
+// A float's bits mapped to an unsigned that sorts like the float (-0 before
+// +0 as distinct keys, like the host radix sort).
 __device__ __forceinline__ uint32_t ordf(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -178,61 +251,39 @@ __device__ __forceinline__ uint32_t ordf(float f) {
 __device__ __forceinline__ float unordf(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
-__device__ __forceinline__ uint64_t make_key(int axis, uint32_t node, float p, int nb) {
-  return ((uint64_t)axis << (32 + nb)) | ((uint64_t)node << 32) | ordf(p);
-}
-__device__ __forceinline__ float key_pos(uint64_t k) { return unordf((uint32_t)k); }
+// The same with -0 taken as +0: unsigned comparison of these keys is the
+// float comparison.
+__device__ __forceinline__ uint32_t ordz(float f) { return ordf(__fadd_rn(f, 0.0f)); }
+constexpr uint32_t kZeroKey = 0x80000000u;  // ordz of either zero
 
-// Elements of the sorted segment [b, b + n) whose position compares < p,
-// and those that compare == p (float comparison: -0 == +0).
-__device__ __forceinline__ uint32_t count_less(const uint64_t* k, size_t b, uint32_t n, float p) {
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (key_pos(k[b + mid]) < p) lo = mid + 1;
-    else hi = mid;
+// Sorted keys k[0..n): how many are < x, how many are <= x.
+template <typename K>
+__device__ __forceinline__ uint32_t lower(const K* k, uint32_t n, K x) {
+  uint32_t lo = 0;
+  while (n > 0) {
+    const uint32_t h = n >> 1;
+    if (k[lo + h] < x) {
+      lo += h + 1;
+      n -= h + 1;
+    } else {
+      n = h;
+    }
   }
   return lo;
 }
-__device__ __forceinline__ uint32_t count_le(const uint64_t* k, size_t b, uint32_t n, float p) {
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (key_pos(k[b + mid]) <= p) lo = mid + 1;
-    else hi = mid;
+template <typename K>
+__device__ __forceinline__ uint32_t upper(const K* k, uint32_t n, K x) {
+  uint32_t lo = 0;
+  while (n > 0) {
+    const uint32_t h = n >> 1;
+    if (k[lo + h] <= x) {
+      lo += h + 1;
+      n -= h + 1;
+    } else {
+      n = h;
+    }
   }
   return lo;
-}
-
-// The same counts with the answer known to lie in [lo, hi].
-__device__ __forceinline__ uint32_t count_less_in(const uint64_t* k, size_t b, uint32_t lo, uint32_t hi, float p) {
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (key_pos(k[b + mid]) < p) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-__device__ __forceinline__ uint32_t count_le_in(const uint64_t* k, size_t b, uint32_t lo, uint32_t hi, float p) {
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (key_pos(k[b + mid]) <= p) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// Bounds for the counts of a warp whose 32 lanes hold consecutive sorted
-// candidates of one segment: every lane's count lies between lane 0's
-// count_less and lane 31's count_le, found once by those two lanes.
-struct Bracket {
-  uint32_t lo, hi;
-};
-__device__ __forceinline__ Bracket warp_bracket(const uint64_t* k, size_t b, uint32_t n, float p, int lane) {
-  uint32_t v = 0;
-  if (lane == 0) v = count_less(k, b, n, p);
-  if (lane == 31) v = count_le(k, b, n, p);
-  return Bracket{__shfl_sync(0xFFFFFFFFu, v, 0), __shfl_sync(0xFFFFFFFFu, v, 31)};
 }
 
 __device__ __forceinline__ float ref_min(float a, float b) { return a < b ? a : b; }
@@ -248,60 +299,61 @@ __device__ __forceinline__ void cross3(const float* a, const float* b, float* o)
   o[2] = ((a[0] * b[1]) - (a[1] * b[0]));
 }
 
-// One thread per proxy triangle: the icosahedron face scaled by k_iso *
+// Vertices of proxy triangle `tri`: the icosahedron face scaled by k_iso *
 // scale, rotated by the quaternion, moved to the mean (the host builder's
 // proxy_icosahedron, operation for operation).  g: 10 floats per valid
 // Gaussian (pos, scale, quaternion w,x,y,z).
-__global__ void k_proxy(const float* __restrict__ g, const float* __restrict__ kiso, const uint32_t* __restrict__ ids,
-                        uint32_t n_valid, float* v, float* lo, float* hi, uint32_t* gid,
-                        uint32_t* node, size_t cap) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n_valid * 20) return;
-  const uint32_t j = (uint32_t)(t / 20), f = (uint32_t)(t % 20);
+__device__ __forceinline__ void proxy_triangle(const float* __restrict__ g, const float* __restrict__ kiso,
+                                               uint32_t tri, float out[3][3]) {
+  const uint32_t j = tri / kFaces, f = tri % kFaces;
   const float* gj = g + 10ull * j;
   const float k = kiso[j];
   const float fs[3] = {gj[3] * k, gj[4] * k, gj[5] * k};
   const float q0 = gj[6];
   const float qv[3] = {gj[7], gj[8], gj[9]};
-  float out[3][3];
+#pragma unroll
   for (int l = 0; l < 3; ++l) {
     const float* vc = c_ico_v[c_ico_f[f][l]];
     const float vs[3] = {vc[0] * fs[0], vc[1] * fs[1], vc[2] * fs[2]};
     float tv[3], tt[3];
     cross3(qv, vs, tv);
+#pragma unroll
     for (int i = 0; i < 3; ++i) tv[i] *= 2.0f;
     cross3(qv, tv, tt);
+#pragma unroll
     for (int i = 0; i < 3; ++i) out[l][i] = (vs[i] + q0 * tv[i] + tt[i]) + gj[i];
   }
-  for (int l = 0; l < 3; ++l)
-    for (int i = 0; i < 3; ++i) v[(3 * l + i) * cap + t] = out[l][i];
+}
+
+__global__ void k_proxy(const float* __restrict__ g, const float* __restrict__ kiso, uint32_t n_valid, float* lo,
+                        float* hi, uint32_t* tri, uint32_t* node, size_t cap) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)n_valid * kFaces) return;
+  float v[3][3];
+  proxy_triangle(g, kiso, (uint32_t)t, v);
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    lo[d * cap + t] = ref_min(ref_min(out[0][d], out[1][d]), out[2][d]);
-    hi[d * cap + t] = ref_max(ref_max(out[0][d], out[1][d]), out[2][d]);
+    lo[d * cap + t] = ref_min(ref_min(v[0][d], v[1][d]), v[2][d]);
+    hi[d * cap + t] = ref_max(ref_max(v[0][d], v[1][d]), v[2][d]);
   }
-  gid[t] = ids[j];
+  tri[t] = (uint32_t)t;
   node[t] = 0;
 }
 
-// Scene box over every proxy vertex: per-block reduction of order-mapped
-// keys, then one atomic per block and bound.
-__global__ void k_scene_box(const float* __restrict__ v, size_t cap, size_t n, uint32_t* box) {
+// Scene box over every proxy triangle: per-warp reduction of order-mapped
+// keys, then one atomic per warp and bound.
+__global__ void k_scene_box(TriView V, size_t n, uint32_t* box) {
   uint32_t mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0, 0, 0};
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    for (int l = 0; l < 3; ++l)
-      for (int d = 0; d < 3; ++d) {
-        const uint32_t k = ordf(v[(3 * l + d) * cap + t]);
-        mn[d] = min(mn[d], k);
-        mx[d] = max(mx[d], k);
-      }
-  for (int d = 0; d < 3; ++d) {
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[d] = min(mn[d], __shfl_xor_sync(0xFFFFFFFFu, mn[d], o));
-      mx[d] = max(mx[d], __shfl_xor_sync(0xFFFFFFFFu, mx[d], o));
+    for (int d = 0; d < 3; ++d) {
+      mn[d] = min(mn[d], ordf(V.lo[d * V.cap + t]));
+      mx[d] = max(mx[d], ordf(V.hi[d * V.cap + t]));
     }
+  for (int d = 0; d < 3; ++d) {
+    const uint32_t a = __reduce_min_sync(0xFFFFFFFFu, mn[d]), b = __reduce_max_sync(0xFFFFFFFFu, mx[d]);
     if ((threadIdx.x & 31) == 0) {
-      atomicMin(&box[2 * d], mn[d]);
-      atomicMax(&box[2 * d + 1], mx[d]);
+      atomicMin(&box[2 * d], a);
+      atomicMax(&box[2 * d + 1], b);
     }
   }
 }
@@ -313,352 +365,24 @@ __global__ void k_box_decode(const uint32_t* box, float* node_lo, float* node_hi
   }
 }
 
-// ------------------------------------------------------------ level kernels
-__global__ void k_run_heads(const uint32_t* __restrict__ gid, const uint32_t* __restrict__ node, size_t T,
-                            uint32_t* flag) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t > T) return;
-  flag[t] = (t < T && (t == 0 || gid[t] != gid[t - 1] || node[t] != node[t - 1])) ? 1u : 0u;
-}
-
-__global__ void k_run_scatter(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ ridx,
-                              const uint32_t* __restrict__ node, size_t T, uint32_t* run_start, uint32_t* run_node) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T || !flag[t]) return;
-  run_start[ridx[t]] = (uint32_t)t;
-  run_node[ridx[t]] = node[t];
-}
-
-// First run of every node: runs are ordered by node, so node n's runs start
-// at the run index of its first triangle (an empty node gets the next node's
-// first run), and G[n] = rb[n+1] - rb[n].  rb[N] = R.
-__global__ void k_node_runs(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ ridx, uint32_t N,
-                            uint32_t* rb, uint32_t* G) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n > N) return;
-  rb[n] = ridx[tb[n]];
-  if (n < N) G[n] = ridx[tb[n + 1]] - ridx[tb[n]];
-}
-
-struct NodeConst {
-  double cell_area_rcp[3], area_mul[3], area_add[3];
-  float cell_min[3], cell_max[3], lim_lo[3], lim_hi[3];
-  double init_cost;
-  uint32_t G, T;
-  int elig;
+// ------------------------------------------------------------ runs and nodes
+struct HeadOp {  // 1 where a (node, Gaussian) run starts
+  const uint32_t *tri, *node;
+  uint64_t T;
+  __device__ uint32_t operator()(uint64_t t) const {
+    if (t >= T) return 0u;
+    return (t == 0 || tri[t] / kFaces != tri[t - 1] / kFaces || node[t] != node[t - 1]) ? 1u : 0u;
+  }
 };
 
-// Per node: leaf cost, eligibility and the per-axis cell constants of
-// try_to_split, in the host builder's types.
-__global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ G,
-                             const float* __restrict__ nlo, const float* __restrict__ nhi, uint32_t N, int level,
-                             Params P, NodeConst* nc, uint32_t* eT, uint32_t* eG) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  NodeConst c;
-  c.T = tb[n + 1] - tb[n];
-  c.G = G[n];
-  const size_t Gs = c.G;
-  double cost = double(Gs) * P.isect_cost;
-  if (P.sah_mode == 7) cost = cost + P.sort_cost * Gs * Gs;
-  if (P.force_split && (size_t)c.T > (size_t)P.force_split) cost = DBL_MAX;
-  c.init_cost = cost;
-  c.elig = (level < P.max_level && c.G > kMinPrim) ? 1 : 0;
-  float blo[3], bhi[3], ext[3];
-  for (int d = 0; d < 3; ++d) {
-    blo[d] = nlo[3 * n + d];
-    bhi[d] = nhi[3 * n + d];
-    ext[d] = bhi[d] - blo[d];
-  }
-  const float cell_area_f = (ext[0] * ext[1]) + (ext[1] * ext[2]) + (ext[0] * ext[2]);
-  const double cell_area = cell_area_f;
-  for (int a = 0; a < 3; ++a) {
-    const int a1 = (a + 1) % 3, a2 = (a + 2) % 3;
-    c.cell_area_rcp[a] = 1 / cell_area;
-    c.area_mul[a] = double(ext[a1]) + double(ext[a2]);
-    c.area_add[a] = double(ext[a1]) * double(ext[a2]);
-    c.cell_min[a] = blo[a];
-    c.cell_max[a] = bhi[a];
-    c.lim_lo[a] = blo[a] + kEps;
-    c.lim_hi[a] = bhi[a] - kEps;
-  }
-  nc[n] = c;
-  eT[n] = c.elig ? c.T : 0u;
-  eG[n] = c.elig ? c.G : 0u;
-}
-
-// Per run: the ID's interval on each axis (first triangle's box, then
-// strict comparisons, in triangle order, as the host sweep builds it) and
-// the keys of the interval starts, ends and planar positions.
-__global__ void k_run_bounds(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node,
-                             uint32_t R, size_t T, const float* __restrict__ lo, const float* __restrict__ hi,
-                             size_t cap, const NodeConst* __restrict__ nc, const uint32_t* __restrict__ rb,
-                             const uint32_t* __restrict__ grb, size_t eGT, int nb, uint64_t* kmin, uint64_t* kmax,
-                             uint64_t* kpl, uint32_t* pl_cnt, unsigned long long* pl_fill, uint32_t N) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t n = run_node[r];
-  if (!nc[n].elig) return;
-  const uint32_t t0 = run_start[r], t1 = r + 1 < R ? run_start[r + 1] : (uint32_t)T;
-  const size_t slot = grb[n] + (r - rb[n]);
-  for (int a = 0; a < 3; ++a) {
-    float mn = lo[a * cap + t0], mx = hi[a * cap + t0];
-    for (uint32_t t = t0 + 1; t < t1; ++t) {
-      const float l = lo[a * cap + t], h = hi[a * cap + t];
-      if (l < mn) mn = l;
-      if (h > mx) mx = h;
-    }
-    kmin[a * eGT + slot] = make_key(a, n, mn, nb);
-    kmax[a * eGT + slot] = make_key(a, n, mx, nb);
-    if (mn == mx) {
-      const unsigned long long at = atomicAdd(pl_fill, 1ull);
-      kpl[at] = make_key(a, n, mn, nb);
-      atomicAdd(&pl_cnt[(size_t)a * N + n], 1u);
-    }
-  }
-}
-
-// Candidate positions of a run (one Gaussian's triangles in one node): the
-// lo and hi edges of its triangles on axis a, bitwise duplicates removed
-// (-0 and +0 stay distinct, as in the full sorted list; the sweep groups
-// equal positions anyway, so the scored candidates are the same).  A run
-// holds at most 20 triangles; longer runs (not produced by the proxy mesh)
-// keep every edge.
-constexpr int kRunEdges = 64;
-
-template <bool WRITE>
-__device__ __forceinline__ uint32_t run_edges(const float* __restrict__ lo, const float* __restrict__ hi, size_t cap,
-                                              uint32_t t0, uint32_t t1, int a, uint32_t n, int nb, uint64_t* out) {
-  const uint32_t m = 2 * (t1 - t0);
-  uint32_t count = 0;
-  if (m > (uint32_t)kRunEdges) {
-    for (uint32_t t = t0; t < t1; ++t) {
-      if (WRITE) {
-        out[count] = make_key(a, n, lo[a * cap + t], nb);
-        out[count + 1] = make_key(a, n, hi[a * cap + t], nb);
-      }
-      count += 2;
-    }
-    return count;
-  }
-  uint32_t v[kRunEdges];
-  for (uint32_t t = t0; t < t1; ++t) {
-    v[2 * (t - t0)] = __float_as_uint(lo[a * cap + t]);
-    v[2 * (t - t0) + 1] = __float_as_uint(hi[a * cap + t]);
-  }
-  for (uint32_t j = 0; j < m; ++j) {
-    bool seen = false;
-    for (uint32_t k = 0; k < j && !seen; ++k) seen = v[k] == v[j];
-    if (seen) continue;
-    if (WRITE) out[count] = make_key(a, n, __uint_as_float(v[j]), nb);
-    ++count;
-  }
-  return count;
-}
-
-// Pass 1: distinct candidate count per (axis, run); 0 for runs of nodes that
-// are not split candidates.
-__global__ void k_run_cand_count(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node,
-                                 uint32_t R, size_t T, const float* __restrict__ lo, const float* __restrict__ hi,
-                                 size_t cap, const NodeConst* __restrict__ nc, unsigned long long* cnt) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t n = run_node[r];
-  const uint32_t t0 = run_start[r], t1 = r + 1 < R ? run_start[r + 1] : (uint32_t)T;
-  for (int a = 0; a < 3; ++a)
-    cnt[(size_t)a * R + r] = nc[n].elig ? run_edges<false>(lo, hi, cap, t0, t1, a, n, 0, nullptr) : 0u;
-}
-
-// Pass 2: the keys, at the scanned offsets.
-__global__ void k_run_cand_write(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node,
-                                 uint32_t R, size_t T, const float* __restrict__ lo, const float* __restrict__ hi,
-                                 size_t cap, const NodeConst* __restrict__ nc, const unsigned long long* __restrict__ off,
-                                 int nb, uint64_t* kc) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t n = run_node[r];
-  if (!nc[n].elig) return;
-  const uint32_t t0 = run_start[r], t1 = r + 1 < R ? run_start[r + 1] : (uint32_t)T;
-  for (int a = 0; a < 3; ++a) run_edges<true>(lo, hi, cap, t0, t1, a, n, nb, kc + off[(size_t)a * R + r]);
-}
-
-__device__ __forceinline__ void decode(uint64_t k, int nb, int* a, uint32_t* n) {
-  *a = (int)(k >> (32 + nb));
-  *n = (uint32_t)((k >> 32) & ((1ull << nb) - 1));
-}
-
-// One thread per sorted candidate: the SAH score of the first candidate of
-// each group of equal positions inside (cell_min + eps, cell_max - eps).
-__global__ void k_eval(const uint64_t* __restrict__ kc, size_t n_cand, const unsigned long long* __restrict__ coff,
-                       const uint32_t* __restrict__ rb, uint32_t R, int nb,
-                       const uint64_t* __restrict__ kmin, const uint64_t* __restrict__ kmax,
-                       const uint64_t* __restrict__ kpl, size_t eGT, const uint32_t* __restrict__ grb,
-                       const uint32_t* __restrict__ plb,
-                       const uint32_t* __restrict__ pl_cnt, const NodeConst* __restrict__ nc, uint32_t N, Params P,
-                       double* cost_out, uint8_t* side_out, unsigned long long* best_bits) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  double cost = __longlong_as_double(0x7FF0000000000000ll);  // +inf: not a candidate
-  uint8_t side = 0;
-  uint32_t seg = kNone;
-  // warp-wide brackets when all 32 lanes sit in one (axis, node) segment
-  uint32_t my_seg = kNone;
-  float my_p = 0.f;
-  if (i < n_cand) {
-    int a0;
-    uint32_t n0;
-    decode(kc[i], nb, &a0, &n0);
-    my_seg = (uint32_t)a0 * N + n0;
-    my_p = key_pos(kc[i]);
-  }
-  const bool uniform = __all_sync(0xFFFFFFFFu, my_seg == __shfl_sync(0xFFFFFFFFu, my_seg, 0) && my_seg != kNone);
-  Bracket bmin{0, 0}, bmax{0, 0}, bpl{0, 0};
-  if (uniform) {
-    const uint32_t a0 = my_seg / N, n0 = my_seg % N;
-    const uint32_t G0 = nc[n0].G;
-    const size_t gb0 = (size_t)a0 * eGT + grb[n0];
-    bmin = warp_bracket(kmin, gb0, G0, my_p, lane);
-    bmax = warp_bracket(kmax, gb0, G0, my_p, lane);
-    bpl = warp_bracket(kpl, plb[my_seg], pl_cnt[my_seg], my_p, lane);
-  }
-  if (i < n_cand) {
-    const uint64_t k = kc[i];
-    int a;
-    uint32_t n;
-    decode(k, nb, &a, &n);
-    const float p = key_pos(k);
-    const size_t s0 = coff[(size_t)a * R + rb[n]];
-    const NodeConst& c = nc[n];
-    const bool head = (i == s0) || !(key_pos(kc[i - 1]) == p);
-    if (head && p > c.lim_lo[a] && p < c.lim_hi[a]) {
-      const uint32_t G = c.G;
-      const size_t gb = (size_t)a * eGT + grb[n];
-      const size_t pb = plb[(size_t)a * N + n];
-      const uint32_t pn = pl_cnt[(size_t)a * N + n];
-      uint32_t open, close, eq_max, pl_lt, pl_le;
-      if (uniform) {
-        open = count_less_in(kmin, gb, bmin.lo, bmin.hi, p);
-        close = count_less_in(kmax, gb, bmax.lo, bmax.hi, p);
-        eq_max = count_le_in(kmax, gb, close, bmax.hi, p) - close;
-        pl_lt = count_less_in(kpl, pb, bpl.lo, bpl.hi, p);
-        pl_le = count_le_in(kpl, pb, pl_lt, bpl.hi, p);
-      } else {
-        open = count_less(kmin, gb, G, p);
-        close = count_less(kmax, gb, G, p);
-        eq_max = count_le(kmax, gb, G, p) - close;
-        pl_lt = count_less(kpl, pb, pn, p);
-        pl_le = count_le(kpl, pb, pn, p);
-      }
-      const int num_planars = (int)(pl_le - pl_lt);
-      const int local_close = (int)eq_max - num_planars;
-
-      const double extent_l = double(p) - c.cell_min[a];
-      const double extent_r = c.cell_max[a] - double(p);
-      const double prob_l = (extent_l * c.area_mul[a] + c.area_add[a]) * c.cell_area_rcp[a];
-      const double prob_r = (extent_r * c.area_mul[a] + c.area_add[a]) * c.cell_area_rcp[a];
-      const int n_left_only = (int)close + local_close;
-      const int n_cross = (int)open - n_left_only;
-      const int n_right_only = int(G) - (n_left_only + n_cross + num_planars);
-      const int tl[2] = {n_left_only + n_cross + num_planars, n_left_only + n_cross};
-      const int tr[2] = {n_right_only + n_cross, n_right_only + n_cross + num_planars};
-      const float eb[2] = {(tl[0] == 0 || tr[0] == 0) ? kEmptyBonus : 1.0f,
-                           (tl[1] == 0 || tr[1] == 0) ? kEmptyBonus : 1.0f};
-      double sah[2];
-      for (int s = 0; s < 2; ++s) {
-        switch (P.sah_mode) {
-          case 0:
-            sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s];
-            break;
-          case 4: {
-            // n * pow(n / 16, 0.5) with the square root, which is what a
-            // correctly rounded pow returns for the exponent 0.5
-            const double xl = double(tl[s]), xr = double(tr[s]);
-            const double sl = tl[s] == 0 ? 0.0 : xl * sqrt(xl / 16.0);
-            const double sr = tr[s] == 0 ? 0.0 : xr * sqrt(xr / 16.0);
-            sah[s] = kTravCost + P.isect_cost * (sl * prob_l + sr * prob_r) * eb[s];
-            break;
-          }
-          case 7:
-            sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s] +
-                     P.sort_cost * (double(tl[s]) * double(tl[s]) * prob_l + double(tr[s]) * double(tr[s]) * prob_r);
-            break;
-          default: {
-            const double n_total = double(tl[s] + tr[s]);
-            const double diff = fabs(double(tl[s]) - double(tr[s]));
-            const double ratio = (n_total > 0.0) ? (diff / n_total) : 0.0;
-            const double penalty = 1.0 + (ratio * 0.1);
-            sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s] * penalty;
-            break;
-          }
-        }
-      }
-      const double cst = sah[0] <= sah[1] ? sah[0] : sah[1];
-      if (cst < c.init_cost) {
-        cost = cst;
-        side = sah[0] <= sah[1] ? 0 : 1;
-        seg = (uint32_t)a * N + n;
-      }
-    }
-    cost_out[i] = cost;
-    side_out[i] = side;
-  }
-  // min over the segment: a warp whose valid lanes share one segment
-  // reduces first; a block whose warps all share one segment reduces again
-  // and issues one atomic (the top levels have three segments and tens of
-  // millions of candidates)
-  unsigned long long bits = (unsigned long long)__double_as_longlong(cost);
-  uint32_t lead = seg;
-  for (int o = 16; o > 0; o >>= 1) lead = min(lead, __shfl_xor_sync(0xFFFFFFFFu, lead, o));
-  const bool warp_uniform = __all_sync(0xFFFFFFFFu, seg == lead || seg == kNone);
-  if (warp_uniform) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, bits, o);
-      bits = other < bits ? other : bits;
-    }
-  } else if (seg != kNone) {
-    atomicMin(&best_bits[seg], bits);
-  }
-  __shared__ uint32_t s_seg[8];
-  __shared__ unsigned long long s_bits[8];
-  const int w = threadIdx.x >> 5;
-  if (lane == 0) {
-    s_seg[w] = warp_uniform ? lead : 0xFFFFFFFEu;  // 0xFFFFFFFE: this warp has already issued its atomics
-    s_bits[w] = bits;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (int)(blockDim.x >> 5);
-    uint32_t bs = kNone;
-    bool same = true;
-    for (int k = 0; k < nw; ++k) {
-      if (s_seg[k] == kNone) continue;
-      if (s_seg[k] == 0xFFFFFFFEu || (bs != kNone && s_seg[k] != bs)) same = false;
-      if (bs == kNone && s_seg[k] != 0xFFFFFFFEu) bs = s_seg[k];
-    }
-    if (same && bs != kNone) {
-      unsigned long long m = ~0ull;
-      for (int k = 0; k < nw; ++k)
-        if (s_seg[k] == bs && s_bits[k] < m) m = s_bits[k];
-      atomicMin(&best_bits[bs], m);
-    } else {
-      for (int k = 0; k < nw; ++k)
-        if (s_seg[k] != kNone && s_seg[k] != 0xFFFFFFFEu) atomicMin(&best_bits[s_seg[k]], s_bits[k]);
-    }
-  }
-}
-
-// Second pass: the first (lowest sorted index) candidate with the minimum.
-__global__ void k_argmin(const uint64_t* __restrict__ kc, const double* __restrict__ cost, size_t n_cand, int nb,
-                         uint32_t N, const unsigned long long* __restrict__ best_bits, unsigned long long* best_idx) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_cand) return;
-  const double c = cost[i];
-  if (isinf(c)) return;
-  int a;
-  uint32_t n;
-  decode(kc[i], nb, &a, &n);
-  const size_t seg = (size_t)a * N + n;
-  if ((unsigned long long)__double_as_longlong(c) == best_bits[seg]) atomicMin(&best_idx[seg], (unsigned long long)i);
+__global__ void k_run_scatter(const uint32_t* __restrict__ ridx, const uint32_t* __restrict__ node, size_t T,
+                              uint32_t* run_start, uint32_t* run_node) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= T) return;
+  const uint32_t r = ridx[t];
+  if (ridx[t + 1] == r) return;
+  run_start[r] = (uint32_t)t;
+  run_node[r] = node[t];
 }
 
 struct Decision {
@@ -667,30 +391,642 @@ struct Decision {
   int side;
 };
 
-__global__ void k_choose(const NodeConst* __restrict__ nc, uint32_t N, const unsigned long long* __restrict__ best_bits,
-                         const unsigned long long* __restrict__ best_idx, const uint64_t* __restrict__ kc,
-                         const uint8_t* __restrict__ side, Decision* dec, uint32_t* is_split) {
+// Search classes by the number of distinct IDs of a node: a warp's six lists
+// of up to 64 keys sort in 21 bitonic steps and four nodes share a block's
+// static shared memory; up to 256 a 128-thread block holds 21 KB, up to 1024
+// a 512-thread block 86 KB, two per SM; beyond that a node alone keeps many
+// blocks busy and its keys go through the device-wide sort.
+constexpr uint32_t kWarpIds = 64, kMidIds = 256, kBlockIds = 1024;
+
+// Per node: its first run, its ID count, the class lists of its split search
+// (nodes of up to kWarpIds need no list) and a leaf decision to begin with.
+// counts: [0] kMidIds nodes, [1] kBlockIds nodes, [2] larger nodes.
+__global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ ridx, uint32_t N,
+                             int level, int max_level, uint32_t* rb, Decision* dec, uint32_t* is_split,
+                             uint32_t* list_mid, uint32_t* list_block, uint32_t* counts, uint32_t* eG) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  double cur = nc[n].init_cost;
-  Decision d{-1, 0.f, 0};
-  if (nc[n].elig) {
-    for (int a = 0; a < 3; ++a) {
-      const size_t seg = (size_t)a * N + n;
-      if (best_idx[seg] == ~0ull) continue;
-      const double c = __longlong_as_double((long long)best_bits[seg]);
-      if (c < cur) {
-        cur = c;
-        d.axis = a;
-        d.split = key_pos(kc[best_idx[seg]]);
-        d.side = side[best_idx[seg]];
+  if (n > N) return;
+  rb[n] = ridx[tb[n]];
+  if (n == N) {
+    is_split[n] = 0u;
+    return;
+  }
+  const uint32_t G = ridx[tb[n + 1]] - ridx[tb[n]];
+  dec[n] = Decision{-1, 0.f, 0};
+  is_split[n] = 0u;
+  const bool elig = level < max_level && G > kMinPrim;
+  if (elig && G > kWarpIds && G <= kMidIds) list_mid[atomicAdd(&counts[0], 1u)] = n;
+  if (elig && G > kMidIds && G <= kBlockIds) list_block[atomicAdd(&counts[1], 1u)] = n;
+  if (eG) {
+    const bool big = elig && G > kBlockIds;
+    eG[n] = big ? G : 0u;
+    if (big) atomicAdd(&counts[2], 1u);
+  }
+}
+
+// ------------------------------------------------------------ scores
+// A node's constants of try_to_split: float extents, and in float and double
+// what the scores multiply with.
+struct Cell {
+  float lo[3], hi[3], am[3], aa[3], rcp, init;
+  uint32_t G;
+};
+
+__device__ __forceinline__ double init_cost(const Params& P, uint32_t G, uint32_t T) {
+  double cost = double((size_t)G) * P.isect_cost;
+  if (P.sah_mode == 7) cost = cost + P.sort_cost * (size_t)G * (size_t)G;
+  if (P.force_split && (size_t)T > (size_t)P.force_split) cost = DBL_MAX;
+  return cost;
+}
+
+__device__ __forceinline__ Cell make_cell(const Params& P, const float* __restrict__ nlo,
+                                          const float* __restrict__ nhi, uint32_t n, uint32_t G, uint32_t T) {
+  Cell c;
+  float ext[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    c.lo[d] = nlo[3ull * n + d];
+    c.hi[d] = nhi[3ull * n + d];
+    ext[d] = c.hi[d] - c.lo[d];
+  }
+  const float area = (ext[0] * ext[1]) + (ext[1] * ext[2]) + (ext[0] * ext[2]);
+  c.rcp = 1.0f / area;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    c.am[a] = ext[(a + 1) % 3] + ext[(a + 2) % 3];
+    c.aa[a] = ext[(a + 1) % 3] * ext[(a + 2) % 3];
+  }
+  c.init = __double2float_ru(init_cost(P, G, T));  // +inf for DBL_MAX
+  c.G = G;
+  return c;
+}
+template <typename V>
+__device__ __forceinline__ V pick(const V v[3], int a) {
+  return a == 0 ? v[0] : a == 1 ? v[1] : v[2];
+}
+
+__device__ __forceinline__ bool in_limits(const Cell& c, int a, float p) {
+  return p > pick(c.lo, a) + kEps && p < pick(c.hi, a) - kEps;
+}
+
+// Counts at a position: intervals begun before it, ended before it, ended at
+// it, and planar at it.
+struct Counts {
+  uint32_t open, close, eq_max, planar;
+};
+
+// FP32 score (the better of the two planar sides).
+__device__ __forceinline__ float score32(const Params& P, const Cell& c, int a, float p, const Counts& k) {
+  const float pl = ((p - pick(c.lo, a)) * pick(c.am, a) + pick(c.aa, a)) * c.rcp;
+  const float pr = ((pick(c.hi, a) - p) * pick(c.am, a) + pick(c.aa, a)) * c.rcp;
+  const int tl1 = (int)k.open, tr0 = (int)(c.G - k.close - k.eq_max), pn = (int)k.planar;
+  float best = __int_as_float(0x7f800000);
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    if (s == 1 && pn == 0) break;  // both sides score the same
+    const int il = s == 0 ? tl1 + pn : tl1, ir = s == 0 ? tr0 : tr0 + pn;
+    const float tl = (float)il, tr = (float)ir;
+    const float eb = (il == 0 || ir == 0) ? kEmptyBonus : 1.0f;
+    float v;
+    if (P.sah_mode == 4) {
+      v = kTravCost + P.isect_cost * (tl * sqrtf(tl * 0.0625f) * pl + tr * sqrtf(tr * 0.0625f) * pr) * eb;
+    } else {
+      v = P.isect_cost * (tl * pl + tr * pr) * eb;
+      if (P.sah_mode != 0 && P.sah_mode != 7) v *= 1.0f + __fdividef(fabsf(tl - tr), fmaxf(tl + tr, 1.0f)) * 0.1f;
+      v += kTravCost;
+      if (P.sah_mode == 7) v += P.sort_cost * (tl * tl * pl + tr * tr * pr);
+    }
+    if (!(v < __int_as_float(0x7f800000))) return __int_as_float(0x7fc00000);  // overflow: NaN, never discarded
+    best = v < best ? v : best;
+  }
+  return best;
+}
+
+// The host builder's score, its types and operation order.
+__device__ __noinline__ double score64(const Params& P, const float* __restrict__ nlo, const float* __restrict__ nhi,
+                                       uint32_t n, uint32_t G, int a, float p, Counts k, int* side) {
+  float ext[3];
+  for (int d = 0; d < 3; ++d) ext[d] = nhi[3ull * n + d] - nlo[3ull * n + d];
+  const float cell_area_f = (ext[0] * ext[1]) + (ext[1] * ext[2]) + (ext[0] * ext[2]);
+  const double cell_area = cell_area_f;
+  const double cell_area_rcp = 1 / cell_area;
+  const int a1 = (a + 1) % 3, a2 = (a + 2) % 3;
+  const double area_mul = double(pick(ext, a1)) + double(pick(ext, a2));
+  const double area_add = double(pick(ext, a1)) * double(pick(ext, a2));
+  const float cell_min = nlo[3ull * n + a], cell_max = nhi[3ull * n + a];
+  const int num_planars = (int)k.planar;
+  const int local_close = (int)k.eq_max - num_planars;
+  const double extent_l = double(p) - cell_min;
+  const double extent_r = cell_max - double(p);
+  const double prob_l = (extent_l * area_mul + area_add) * cell_area_rcp;
+  const double prob_r = (extent_r * area_mul + area_add) * cell_area_rcp;
+  const int n_left_only = (int)k.close + local_close;
+  const int n_cross = (int)k.open - n_left_only;
+  const int n_right_only = int(G) - (n_left_only + n_cross + num_planars);
+  const int tl[2] = {n_left_only + n_cross + num_planars, n_left_only + n_cross};
+  const int tr[2] = {n_right_only + n_cross, n_right_only + n_cross + num_planars};
+  const float eb[2] = {(tl[0] == 0 || tr[0] == 0) ? kEmptyBonus : 1.0f,
+                       (tl[1] == 0 || tr[1] == 0) ? kEmptyBonus : 1.0f};
+  double sah[2];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    switch (P.sah_mode) {
+      case 0:
+        sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s];
+        break;
+      case 4: {
+        // n * pow(n / 16, 0.5) with the square root, which is what a
+        // correctly rounded pow returns for the exponent 0.5
+        const double xl = double(tl[s]), xr = double(tr[s]);
+        const double sl = tl[s] == 0 ? 0.0 : xl * sqrt(xl / 16.0);
+        const double sr = tr[s] == 0 ? 0.0 : xr * sqrt(xr / 16.0);
+        sah[s] = kTravCost + P.isect_cost * (sl * prob_l + sr * prob_r) * eb[s];
+        break;
+      }
+      case 7:
+        sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s] +
+                 P.sort_cost * (double(tl[s]) * double(tl[s]) * prob_l + double(tr[s]) * double(tr[s]) * prob_r);
+        break;
+      default: {
+        const double n_total = double(tl[s] + tr[s]);
+        const double diff = fabs(double(tl[s]) - double(tr[s]));
+        const double ratio = (n_total > 0.0) ? (diff / n_total) : 0.0;
+        const double penalty = 1.0 + (ratio * 0.1);
+        sah[s] = kTravCost + P.isect_cost * (double(tl[s]) * prob_l + double(tr[s]) * prob_r) * eb[s] * penalty;
+        break;
       }
     }
   }
-  dec[n] = d;
-  is_split[n] = d.axis >= 0 ? 1u : 0u;
+  *side = sah[0] <= sah[1] ? 0 : 1;
+  return sah[0] <= sah[1] ? sah[0] : sah[1];
 }
 
+// Candidates in the sequential sweep's order: lowest axis, then lowest
+// position (bits), the planar side riding along.
+__device__ __forceinline__ uint64_t cand_key(int a, float p, int side) {
+  return ((uint64_t)a << 33) | ((uint64_t)ordf(p) << 1) | (uint64_t)side;
+}
+__device__ __forceinline__ Decision key_decision(uint64_t k) {
+  return Decision{(int)(k >> 33), unordf((uint32_t)(k >> 1)), (int)(k & 1u)};
+}
+
+// ------------------------------------------------------------ split search of one node
+// NT threads (a warp or a block) search one node of at most CAP IDs.  Per
+// axis the interval starts and ends are sorted in shared memory (bitonic;
+// 6 lists side by side), every event is scored in FP32 with its gap bound,
+// the few candidates within the margin are scored in FP64, then the node's
+// triangle edges inside the surviving gaps.
+template <int NT, int CAP>
+struct SearchMem {
+  uint32_t k[6][CAP];       // sorted ordz keys: starts of axes 0..2, ends of axes 0..2
+  uint32_t pl[3][CAP];      // planar positions, unsorted
+  float cost[6][CAP], bound[6][CAP];
+  uint32_t n_pl[3], hull_lo[3], hull_hi[3];
+  float red[NT / 32];
+  double best_c[NT / 32];
+  uint64_t best_k[NT / 32];
+};
+
+template <int NT>
+__device__ __forceinline__ void group_sync() {
+  if (NT == 32) __syncwarp();
+  else __syncthreads();
+}
+
+// tid: index inside the group.  n: node; runs [r0, r0 + G), triangles [t0, t1).
+template <int NT, int CAP>
+__device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, const Params& P, uint32_t n, uint32_t r0,
+                                            uint32_t G, uint32_t t0, uint32_t t1,
+                                            const uint32_t* __restrict__ run_start, const TriView& V,
+                                            const float* __restrict__ nlo, const float* __restrict__ nhi,
+                                            Decision* dec, uint32_t* is_split) {
+  const float kInf = __int_as_float(0x7f800000);
+  uint32_t M = 32;
+  while (M < G) M <<= 1;
+  if (tid < 3) {
+    S.n_pl[tid] = 0u;
+    S.hull_lo[tid] = 0xFFFFFFFFu;
+    S.hull_hi[tid] = 0u;
+  }
+  group_sync<NT>();
+  for (uint32_t r = tid; r < M; r += NT) {
+    uint32_t km[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
+    if (r < G) {
+      const uint32_t a0 = run_start[r0 + r], a1 = r + 1 < G ? run_start[r0 + r + 1] : t1;
+      float mn[3], mx[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = V.lo[a * V.cap + a0];
+        mx[a] = V.hi[a * V.cap + a0];
+      }
+      for (uint32_t t = a0 + 1; t < a1; ++t)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float l = V.lo[a * V.cap + t], h = V.hi[a * V.cap + t];
+          if (l < mn[a]) mn[a] = l;
+          if (h > mx[a]) mx[a] = h;
+        }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        km[a] = ordz(mn[a]);
+        km[3 + a] = ordz(mx[a]);
+        if (mn[a] == mx[a]) S.pl[a][atomicAdd(&S.n_pl[a], 1u)] = km[a];
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < 6; ++l) S.k[l][r] = km[l];
+  }
+  group_sync<NT>();
+  // bitonic sort of the six lists
+  for (uint32_t size = 2; size <= M; size <<= 1)
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t i = tid; i < 6 * (M / 2); i += NT) {
+        const uint32_t l = i / (M / 2), j = i & (M / 2 - 1);
+        const uint32_t x = 2 * j - (j & (stride - 1)), y = x + stride;
+        const uint32_t u = S.k[l][x], v = S.k[l][y];
+        if ((u > v) == ((x & size) == 0)) {
+          S.k[l][x] = v;
+          S.k[l][y] = u;
+        }
+      }
+      group_sync<NT>();
+    }
+  const Cell c = make_cell(P, nlo, nhi, n, G, t1 - t0);
+  auto counts_at = [&](int a, uint32_t kp) {
+    Counts k;
+    k.open = lower(S.k[a], G, kp);
+    k.close = lower(S.k[3 + a], G, kp);
+    k.eq_max = upper(S.k[3 + a], G, kp) - k.close;
+    k.planar = 0;
+    for (uint32_t j = 0; j < S.n_pl[a]; ++j) k.planar += S.pl[a][j] == kp ? 1u : 0u;
+    return k;
+  };
+  // events: FP32 score, and a lower bound over the gap up to the next event
+  float best32 = c.init;
+  for (uint32_t i = tid; i < 6 * G; i += NT) {
+    const uint32_t l = i / G, j = i - l * G;
+    const int a = (int)(l % 3);
+    const uint32_t kp = S.k[l][j];
+    const float p = unordf(kp);
+    float cost = kInf, bound = kInf;
+    if (!(j > 0 && S.k[l][j - 1] == kp)) {  // equal events score once
+      const Counts k = counts_at(a, kp);
+      if (in_limits(c, a, p)) cost = score32(P, c, a, p, k);
+      const uint32_t le_mn = upper(S.k[a], G, kp), le_mx = k.close + k.eq_max;
+      const uint32_t nmn = le_mn < G ? S.k[a][le_mn] : 0xFFFFFFFFu, nmx = le_mx < G ? S.k[3 + a][le_mx] : 0xFFFFFFFFu;
+      const uint32_t kn = min(nmn, nmx);
+      if (kn != 0xFFFFFFFFu) {
+        const float q = unordf(kn);
+        const float pa = fmaxf(p, pick(c.lo, a) + kEps), pb = fminf(q, pick(c.hi, a) - kEps);
+        if (!(pa > pb)) {
+          const Counts kg{le_mn, le_mx, 0u, 0u};
+          const float ba = score32(P, c, a, pa, kg), bb = score32(P, c, a, pb, kg);
+          bound = (ba < bb || !(ba == ba)) ? ba : bb;
+        }
+      }
+    }
+    S.cost[l][j] = cost;
+    S.bound[l][j] = bound;
+    best32 = cost < best32 ? cost : best32;
+  }
+  for (int o = 16; o > 0; o >>= 1) best32 = fminf(best32, __shfl_xor_sync(0xFFFFFFFFu, best32, o));
+  if (NT > 32) {
+    if ((tid & 31) == 0) S.red[tid >> 5] = best32;
+    __syncthreads();
+    for (int w = 0; w < NT / 32; ++w) best32 = fminf(best32, S.red[w]);
+  }
+  const float limit = P.filter ? best32 * (1.0f + kMargin) : kInf;
+  const double init = init_cost(P, G, t1 - t0);
+  double best = init;
+  uint64_t best_k = ~0ull;
+  auto consider = [&](int a, float p, const Counts& k) {
+    int side;
+    const double cst = score64(P, nlo, nhi, n, G, a, p, k, &side);
+    if (cst < init) {
+      const uint64_t key = cand_key(a, p, side);
+      if (cst < best || (cst == best && key < best_k)) {
+        best = cst;
+        best_k = key;
+      }
+    }
+  };
+  // events and gaps that are not worse than the best by more than the margin
+  for (uint32_t i = tid; i < 6 * G; i += NT) {
+    const uint32_t l = i / G, j = i - l * G;
+    const int a = (int)(l % 3);
+    const float cost = S.cost[l][j], bound = S.bound[l][j];
+    if (!(cost > limit) && cost != kInf) {
+      const uint32_t kp = S.k[l][j];
+      consider(a, unordf(kp), counts_at(a, kp));
+      if (kp == kZeroKey) {  // the edges at zero say which zero it is
+        atomicMin(&S.hull_lo[a], kp);
+        atomicMax(&S.hull_hi[a], kp);
+      }
+    }
+    if (!(bound > limit) && (bound != kInf || !P.filter)) {
+      const uint32_t kp = S.k[l][j];
+      const uint32_t le_mn = upper(S.k[a], G, kp), le_mx = upper(S.k[3 + a], G, kp);
+      const uint32_t kn = min(le_mn < G ? S.k[a][le_mn] : 0xFFFFFFFFu, le_mx < G ? S.k[3 + a][le_mx] : 0xFFFFFFFFu);
+      atomicMin(&S.hull_lo[a], kp);
+      atomicMax(&S.hull_hi[a], kn);
+    }
+  }
+  group_sync<NT>();
+  // triangle edges inside the surviving gaps (interval ends among them: their
+  // own bits decide between -0 and +0)
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t hl = S.hull_lo[a], hh = S.hull_hi[a];
+    if (hl > hh) continue;
+    for (uint32_t t = t0 + tid; t < t1; t += NT) {
+      const float e[2] = {V.lo[a * V.cap + t], V.hi[a * V.cap + t]};
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const float p = e[s];
+        const uint32_t kp = ordz(p);
+        if (kp < hl || kp > hh || !in_limits(c, a, p)) continue;
+        const Counts k = counts_at(a, kp);
+        if (score32(P, c, a, p, k) > limit) continue;
+        consider(a, p, k);
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double oc = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+    const uint64_t ok = __shfl_xor_sync(0xFFFFFFFFu, best_k, o);
+    if (oc < best || (oc == best && ok < best_k)) {
+      best = oc;
+      best_k = ok;
+    }
+  }
+  if (NT > 32) {
+    if ((tid & 31) == 0) {
+      S.best_c[tid >> 5] = best;
+      S.best_k[tid >> 5] = best_k;
+    }
+    __syncthreads();
+    for (int w = 0; w < NT / 32; ++w)
+      if (S.best_c[w] < best || (S.best_c[w] == best && S.best_k[w] < best_k)) {
+        best = S.best_c[w];
+        best_k = S.best_k[w];
+      }
+  }
+  if (tid == 0 && best_k != ~0ull) {
+    dec[n] = key_decision(best_k);
+    is_split[n] = 1u;
+  }
+}
+
+// Nodes of up to kWarpIds IDs: one warp each, over every node of the level.
+constexpr int kSearchWarps = 4;
+__global__ void __launch_bounds__(32 * kSearchWarps)
+    k_search_warp(Params P, uint32_t N, int level, const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb,
+                  const uint32_t* __restrict__ run_start, TriView V, const float* __restrict__ nlo,
+                  const float* __restrict__ nhi, Decision* dec, uint32_t* is_split) {
+  __shared__ SearchMem<32, kWarpIds> S[kSearchWarps];
+  const int w = threadIdx.x >> 5;
+  const uint32_t n = blockIdx.x * kSearchWarps + w;
+  if (n >= N || level >= P.max_level) return;
+  const uint32_t r0 = rb[n], G = rb[n + 1] - r0;
+  if (G <= kMinPrim || G > kWarpIds) return;
+  search_node<32, (int)kWarpIds>(S[w], threadIdx.x & 31, P, n, r0, G, tb[n], tb[n + 1], run_start, V, nlo, nhi, dec,
+                                 is_split);
+}
+
+// Listed nodes: one block each (the grid walks the list).
+template <int NT, int CAP>
+__global__ void __launch_bounds__(NT)
+    k_search_block(Params P, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
+                   const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb,
+                   const uint32_t* __restrict__ run_start, TriView V, const float* __restrict__ nlo,
+                   const float* __restrict__ nhi, Decision* dec, uint32_t* is_split) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  SearchMem<NT, CAP>& S = *reinterpret_cast<SearchMem<NT, CAP>*>(raw);
+  for (uint32_t i = blockIdx.x; i < *count; i += gridDim.x) {
+    const uint32_t n = list[i], r0 = rb[n];
+    search_node<NT, CAP>(S, threadIdx.x, P, n, r0, rb[n + 1] - r0, tb[n], tb[n + 1], run_start, V, nlo, nhi, dec,
+                         is_split);
+    __syncthreads();
+  }
+}
+
+// ------------------------------------------------------------ split search of large nodes
+// The same search over globally sorted keys: (axis, node, position) -> 64 bits
+// ordered by axis, then node, then position (ordz).
+__device__ __forceinline__ uint64_t make_key(int axis, uint32_t node, uint32_t kp, int nb) {
+  return ((uint64_t)axis << (32 + nb)) | ((uint64_t)node << 32) | kp;
+}
+__device__ __forceinline__ void decode(uint64_t k, int nb, int* a, uint32_t* n) {
+  *a = (int)(k >> (32 + nb));
+  *n = (uint32_t)((k >> 32) & ((1ull << nb) - 1));
+}
+
+struct Big {
+  const uint64_t *kmin, *kmax, *kpl;  // sorted keys; node n's segment on axis a starts at a * eG + grb[n]
+  const uint32_t *grb, *eGn;          // first slot of each large node, its ID count (0: not large)
+  size_t eG;                          // IDs of all large nodes
+  uint32_t n_pl;
+  int nb;
+};
+
+// Per run of a large node: the ID's interval on each axis (first triangle's
+// box, then strict comparisons, in triangle order, as the host sweep builds
+// it) as keys.
+__global__ void k_run_bounds(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node,
+                             const uint32_t* __restrict__ rb, uint32_t N, size_t T, TriView V, Big B, uint64_t* kmin,
+                             uint64_t* kmax, uint64_t* kpl, uint32_t* pl_fill) {
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= rb[N]) return;
+  const uint32_t n = run_node[r];
+  if (B.eGn[n] == 0u) return;
+  const uint32_t t0 = run_start[r], t1 = r + 1 < rb[N] ? run_start[r + 1] : (uint32_t)T;
+  const size_t slot = B.grb[n] + (r - rb[n]);
+  for (int a = 0; a < 3; ++a) {
+    float mn = V.lo[a * V.cap + t0], mx = V.hi[a * V.cap + t0];
+    for (uint32_t t = t0 + 1; t < t1; ++t) {
+      const float l = V.lo[a * V.cap + t], h = V.hi[a * V.cap + t];
+      if (l < mn) mn = l;
+      if (h > mx) mx = h;
+    }
+    kmin[a * B.eG + slot] = make_key(a, n, ordz(mn), B.nb);
+    kmax[a * B.eG + slot] = make_key(a, n, ordz(mx), B.nb);
+    if (mn == mx) kpl[atomicAdd(pl_fill, 1u)] = make_key(a, n, ordz(mn), B.nb);
+  }
+}
+
+__device__ __forceinline__ Counts big_counts(const Big& B, int a, uint32_t n, uint32_t kp) {
+  const size_t b = a * B.eG + B.grb[n];
+  const uint32_t G = B.eGn[n];
+  const uint64_t key = make_key(a, n, kp, B.nb);
+  Counts k;
+  k.open = lower(B.kmin + b, G, key);
+  k.close = lower(B.kmax + b, G, key);
+  k.eq_max = upper(B.kmax + b, G, key) - k.close;
+  k.planar = B.n_pl ? upper(B.kpl, B.n_pl, key) - lower(B.kpl, B.n_pl, key) : 0u;
+  return k;
+}
+
+// State of a large node's search: best FP32 event (float bits; scores are
+// positive where the filter is on), best FP64 cost, its first candidate, and
+// per axis the hull of the surviving gaps.
+struct BigState {
+  uint32_t* best32;
+  unsigned long long *best64, *key;
+  uint32_t *hull_lo, *hull_hi;
+};
+// order-preserving map of a double to unsigned
+__device__ __forceinline__ unsigned long long ordd(double d) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(d);
+  return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+
+// Pass 1: FP32 score and gap bound of every event; the node's best score.
+__global__ void k_event_scores(Params P, Big B, const uint32_t* __restrict__ tb, const float* __restrict__ nlo,
+                               const float* __restrict__ nhi, float2* out, BigState st) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const float kInf = __int_as_float(0x7f800000);
+  float cost = kInf, bound = kInf;
+  uint32_t n = kNone;
+  if (i < 6 * B.eG) {
+    const bool is_max = i >= 3 * B.eG;
+    const size_t j = is_max ? i - 3 * B.eG : i;
+    const uint64_t* own = is_max ? B.kmax : B.kmin;
+    const uint64_t key = own[j];
+    int a;
+    decode(key, B.nb, &a, &n);
+    if (j == 0 || own[j - 1] != key) {
+      const uint32_t kp = (uint32_t)key, G = B.eGn[n];
+      const float p = unordf(kp);
+      const Cell c = make_cell(P, nlo, nhi, n, G, tb[n + 1] - tb[n]);
+      const Counts k = big_counts(B, a, n, kp);
+      if (in_limits(c, a, p)) cost = score32(P, c, a, p, k);
+      const size_t b = a * B.eG + B.grb[n];
+      const uint32_t le_mn = upper(B.kmin + b, G, key), le_mx = k.close + k.eq_max;
+      const uint32_t kn = min(le_mn < G ? (uint32_t)B.kmin[b + le_mn] : 0xFFFFFFFFu,
+                              le_mx < G ? (uint32_t)B.kmax[b + le_mx] : 0xFFFFFFFFu);
+      if (kn != 0xFFFFFFFFu) {
+        const float pa = fmaxf(p, pick(c.lo, a) + kEps), pb = fminf(unordf(kn), pick(c.hi, a) - kEps);
+        if (!(pa > pb)) {
+          const Counts kg{le_mn, le_mx, 0u, 0u};
+          const float ba = score32(P, c, a, pa, kg), bb = score32(P, c, a, pb, kg);
+          bound = (ba < bb || !(ba == ba)) ? ba : bb;
+        }
+      }
+    }
+    out[i] = make_float2(cost, bound);
+  }
+  // one atomic per warp when its events belong to one node, as nearly all do
+  const uint32_t bits = cost >= 0.0f ? __float_as_uint(cost) : 0x7f800000u;  // NaN and negative: no limit from them
+  const uint32_t lead = __shfl_sync(0xFFFFFFFFu, n, 0);
+  if (__all_sync(0xFFFFFFFFu, n == lead)) {
+    const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, bits);
+    if ((threadIdx.x & 31) == 0 && n != kNone && m < 0x7f800000u) atomicMin(&st.best32[n], m);
+  } else if (n != kNone && bits < 0x7f800000u) {
+    atomicMin(&st.best32[n], bits);
+  }
+}
+
+__device__ __forceinline__ float big_limit(const Params& P, const BigState& st, uint32_t n) {
+  return P.filter ? __uint_as_float(st.best32[n]) * (1.0f + kMargin) : __int_as_float(0x7f800000);
+}
+
+// FIRST: reduce the FP64 cost; otherwise the first candidate that has it.
+template <bool FIRST>
+__device__ __forceinline__ void big_consider(const Params& P, const Big& B, const BigState& st,
+                                             const uint32_t* __restrict__ tb, const float* __restrict__ nlo,
+                                             const float* __restrict__ nhi, uint32_t n, int a, float p,
+                                             const Counts& k) {
+  int side;
+  const double cst = score64(P, nlo, nhi, n, B.eGn[n], a, p, k, &side);
+  if (!(cst < init_cost(P, B.eGn[n], tb[n + 1] - tb[n]))) return;
+  const unsigned long long o = ordd(cst);
+  if (FIRST) {
+    if (o < st.best64[n]) atomicMin(&st.best64[n], o);
+  } else if (o == st.best64[n]) {
+    atomicMin(&st.key[n], (unsigned long long)cand_key(a, p, side));
+  }
+}
+
+// Pass 2 (FIRST) and 4: events within the margin; pass 2 also gathers the
+// hull of the gaps whose bound is.
+template <bool FIRST>
+__global__ void k_event_exact(Params P, Big B, const uint32_t* __restrict__ tb, const float* __restrict__ nlo,
+                              const float* __restrict__ nhi, const float2* __restrict__ scores, BigState st) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 6 * B.eG) return;
+  const float kInf = __int_as_float(0x7f800000);
+  const bool is_max = i >= 3 * B.eG;
+  const uint64_t key = is_max ? B.kmax[i - 3 * B.eG] : B.kmin[i];
+  int a;
+  uint32_t n;
+  decode(key, B.nb, &a, &n);
+  const float limit = big_limit(P, st, n);
+  const float2 s = scores[i];
+  const uint32_t kp = (uint32_t)key;
+  if (!(s.x > limit) && s.x != kInf) {
+    big_consider<FIRST>(P, B, st, tb, nlo, nhi, n, a, unordf(kp), big_counts(B, a, n, kp));
+    if (FIRST && kp == kZeroKey) {  // the edges at zero say which zero it is
+      atomicMin(&st.hull_lo[3ull * n + a], kp);
+      atomicMax(&st.hull_hi[3ull * n + a], kp);
+    }
+  }
+  if (FIRST && !(s.y > limit) && (s.y != kInf || !P.filter)) {
+    const size_t b = a * B.eG + B.grb[n];
+    const uint32_t G = B.eGn[n];
+    const uint32_t le_mn = upper(B.kmin + b, G, key), le_mx = upper(B.kmax + b, G, key);
+    const uint32_t kn = min(le_mn < G ? (uint32_t)B.kmin[b + le_mn] : 0xFFFFFFFFu,
+                            le_mx < G ? (uint32_t)B.kmax[b + le_mx] : 0xFFFFFFFFu);
+    atomicMin(&st.hull_lo[3ull * n + a], kp);
+    atomicMax(&st.hull_hi[3ull * n + a], kn);
+  }
+}
+
+// Pass 3 (FIRST) and 5: triangle edges inside the hulls.
+template <bool FIRST>
+__global__ void k_edge_exact(Params P, Big B, TriView V, size_t T, const uint32_t* __restrict__ tb,
+                             const float* __restrict__ nlo, const float* __restrict__ nhi, BigState st) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= T) return;
+  const uint32_t n = V.node[t];
+  if (B.eGn[n] == 0u) return;
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t hl = st.hull_lo[3ull * n + a], hh = st.hull_hi[3ull * n + a];
+    if (hl > hh) continue;
+    const float e[2] = {V.lo[a * V.cap + t], V.hi[a * V.cap + t]};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const float p = e[s];
+      const uint32_t kp = ordz(p);
+      if (kp < hl || kp > hh) continue;
+      const Cell c = make_cell(P, nlo, nhi, n, B.eGn[n], tb[n + 1] - tb[n]);
+      if (!in_limits(c, a, p)) continue;
+      const Counts k = big_counts(B, a, n, kp);
+      if (score32(P, c, a, p, k) > big_limit(P, st, n)) continue;
+      big_consider<FIRST>(P, B, st, tb, nlo, nhi, n, a, p, k);
+    }
+  }
+}
+
+__global__ void k_big_init(const Params P, Big B, const uint32_t* __restrict__ tb, uint32_t N, BigState st) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const float init = __double2float_ru(init_cost(P, B.eGn[n], tb[n + 1] - tb[n]));
+  st.best32[n] = init >= 0.0f ? __float_as_uint(init) : 0x7f800000u;
+  st.best64[n] = ~0ull;
+  st.key[n] = ~0ull;
+  for (int a = 0; a < 3; ++a) {
+    st.hull_lo[3ull * n + a] = 0xFFFFFFFFu;
+    st.hull_hi[3ull * n + a] = 0u;
+  }
+}
+
+__global__ void k_big_choose(Big B, uint32_t N, BigState st, Decision* dec, uint32_t* is_split) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N || B.eGn[n] == 0u || st.key[n] == ~0ull) return;
+  dec[n] = key_decision(st.key[n]);
+  is_split[n] = 1u;
+}
+
+// ------------------------------------------------------------ partition
 // Which children a triangle goes to (push_triangles_to_child_vector).
 __device__ __forceinline__ void sides_of(float mn, float mx, const Decision& d, bool* l, bool* r) {
   if (mn != mx) {
@@ -702,31 +1038,35 @@ __device__ __forceinline__ void sides_of(float mn, float mx, const Decision& d, 
   }
 }
 
-__global__ void k_part_flags(const float* __restrict__ lo, const float* __restrict__ hi, size_t cap, size_t T,
-                             const uint32_t* __restrict__ node, const Decision* __restrict__ dec, uint32_t* fl,
-                             uint32_t* fr) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t > T) return;
-  bool l = false, r = false;
-  if (t < T) {
-    const Decision d = dec[node[t]];
-    if (d.axis >= 0) sides_of(lo[d.axis * cap + t], hi[d.axis * cap + t], d, &l, &r);
+struct SideOp {  // left count in the low word, right count in the high word
+  TriView V;
+  const Decision* dec;
+  uint64_t T;
+  __device__ uint64_t operator()(uint64_t t) const {
+    if (t >= T) return 0ull;
+    const Decision d = dec[V.node[t]];
+    if (d.axis < 0) return 0ull;
+    bool l, r;
+    sides_of(V.lo[d.axis * V.cap + t], V.hi[d.axis * V.cap + t], d, &l, &r);
+    return (l ? 1ull : 0ull) | (r ? 1ull << 32 : 0ull);
   }
-  fl[t] = l;
-  fr[t] = r;
-}
+};
+__device__ __forceinline__ uint32_t lo32(uint64_t x) { return (uint32_t)x; }
+__device__ __forceinline__ uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
 
-__global__ void k_child_counts(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ sl,
-                               const uint32_t* __restrict__ sr, const uint32_t* __restrict__ is_split,
-                               const uint32_t* __restrict__ ns, uint32_t N, uint32_t* cc) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N || !is_split[n]) return;
-  cc[2 * ns[n]] = sl[tb[n + 1]] - sl[tb[n]];
-  cc[2 * ns[n] + 1] = sr[tb[n + 1]] - sr[tb[n]];
-}
+struct NodeOp {  // split nodes in the low word, leaf IDs in the high word
+  const uint32_t *is_split, *rb;
+  uint32_t N;
+  __device__ uint64_t operator()(uint64_t n) const {
+    if (n >= N) return 0ull;
+    return is_split[n] ? 1ull : (uint64_t)(rb[n + 1] - rb[n]) << 32;
+  }
+};
 
-// clip_triangle for one straddling triangle (host clip_tri, same arithmetic).
-__device__ bool edge_plane(const float* p0, const float* p1, const float* pp, const float* pn, float* hit) {
+// clip_triangle for one straddling triangle (host clip_tri, same arithmetic):
+// where the segment p0 p1 meets the plane x[axis] = split.
+__device__ __forceinline__ bool edge_plane(const float* p0, const float* p1, const float* pp, const float* pn,
+                                           float* hit) {
   float u[3], w[3];
   u[0] = p1[0] - p0[0];
   u[1] = p1[1] - p0[1];
@@ -745,147 +1085,271 @@ __device__ bool edge_plane(const float* p0, const float* p1, const float* pp, co
   return true;
 }
 
-__device__ void clip_box(const float v[3][3], float lo[3], float hi[3], int axis, float split, int side) {
-  float pn[3] = {0.f, 0.f, 0.f};
-  pn[axis] = 1.f;
-  const float pp[3] = {pn[0] * split, pn[1] * split, pn[2] * split};
-  float L[9][3], R[9][3];
-  int nl = 0, nr = 0;
-  for (int k = 0; k < 3; ++k) {
-    float* dst = (v[k][axis] < split) ? L[nl++] : R[nr++];
-    dst[0] = v[k][0];
-    dst[1] = v[k][1];
-    dst[2] = v[k][2];
-  }
-  const int l0 = nl, r0 = nr;
-  for (int j = 0; j < l0; ++j)
-    for (int k = 0; k < r0; ++k) {
-      float h[3];
-      if (edge_plane(L[j], R[k], pp, pn, h)) {
-        for (int d = 0; d < 3; ++d) {
-          L[nl][d] = h[d];
-          R[nr][d] = h[d];
-        }
-        ++nl;
-        ++nr;
-      }
-    }
-  float(*V)[3] = side == 0 ? L : R;
-  const int nv = side == 0 ? nl : nr;
-  float nlo[3] = {0.f, 0.f, 0.f}, nhi[3] = {0.f, 0.f, 0.f};
-  if (nv > 0) {
-    for (int d = 0; d < 3; ++d) nlo[d] = nhi[d] = V[0][d];
-    for (int j = 1; j < nv; ++j)
-      for (int d = 0; d < 3; ++d) {
-        nlo[d] = ref_min(nlo[d], V[j][d]);
-        nhi[d] = ref_max(nhi[d], V[j][d]);
-      }
+// Box of the part of triangle v on each side of the plane, clamped to the
+// triangle's box [lo, hi]: the side's own vertices in order, then the
+// plane's hits in (left vertex, right vertex) order, shared by both sides.
+struct ClipBox {
+  float lo[2][3], hi[2][3];
+  bool any[2];
+  __device__ __forceinline__ void add(int s, const float* p) {
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      nlo[d] = ref_max(nlo[d], lo[d]);
-      nhi[d] = ref_min(nhi[d], hi[d]);
+      lo[s][d] = any[s] ? ref_min(lo[s][d], p[d]) : p[d];
+      hi[s][d] = any[s] ? ref_max(hi[s][d], p[d]) : p[d];
     }
+    any[s] = true;
   }
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = nlo[d];
-    hi[d] = nhi[d];
+};
+__device__ __forceinline__ void clip_boxes(const float v[3][3], const float lo[3], const float hi[3], int axis,
+                                           float split, ClipBox& C) {
+  const float pn[3] = {axis == 0 ? 1.f : 0.f, axis == 1 ? 1.f : 0.f, axis == 2 ? 1.f : 0.f};
+  const float pp[3] = {pn[0] * split, pn[1] * split, pn[2] * split};
+  bool left[3];
+  C.any[0] = C.any[1] = false;
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) C.lo[s][d] = C.hi[s][d] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    left[k] = pick(v[k], axis) < split;
+    if (left[k]) C.add(0, v[k]);
+    else C.add(1, v[k]);
   }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (j == k) continue;
+      float h[3];
+      if (left[j] && !left[k] && edge_plane(v[j], v[k], pp, pn, h)) {
+        C.add(0, h);
+        C.add(1, h);
+      }
+    }
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+    if (C.any[s])
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        C.lo[s][d] = ref_max(C.lo[s][d], lo[d]);
+        C.hi[s][d] = ref_min(C.hi[s][d], hi[d]);
+      }
 }
 
-__global__ void k_part_scatter(const float* __restrict__ v, const float* __restrict__ lo, const float* __restrict__ hi,
-                               const uint32_t* __restrict__ gid, const uint32_t* __restrict__ node, size_t cap,
-                               size_t T, const uint32_t* __restrict__ tb, const Decision* __restrict__ dec,
-                               const uint32_t* __restrict__ ns, const uint32_t* __restrict__ sl,
-                               const uint32_t* __restrict__ sr, const uint32_t* __restrict__ ntb, float* v2,
-                               float* lo2, float* hi2, uint32_t* gid2, uint32_t* node2, size_t cap2) {
+// Triangles to their children.  sc: exclusive scan of SideOp; a split node's
+// children take consecutive ranges, so a left slot is the left count before t
+// plus the right count before the node, a right slot the right count before
+// t plus the left count up to the node's end.
+__global__ void k_part_scatter(TriView V, size_t T, const float* __restrict__ g, const float* __restrict__ kiso,
+                               const uint32_t* __restrict__ tb, const Decision* __restrict__ dec,
+                               const uint64_t* __restrict__ nsc, const uint64_t* __restrict__ sc, float* lo2,
+                               float* hi2, uint32_t* tri2, uint32_t* node2, size_t cap2) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
-  const uint32_t n = node[t];
+  const uint32_t n = V.node[t];
   const Decision d = dec[n];
   if (d.axis < 0) return;
-  bool gl, gr;
-  sides_of(lo[d.axis * cap + t], hi[d.axis * cap + t], d, &gl, &gr);
-  if (!gl && !gr) return;
-  float vv[3][3], blo[3], bhi[3];
-  for (int l = 0; l < 3; ++l)
-    for (int i = 0; i < 3; ++i) vv[l][i] = v[(3 * l + i) * cap + t];
+  float blo[3], bhi[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    blo[a] = lo[a * cap + t];
-    bhi[a] = hi[a * cap + t];
+    blo[a] = V.lo[a * V.cap + t];
+    bhi[a] = V.hi[a * V.cap + t];
   }
-  const bool straddle = blo[d.axis] < d.split && bhi[d.axis] > d.split;
-  for (int s = 0; s < 2; ++s) {
-    if (s == 0 ? !gl : !gr) continue;
-    const uint32_t child = 2 * ns[n] + s;
-    const size_t pos = ntb[child] + (s == 0 ? (sl[t] - sl[tb[n]]) : (sr[t] - sr[tb[n]]));
-    float clo[3] = {blo[0], blo[1], blo[2]}, chi[3] = {bhi[0], bhi[1], bhi[2]};
-    if (straddle) clip_box(vv, clo, chi, d.axis, d.split, s);
-    for (int k = 0; k < 9; ++k) v2[k * cap2 + pos] = v[k * cap + t];
+  const float mn = pick(blo, d.axis), mx = pick(bhi, d.axis);
+  bool go[2];
+  sides_of(mn, mx, d, &go[0], &go[1]);
+  if (!go[0] && !go[1]) return;
+  const uint32_t tri = V.tri[t];
+  const uint64_t s = sc[t];
+  const size_t pos[2] = {(size_t)lo32(s) + hi32(sc[tb[n]]), (size_t)hi32(s) + lo32(sc[tb[n + 1]])};
+  const uint32_t child = 2 * lo32(nsc[n]);
+  ClipBox C;
+  if (mn < d.split && mx > d.split) {
+    float v[3][3];
+    proxy_triangle(g, kiso, tri, v);
+    clip_boxes(v, blo, bhi, d.axis, d.split, C);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        C.lo[k][a] = blo[a];
+        C.hi[k][a] = bhi[a];
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (!go[k]) continue;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo2[a * cap2 + pos] = clo[a];
-      hi2[a * cap2 + pos] = chi[a];
+      lo2[a * cap2 + pos[k]] = C.lo[k][a];
+      hi2[a * cap2 + pos[k]] = C.hi[k][a];
     }
-    gid2[pos] = gid[t];
-    node2[pos] = child;
+    tri2[pos[k]] = tri;
+    node2[pos[k]] = child + k;
   }
 }
 
-__global__ void k_child_boxes(const float* __restrict__ nlo, const float* __restrict__ nhi,
-                              const Decision* __restrict__ dec, const uint32_t* __restrict__ ns, uint32_t N,
-                              float* clo, float* chi) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N || dec[n].axis < 0) return;
-  for (int s = 0; s < 2; ++s) {
-    const uint32_t c = 2 * ns[n] + s;
-    for (int d = 0; d < 3; ++d) {
-      clo[3 * c + d] = nlo[3 * n + d];
-      chi[3 * c + d] = nhi[3 * n + d];
-    }
-    if (s == 0) chi[3 * c + dec[n].axis] = dec[n].split;
-    else clo[3 * c + dec[n].axis] = dec[n].split;
-  }
-}
-
-__global__ void k_leaf_sizes(const uint32_t* __restrict__ is_split, const uint32_t* __restrict__ G, uint32_t N,
-                             uint32_t* lsz) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n < N) lsz[n] = is_split[n] ? 0u : G[n];
-}
-
-__global__ void k_leaf_ids(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node, uint32_t R,
-                           const uint32_t* __restrict__ gid, const uint32_t* __restrict__ is_split,
-                           const uint32_t* __restrict__ rb, const uint32_t* __restrict__ loff, uint32_t* pool) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t n = run_node[r];
-  if (is_split[n]) return;
-  pool[loff[n] + (r - rb[n])] = gid[run_start[r]];
-}
-
-// Host record of one node, breadth-first numbering.
+// A node of the finished level, as the numbering reads it.
 struct Rec {
-  int axis;
-  float split;
-  uint32_t first_child;  // global BFS index of the left child
+  int axis;        // -1: leaf
+  uint32_t split;  // split bits
+  uint32_t child;  // index of the left child in the next level
   uint32_t leaf_off, leaf_cnt;
 };
 
+// Sizes of the next level, read back once per level.
+struct LevelSum {
+  unsigned long long triangles;
+  uint32_t n_split, leaf_ids, max_ids;  // max_ids: most IDs in a split node
+};
+
+// Per node: its record, and for split nodes the children's boxes and first
+// triangles.
+__global__ void k_children(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb, uint32_t N,
+                           const Decision* __restrict__ dec, const uint64_t* __restrict__ nsc,
+                           const uint64_t* __restrict__ sc, uint32_t pool_base, const float* __restrict__ nlo,
+                           const float* __restrict__ nhi, float* clo, float* chi, uint32_t* ctb, Rec* rec,
+                           LevelSum* sum) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t ids = 0;
+  if (n < N) {
+    const Decision d = dec[n];
+    const uint64_t e = nsc[n];
+    const uint32_t G = rb[n + 1] - rb[n];
+    Rec r;
+    r.axis = d.axis;
+    r.split = __float_as_uint(d.split);
+    r.child = 2 * lo32(e);
+    r.leaf_off = pool_base + hi32(e);
+    r.leaf_cnt = d.axis < 0 ? G : 0u;
+    rec[n] = r;
+    if (d.axis >= 0) {
+      ids = G;
+      const uint64_t s0 = sc[tb[n]], s1 = sc[tb[n + 1]];
+      ctb[r.child] = lo32(s0) + hi32(s0);
+      ctb[r.child + 1] = lo32(s1) + hi32(s0);
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float l = nlo[3ull * n + k], h = nhi[3ull * n + k];
+          clo[3ull * (r.child + s) + k] = s == 1 && k == d.axis ? d.split : l;
+          chi[3ull * (r.child + s) + k] = s == 0 && k == d.axis ? d.split : h;
+        }
+    }
+    if (n == N - 1) {
+      const uint64_t ne = nsc[N], se = sc[tb[N]];
+      sum->triangles = (unsigned long long)lo32(se) + hi32(se);
+      sum->n_split = lo32(ne);
+      sum->leaf_ids = hi32(ne);
+      ctb[2 * lo32(ne)] = lo32(se) + hi32(se);
+    }
+  }
+  ids = __reduce_max_sync(0xFFFFFFFFu, ids);
+  if ((threadIdx.x & 31) == 0 && ids) atomicMax(&sum->max_ids, ids);
+}
+
+__global__ void k_leaf_ids(const uint32_t* __restrict__ run_start, const uint32_t* __restrict__ run_node,
+                           const uint32_t* __restrict__ tri, const uint32_t* __restrict__ ids,
+                           const uint32_t* __restrict__ is_split, const uint32_t* __restrict__ rb, uint32_t N,
+                           const uint64_t* __restrict__ nsc, uint32_t* pool) {
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < rb[N]; r += gridDim.x * blockDim.x) {
+    const uint32_t n = run_node[r];
+    if (is_split[n]) continue;
+    pool[hi32(nsc[n]) + (r - rb[n])] = ids[tri[run_start[r]] / kFaces];
+  }
+}
+
+// ------------------------------------------------------------ numbering
+// Bottom up: inner nodes and leaf IDs of every subtree.
+__global__ void k_subtree(const Rec* __restrict__ rec, uint32_t N, const uint2* __restrict__ below, uint2* own,
+                          uint32_t* max_leaf) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t leaf = 0;
+  if (n < N) {
+    const Rec r = rec[n];
+    if (r.axis < 0) {
+      own[n] = make_uint2(0u, r.leaf_cnt);
+      leaf = r.leaf_cnt;
+    } else {
+      const uint2 a = below[r.child], b = below[r.child + 1];
+      own[n] = make_uint2(1u + a.x + b.x, a.y + b.y);
+    }
+  }
+  leaf = __reduce_max_sync(0xFFFFFFFFu, leaf);
+  if ((threadIdx.x & 31) == 0 && leaf) atomicMax(max_leaf, leaf);
+}
+
+// Where a node goes: its slot, the number of inner nodes before it and of
+// leaf IDs before it in depth-first, left-first order.
+struct Place {
+  uint32_t slot, rank, ids;
+};
+// Top down: the reference allocates a child pair when it pops the parent, so
+// the pair of the inner node of rank k is (1 + 2k, 2 + 2k).
+__global__ void k_place(const Rec* __restrict__ rec, uint32_t N, const uint2* __restrict__ below,
+                        const Place* __restrict__ at, Place* next, uint2* nodes, const uint32_t* __restrict__ pool,
+                        uint32_t* offsets) {
+  const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // 8 lanes per node copy a leaf's IDs
+  const uint32_t lane = threadIdx.x & 7u;
+  if (n >= N) return;
+  const Rec r = rec[n];
+  const Place p = at[n];
+  if (r.axis < 0) {
+    if (lane == 0) nodes[p.slot] = make_uint2((r.leaf_cnt << 3) | 3u, p.ids);
+    for (uint32_t i = lane; i < r.leaf_cnt; i += 8) offsets[p.ids + i] = pool[r.leaf_off + i];
+  } else if (lane == 0) {
+    const uint32_t c = 1u + 2u * p.rank;
+    const uint2 l = below[r.child];
+    nodes[p.slot] = make_uint2((c << 3) | (uint32_t)r.axis, r.split);
+    next[r.child] = Place{c, p.rank + 1u, p.ids};
+    next[r.child + 1] = Place{c + 1u, p.rank + 1u + l.x, p.ids + l.y};
+  }
+}
+
+template <int NT, int CAP>
+void launch_search_block(Stream& S, const Params& P, const uint32_t* list, const uint32_t* count, uint32_t most,
+                         const uint32_t* tb, const uint32_t* rb, const uint32_t* run_start, const TriView& V,
+                         const float* nlo, const float* nhi, Decision* dec, uint32_t* is_split) {
+  const int bytes = (int)sizeof(SearchMem<NT, CAP>);
+  S.check(cudaFuncSetAttribute(k_search_block<NT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  const unsigned grid = std::max(1u, std::min(most, 4096u));
+  k_search_block<NT, CAP><<<grid, NT, bytes, S.s>>>(P, list, count, tb, rb, run_start, V, nlo, nhi, dec, is_split);
+}
+
 }  // namespace
 
-int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, HostTree& out, BuildStats* stats,
+int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_tree* out, BuildStats* stats,
                    std::string& err) {
   using clk = std::chrono::steady_clock;
   auto t0 = clk::now();
+  memset(out, 0, sizeof(*out));
+  // the host arrays of the result: released on every exit but the last
+  struct HostArrays {
+    void *nodes = nullptr, *offsets = nullptr, *valid = nullptr;
+    ~HostArrays() {
+      free(nodes);
+      free(offsets);
+      free(valid);
+    }
+  } H;
+  H.valid = calloc((size_t)n + 1, 1);
+  if (!H.valid) throw std::bad_alloc();
+  uint8_t* valid = static_cast<uint8_t*>(H.valid);
   // per-Gaussian proxy scale on the host (the host builder's function)
   std::vector<float> gv;
   std::vector<float> kiso;
   std::vector<uint32_t> ids;
   gv.reserve((size_t)n * 10);
-  out.valid.assign(n, 0);
+  kiso.reserve(n);
+  ids.reserve(n);
   for (uint32_t i = 0; i < n; ++i) {
     const float* g = gauss + (size_t)i * 64;
     float k;
     if (!proxy_kiso(g, &k)) continue;
-    out.valid[i] = 1;
+    valid[i] = 1;
     gv.insert(gv.end(), {g[0], g[1], g[2], g[4], g[5], g[6], g[8], g[9], g[10], g[11]});
     kiso.push_back(k);
     ids.push_back(i);
@@ -895,281 +1359,267 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, HostTr
     err = "every Gaussian is below the opacity cut; nothing to build";
     return KDGR_ERR_INVALID_ARG;
   }
+  if ((uint64_t)n_valid * kFaces > 0xFFFFFFF0ull) {
+    err = "more than 2^32 proxy triangles";
+    return KDGR_ERR_LIMIT;
+  }
   bool limit_hit = false;
   Stream S;
-  S.check(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
-  {
-    int dev = 0;
-    S.check(cudaGetDevice(&dev));
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    S.check(cudaMemPoolCreate(&S.pool, &props));
-    uint64_t keep = UINT64_MAX;
-    if (S.pool) S.check(cudaMemPoolSetAttribute(S.pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  }
-  S.check(cudaMemcpyToSymbolAsync(c_ico_v, kIcosaVerts, sizeof kIcosaVerts, 0, cudaMemcpyHostToDevice, S.s));
-  S.check(cudaMemcpyToSymbolAsync(c_ico_f, kIcosaFaces, sizeof kIcosaFaces, 0, cudaMemcpyHostToDevice, S.s));
-  const Params P{bp.max_level, bp.force_split, bp.isect_cost, bp.sah_mode, bp.sort_cost};
-  std::vector<Rec> recs;  // all nodes, breadth first
-  DBuf<uint32_t> pool;
+  int dev = 0;
+  S.check(cudaGetDevice(&dev));
+  if (S.err == cudaSuccess) S.check(pool_enter(dev, &S.pool));
+  const bool in_pool = S.pool != nullptr;
+  if (in_pool) S.check(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
+  const Params P{bp.max_level,  bp.force_split, bp.isect_cost,
+                 bp.sah_mode,   bp.sort_cost,   (bp.isect_cost >= 0.0f && bp.sort_cost >= 0.0f) ? 1 : 0};
+  uint32_t depth = 0, n_leaves = 0, max_leaf = 0, n_nodes = 0;
   size_t pool_used = 0;
-  uint32_t depth = 0;
   float box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};
-  {
+  auto t2 = t0;
+  if (S.err == cudaSuccess) {
+    S.check(cudaMemcpyToSymbolAsync(c_ico_v, kIcosaVerts, sizeof kIcosaVerts, 0, cudaMemcpyHostToDevice, S.s));
+    S.check(cudaMemcpyToSymbolAsync(c_ico_f, kIcosaFaces, sizeof kIcosaFaces, 0, cudaMemcpyHostToDevice, S.s));
     DBuf<float> d_g(S, gv.size()), d_k(S, kiso.size());
     DBuf<uint32_t> d_ids(S, ids.size());
     S.check(cudaMemcpyAsync(d_g.p, gv.data(), gv.size() * 4, cudaMemcpyHostToDevice, S.s));
     S.check(cudaMemcpyAsync(d_k.p, kiso.data(), kiso.size() * 4, cudaMemcpyHostToDevice, S.s));
     S.check(cudaMemcpyAsync(d_ids.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, S.s));
-    size_t T = (size_t)n_valid * 20;
+    size_t T = (size_t)n_valid * kFaces;
     TriSet cur;
     cur.alloc(S, T);
-    k_proxy<<<grid_for(T, 256), 256, 0, S.s>>>(d_g.p, d_k.p, d_ids.p, n_valid, cur.v.p, cur.lo.p, cur.hi.p,
-                                               cur.gid.p, cur.node.p, cur.cap);
-    S.check(cudaGetLastError());
     DBuf<uint32_t> d_box(S, 6);
-    const uint32_t box_init[6] = {0xFFFFFFFFu, 0, 0xFFFFFFFFu, 0, 0xFFFFFFFFu, 0};
-    S.check(cudaMemcpyAsync(d_box.p, box_init, sizeof box_init, cudaMemcpyHostToDevice, S.s));
-    k_scene_box<<<1024, 256, 0, S.s>>>(cur.v.p, cur.cap, T, d_box.p);
     DBuf<float> nlo(S, 3), nhi(S, 3);
-    k_box_decode<<<1, 32, 0, S.s>>>(d_box.p, nlo.p, nhi.p);
-    S.check(cudaMemcpyAsync(box_lo, nlo.p, 12, cudaMemcpyDeviceToHost, S.s));
-    S.check(cudaMemcpyAsync(box_hi, nhi.p, 12, cudaMemcpyDeviceToHost, S.s));
     DBuf<uint32_t> tb(S, 2);
-    const uint32_t tb0[2] = {0, (uint32_t)T};
-    S.check(cudaMemcpyAsync(tb.p, tb0, 8, cudaMemcpyHostToDevice, S.s));
-    S.check(cudaStreamSynchronize(S.s));
-    uint32_t N = 1;
-    if (T > 0xFFFFFFF0ull) {  // leave through the normal exit so every buffer is freed first
-      err = "more than 2^32 proxy triangles";
-      limit_hit = true;
-      N = 0;
+    if (S.err == cudaSuccess) {
+      k_proxy<<<grid_for(T, 256), 256, 0, S.s>>>(d_g.p, d_k.p, n_valid, cur.lo.p, cur.hi.p, cur.tri.p, cur.node.p,
+                                                 cur.cap);
+      const uint32_t box_init[6] = {0xFFFFFFFFu, 0, 0xFFFFFFFFu, 0, 0xFFFFFFFFu, 0};
+      S.check(cudaMemcpyAsync(d_box.p, box_init, sizeof box_init, cudaMemcpyHostToDevice, S.s));
+      k_scene_box<<<std::min(1024u, grid_for(T, 256)), 256, 0, S.s>>>(view(cur), T, d_box.p);
+      k_box_decode<<<1, 32, 0, S.s>>>(d_box.p, nlo.p, nhi.p);
+      S.check(cudaMemcpyAsync(box_lo, nlo.p, 12, cudaMemcpyDeviceToHost, S.s));
+      S.check(cudaMemcpyAsync(box_hi, nhi.p, 12, cudaMemcpyDeviceToHost, S.s));
+      const uint32_t tb0[2] = {0, (uint32_t)T};
+      S.check(cudaMemcpyAsync(tb.p, tb0, 8, cudaMemcpyHostToDevice, S.s));
+      S.check(cudaGetLastError());
+      S.check(cudaStreamSynchronize(S.s));
     }
     auto t1 = clk::now();
     if (stats) stats->proxy_s = std::chrono::duration<double>(t1 - t0).count();
     if (stats) stats->n_triangles = T;
     if (stats) stats->n_valid = n_valid;
 
-    uint32_t base = 0;  // global BFS index of the level's first node
+    DBuf<uint32_t> pool;
+    DBuf<uint8_t> tmp;  // scan and sort workspace
+    std::vector<DBuf<Rec>> levels;
+    std::vector<uint32_t> level_n;
+    uint32_t N = 1, max_ids = n_valid;
     for (int level = 0; N > 0 && S.err == cudaSuccess; ++level) {
 #ifdef KDGR_BUILD_TRACE  // compile-time diagnostic: per-level wall time and sizes on stderr
       const auto lt0 = clk::now();
-      struct LevelTrace {
-        std::chrono::steady_clock::time_point t0;
-        int level;
-        const uint32_t* n;
-        const size_t* t;
-        ~LevelTrace() {
-          fprintf(stderr, "[kdbuild_gpu] level %d: %u nodes, %zu triangles, %.2f ms\n", level, *n, *t,
-                  std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
-        }
-      };
-      const uint32_t n_in = N;
-      const size_t t_in = T;
-      LevelTrace trace_guard{lt0, level, &n_in, &t_in};
+      fprintf(stderr, "[kdbuild_gpu] level %d: %u nodes, %zu triangles, at most %u IDs", level, N, T, max_ids);
 #endif
       depth = (uint32_t)level;
-      int nb = 1;
-      while ((1u << nb) < N) ++nb;
+      const TriView V = view(cur);
       // 1. runs of (node, ID)
-      DBuf<uint32_t> flag(S, T + 1), ridx(S, T + 1);
-      k_run_heads<<<grid_for(T + 1, 256), 256, 0, S.s>>>(cur.gid.p, cur.node.p, T, flag.p);
-      exclusive_sum(S, flag.p, ridx.p, T + 1);
-      const uint32_t R = read_one(S, ridx.p + T);
-      DBuf<uint32_t> run_start(S, R + 1), run_node(S, R + 1), G(S, N + 1), rb(S, N + 1);
-      k_run_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(flag.p, ridx.p, cur.node.p, T, run_start.p, run_node.p);
-      k_node_runs<<<grid_for((size_t)N + 1, 128), 128, 0, S.s>>>(tb.p, ridx.p, N, rb.p, G.p);
-      flag.release();
-      ridx.release();
-      // 2. node constants, eligible-node compaction
-      DBuf<NodeConst> nc(S, N);
-      DBuf<uint32_t> eT(S, N + 1), eG(S, N + 1), ctb(S, N + 1), grb(S, N + 1);
-      eT.zero();
-      eG.zero();
-      k_node_setup<<<grid_for(N, 128), 128, 0, S.s>>>(tb.p, G.p, nlo.p, nhi.p, N, level, P, nc.p, eT.p, eG.p);
-      exclusive_sum(S, eT.p, ctb.p, N + 1);
-      exclusive_sum(S, eG.p, grb.p, N + 1);
-      const size_t eTT = read_one(S, ctb.p + N), eGT = read_one(S, grb.p + N);
+      DBuf<uint32_t> ridx(S, T + 1), run_start(S, T + 1), run_node(S, T + 1), rb(S, (size_t)N + 1);
+      if (S.err != cudaSuccess) break;
+      exclusive_sum_of(S, tmp, HeadOp{V.tri, V.node, T}, ridx.p, T + 1);
+      k_run_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(ridx.p, V.node, T, run_start.p, run_node.p);
+      // 2. node classes and split search; large nodes can only appear below a large node
+      const bool may_be_big = max_ids > kBlockIds;
       DBuf<Decision> dec(S, N);
-      DBuf<uint32_t> is_split(S, N + 1);
-      if (eTT > 0) {
-        // 3. keys, sorts, scores
-        DBuf<unsigned long long> ccnt(S, 3 * (size_t)R + 1), coff(S, 3 * (size_t)R + 1);
-        ccnt.zero();
-        k_run_cand_count<<<grid_for(R, 128), 128, 0, S.s>>>(run_start.p, run_node.p, R, T, cur.lo.p, cur.hi.p,
-                                                            cur.cap, nc.p, ccnt.p);
-        exclusive_sum(S, ccnt.p, coff.p, 3 * (size_t)R + 1);
-        ccnt.release();
-        const size_t nc_keys = read_one(S, coff.p + 3 * (size_t)R);
-        DBuf<uint64_t> kc(S, nc_keys), kc_alt(S, nc_keys);
-        k_run_cand_write<<<grid_for(R, 128), 128, 0, S.s>>>(run_start.p, run_node.p, R, T, cur.lo.p, cur.hi.p,
-                                                            cur.cap, nc.p, coff.p, nb, kc.p);
-        DBuf<uint64_t> kmin(S, 3 * eGT), kmax(S, 3 * eGT), kpl(S, 3 * eGT), alt(S, 3 * eGT);
-        DBuf<uint32_t> pl_cnt(S, 3 * (size_t)N + 1), plb(S, 3 * (size_t)N + 1);
-        DBuf<unsigned long long> pl_fill(S, 1);
-        pl_cnt.zero();
-        pl_fill.zero();
-        k_run_bounds<<<grid_for(R, 128), 128, 0, S.s>>>(run_start.p, run_node.p, R, T, cur.lo.p, cur.hi.p, cur.cap,
-                                                        nc.p, rb.p, grb.p, eGT, nb, kmin.p, kmax.p, kpl.p, pl_cnt.p,
-                                                        pl_fill.p, N);
-        exclusive_sum(S, pl_cnt.p, plb.p, 3 * (size_t)N + 1);
-        const size_t n_pl = read_one(S, pl_fill.p);
-        const int end_bit = 32 + nb + 2;
-        sort_keys(S, kc, kc_alt, nc_keys, end_bit);
-        kc_alt.release();
-        sort_keys(S, kmin, alt, 3 * eGT, end_bit);
-        sort_keys(S, kmax, alt, 3 * eGT, end_bit);
-        sort_keys(S, kpl, alt, n_pl, end_bit);
-        alt.release();
-        DBuf<double> cost(S, nc_keys);
-        DBuf<uint8_t> side(S, nc_keys);
-        DBuf<unsigned long long> best_bits(S, 3 * (size_t)N), best_idx(S, 3 * (size_t)N);
-        best_bits.fill_ff();
-        best_idx.fill_ff();
-        k_eval<<<grid_for(nc_keys, 256), 256, 0, S.s>>>(kc.p, nc_keys, coff.p, rb.p, R, nb, kmin.p, kmax.p, kpl.p,
-                                                        eGT, grb.p, plb.p, pl_cnt.p, nc.p, N, P, cost.p, side.p,
-                                                        best_bits.p);
-        k_argmin<<<grid_for(nc_keys, 256), 256, 0, S.s>>>(kc.p, cost.p, nc_keys, nb, N, best_bits.p, best_idx.p);
-        k_choose<<<grid_for(N, 128), 128, 0, S.s>>>(nc.p, N, best_bits.p, best_idx.p, kc.p, side.p, dec.p,
-                                                    is_split.p);
-      } else {
-        std::vector<Decision> leafs(N, Decision{-1, 0.f, 0});
-        S.check(cudaMemcpyAsync(dec.p, leafs.data(), N * sizeof(Decision), cudaMemcpyHostToDevice, S.s));
-        is_split.zero();
+      DBuf<uint32_t> is_split(S, (size_t)N + 1), lists(S, 2 * (size_t)N), counts(S, 3), eG;
+      if (may_be_big) {
+        eG.alloc(S, (size_t)N + 1);
+        eG.zero();
       }
-      S.check(cudaGetLastError());
-      // 4. leaves: their run IDs into the pool
-      DBuf<uint32_t> lsz(S, N + 1), loff(S, N + 1);
-      lsz.zero();
-      k_leaf_sizes<<<grid_for(N, 128), 128, 0, S.s>>>(is_split.p, G.p, N, lsz.p);
-      exclusive_sum(S, lsz.p, loff.p, N + 1);
-      const size_t leaf_total = read_one(S, loff.p + N);
-      if (pool_used + leaf_total > pool.n) {
-        DBuf<uint32_t> bigger(S, std::max(pool.n * 2, pool_used + leaf_total + 1024));
-        if (pool_used)
-          S.check(cudaMemcpyAsync(bigger.p, pool.p, pool_used * 4, cudaMemcpyDeviceToDevice, S.s));
-        pool = std::move(bigger);
-      }
-      k_leaf_ids<<<grid_for(R, 256), 256, 0, S.s>>>(run_start.p, run_node.p, R, cur.gid.p, is_split.p, rb.p, loff.p,
-                                                    pool.p + pool_used);
-      // 5. partition into the next level
-      DBuf<uint32_t> ns(S, N + 1);
-      S.check(cudaMemsetAsync(is_split.p + N, 0, 4, S.s));
-      exclusive_sum(S, is_split.p, ns.p, N + 1);
-      const uint32_t n_split = read_one(S, ns.p + N);
-      // host records of this level
-      {
-        std::vector<Decision> hd(N);
-        std::vector<uint32_t> hns(N), hG(N), hloff(N);
-        S.check(cudaMemcpyAsync(hd.data(), dec.p, N * sizeof(Decision), cudaMemcpyDeviceToHost, S.s));
-        S.check(cudaMemcpyAsync(hns.data(), ns.p, N * 4, cudaMemcpyDeviceToHost, S.s));
-        S.check(cudaMemcpyAsync(hG.data(), G.p, N * 4, cudaMemcpyDeviceToHost, S.s));
-        S.check(cudaMemcpyAsync(hloff.data(), loff.p, N * 4, cudaMemcpyDeviceToHost, S.s));
+      if (S.err != cudaSuccess) break;
+      counts.zero();
+      k_node_setup<<<grid_for((size_t)N + 1, 128), 128, 0, S.s>>>(tb.p, ridx.p, N, level, P.max_level, rb.p, dec.p,
+                                                                  is_split.p, lists.p, lists.p + N, counts.p, eG.p);
+      k_search_warp<<<grid_for(N, kSearchWarps), 32 * kSearchWarps, 0, S.s>>>(P, N, level, tb.p, rb.p, run_start.p, V,
+                                                                              nlo.p, nhi.p, dec.p, is_split.p);
+      if (max_ids > kWarpIds)
+        launch_search_block<128, (int)kMidIds>(S, P, lists.p, counts.p, N, tb.p, rb.p, run_start.p, V, nlo.p, nhi.p,
+                                               dec.p, is_split.p);
+      if (max_ids > kMidIds)
+        launch_search_block<512, (int)kBlockIds>(S, P, lists.p + N, counts.p + 1, N, tb.p, rb.p, run_start.p, V,
+                                                 nlo.p, nhi.p, dec.p, is_split.p);
+      if (may_be_big) {
+        DBuf<uint32_t> grb(S, (size_t)N + 1);
+        if (S.err != cudaSuccess) break;
+        exclusive_sum(S, tmp, (const uint32_t*)eG.p, grb.p, (size_t)N + 1);
+        uint32_t eGT = 0;
+        S.check(cudaMemcpyAsync(&eGT, grb.p + N, 4, cudaMemcpyDeviceToHost, S.s));
         S.check(cudaStreamSynchronize(S.s));
-        for (uint32_t i = 0; i < N; ++i) {
-          Rec r;
-          r.axis = hd[i].axis;
-          r.split = hd[i].split;
-          r.first_child = base + N + 2 * hns[i];
-          r.leaf_off = (uint32_t)(pool_used + hloff[i]);
-          r.leaf_cnt = hd[i].axis < 0 ? hG[i] : 0;
-          recs.push_back(r);
+        if (eGT > 0) {
+          Big B{};
+          B.grb = grb.p;
+          B.eGn = eG.p;
+          B.eG = eGT;
+          B.nb = 1;
+          while ((1ull << B.nb) < N) ++B.nb;
+          DBuf<uint64_t> kmin(S, 3 * (size_t)eGT), kmax(S, 3 * (size_t)eGT), kpl(S, 3 * (size_t)eGT),
+              alt(S, 3 * (size_t)eGT);
+          DBuf<uint32_t> pl_fill(S, 1), best32(S, N), hull(S, 6 * (size_t)N);
+          DBuf<unsigned long long> best64(S, 2 * (size_t)N);
+          DBuf<float2> scores(S, 6 * (size_t)eGT);
+          if (S.err != cudaSuccess) break;
+          pl_fill.zero();
+          k_run_bounds<<<grid_for(T, 128), 128, 0, S.s>>>(run_start.p, run_node.p, rb.p, N, T, V, B, kmin.p, kmax.p,
+                                                          kpl.p, pl_fill.p);
+          S.check(cudaMemcpyAsync(&B.n_pl, pl_fill.p, 4, cudaMemcpyDeviceToHost, S.s));
+          const int end_bit = 32 + B.nb + 2;
+          sort_keys(S, tmp, kmin, alt, 3 * (size_t)eGT, end_bit);
+          sort_keys(S, tmp, kmax, alt, 3 * (size_t)eGT, end_bit);
+          S.check(cudaStreamSynchronize(S.s));
+          sort_keys(S, tmp, kpl, alt, B.n_pl, end_bit);
+          B.kmin = kmin.p;
+          B.kmax = kmax.p;
+          B.kpl = kpl.p;
+          BigState st{best32.p, best64.p, best64.p + N, hull.p, hull.p + 3 * (size_t)N};
+          const unsigned ge = grid_for(6 * (size_t)eGT, 256), gt = grid_for(T, 256), gn = grid_for(N, 128);
+          k_big_init<<<gn, 128, 0, S.s>>>(P, B, tb.p, N, st);
+          k_event_scores<<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
+          k_event_exact<true><<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
+          k_edge_exact<true><<<gt, 256, 0, S.s>>>(P, B, V, T, tb.p, nlo.p, nhi.p, st);
+          k_event_exact<false><<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
+          k_edge_exact<false><<<gt, 256, 0, S.s>>>(P, B, V, T, tb.p, nlo.p, nhi.p, st);
+          k_big_choose<<<gn, 128, 0, S.s>>>(B, N, st, dec.p, is_split.p);
         }
       }
-      pool_used += leaf_total;
-      if (n_split == 0) break;
-      const uint32_t N2 = 2 * n_split;
-      DBuf<uint32_t> fl(S, T + 1), fr(S, T + 1), sl(S, T + 1), sr(S, T + 1);
-      k_part_flags<<<grid_for(T + 1, 256), 256, 0, S.s>>>(cur.lo.p, cur.hi.p, cur.cap, T, cur.node.p, dec.p, fl.p,
-                                                          fr.p);
-      exclusive_sum(S, fl.p, sl.p, T + 1);
-      exclusive_sum(S, fr.p, sr.p, T + 1);
-      fl.release();
-      fr.release();
-      DBuf<uint32_t> cc(S, N2 + 1), ntb(S, N2 + 1);
-      cc.zero();
-      k_child_counts<<<grid_for(N, 128), 128, 0, S.s>>>(tb.p, sl.p, sr.p, is_split.p, ns.p, N, cc.p);
-      exclusive_sum(S, cc.p, ntb.p, N2 + 1);
-      const size_t T2 = read_one(S, ntb.p + N2);
-      if (T2 > 0xFFFFFFF0ull) {
-        err = "more than 2^32 triangle references in one level";
-        limit_hit = true;
-        break;
-      }
-      TriSet nxt;
-      nxt.alloc(S, std::max<size_t>(T2, 1));
-      k_part_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(cur.v.p, cur.lo.p, cur.hi.p, cur.gid.p, cur.node.p, cur.cap,
-                                                        T, tb.p, dec.p, ns.p, sl.p, sr.p, ntb.p, nxt.v.p, nxt.lo.p,
-                                                        nxt.hi.p, nxt.gid.p, nxt.node.p, nxt.cap);
-      DBuf<float> clo(S, 3 * (size_t)N2), chi(S, 3 * (size_t)N2);
-      k_child_boxes<<<grid_for(N, 128), 128, 0, S.s>>>(nlo.p, nhi.p, dec.p, ns.p, N, clo.p, chi.p);
       S.check(cudaGetLastError());
+      // 3. children: node numbers, leaf ID ranges, triangle ranges
+      DBuf<uint64_t> nsc(S, (size_t)N + 1), sc(S, T + 1);
+      DBuf<Rec> rec(S, N);
+      DBuf<float> clo(S, 6 * (size_t)N), chi(S, 6 * (size_t)N);
+      DBuf<uint32_t> ctb(S, 2 * (size_t)N + 1);
+      DBuf<LevelSum> d_sum(S, 1);
+      if (S.err != cudaSuccess) break;
+      d_sum.zero();
+      exclusive_sum_of(S, tmp, NodeOp{is_split.p, rb.p, N}, nsc.p, (size_t)N + 1);
+      exclusive_sum_of(S, tmp, SideOp{V, dec.p, T}, sc.p, T + 1);
+      k_children<<<grid_for(N, 128), 128, 0, S.s>>>(tb.p, rb.p, N, dec.p, nsc.p, sc.p, (uint32_t)pool_used, nlo.p,
+                                                    nhi.p, clo.p, chi.p, ctb.p, rec.p, d_sum.p);
+      LevelSum sum{};
+      S.check(cudaMemcpyAsync(&sum, d_sum.p, sizeof sum, cudaMemcpyDeviceToHost, S.s));
       S.check(cudaStreamSynchronize(S.s));
-      cur = std::move(nxt);
-      nlo = std::move(clo);
-      nhi = std::move(chi);
-      tb = std::move(ntb);
-      base += N;
-      N = N2;
-      T = T2;
+      if (S.err != cudaSuccess) break;
+      // 4. leaves: their run IDs into the pool
+      if (pool_used + sum.leaf_ids > pool.n) {
+        DBuf<uint32_t> bigger(S, std::max(pool.n * 2, pool_used + sum.leaf_ids + 1024));
+        if (pool_used && S.err == cudaSuccess)
+          S.check(cudaMemcpyAsync(bigger.p, pool.p, pool_used * 4, cudaMemcpyDeviceToDevice, S.s));
+        pool = std::move(bigger);
+        if (S.err != cudaSuccess) break;
+      }
+      if (sum.leaf_ids)
+        k_leaf_ids<<<std::min(grid_for(T, 256), 4096u), 256, 0, S.s>>>(run_start.p, run_node.p, V.tri, d_ids.p,
+                                                                       is_split.p, rb.p, N, nsc.p, pool.p + pool_used);
+      pool_used += sum.leaf_ids;
+      levels.push_back(std::move(rec));
+      level_n.push_back(N);
+      // 5. partition into the next level
+      if (sum.n_split > 0) {
+        if (sum.triangles > 0xFFFFFFF0ull || pool_used > 0xFFFFFFF0ull) {
+          err = "more than 2^32 triangle references in one level";
+          limit_hit = true;
+          break;
+        }
+        TriSet nxt;
+        nxt.alloc(S, std::max<size_t>(sum.triangles, 1));
+        if (S.err != cudaSuccess) break;
+        k_part_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(V, T, d_g.p, d_k.p, tb.p, dec.p, nsc.p, sc.p, nxt.lo.p,
+                                                          nxt.hi.p, nxt.tri.p, nxt.node.p, nxt.cap);
+        S.check(cudaGetLastError());
+        cur = std::move(nxt);
+        nlo = std::move(clo);
+        nhi = std::move(chi);
+        tb = std::move(ctb);
+      }
+      N = 2 * sum.n_split;
+      T = sum.triangles;
+      max_ids = sum.max_ids;
+#ifdef KDGR_BUILD_TRACE
+      cudaStreamSynchronize(S.s);
+      fprintf(stderr, ", %.2f ms\n", std::chrono::duration<double, std::milli>(clk::now() - lt0).count());
+#endif
     }
+    // number as the reference allocates: child pairs in depth-first,
+    // left-first order; leaf ID lists in the same order
+    if (S.err == cudaSuccess && !limit_hit) {
+      const int L = (int)levels.size();
+      std::vector<DBuf<uint2>> sub(L);
+      DBuf<uint32_t> d_max(S, 1);
+      d_max.zero();
+      for (int l = L - 1; l >= 0 && S.err == cudaSuccess; --l) {
+        sub[l].alloc(S, level_n[l]);
+        if (S.err != cudaSuccess) break;
+        k_subtree<<<grid_for(level_n[l], 128), 128, 0, S.s>>>(levels[l].p, level_n[l],
+                                                              l + 1 < L ? sub[l + 1].p : nullptr, sub[l].p, d_max.p);
+      }
+      uint2 total = make_uint2(0u, 0u);
+      if (S.err == cudaSuccess) {
+        S.check(cudaMemcpyAsync(&total, sub[0].p, sizeof total, cudaMemcpyDeviceToHost, S.s));
+        S.check(cudaMemcpyAsync(&max_leaf, d_max.p, 4, cudaMemcpyDeviceToHost, S.s));
+        S.check(cudaStreamSynchronize(S.s));
+      }
+      t2 = clk::now();
+      if (S.err == cudaSuccess) {
+        n_leaves = total.x + 1u;
+        n_nodes = 1u + 2u * total.x;
+        DBuf<uint2> d_nodes(S, n_nodes);
+        DBuf<uint32_t> d_off(S, pool_used + 1);
+        DBuf<Place> at(S, 1), next;
+        at.zero();  // the root: slot 0, no inner node and no ID before it
+        for (int l = 0; l < L && S.err == cudaSuccess; ++l) {
+          next.alloc(S, l + 1 < L ? level_n[l + 1] : 1);
+          if (S.err != cudaSuccess) break;
+          k_place<<<grid_for(8ull * level_n[l], 256), 256, 0, S.s>>>(levels[l].p, level_n[l],
+                                                                     l + 1 < L ? sub[l + 1].p : nullptr, at.p, next.p,
+                                                                     d_nodes.p, pool.p, d_off.p);
+          at = std::move(next);
+        }
+        S.check(cudaGetLastError());
+        H.nodes = malloc(8ull * n_nodes + 4);
+        H.offsets = malloc(4 * pool_used + 4);
+        if (H.nodes && H.offsets && S.err == cudaSuccess) {
+          S.check(cudaMemcpyAsync(H.nodes, d_nodes.p, 8ull * n_nodes, cudaMemcpyDeviceToHost, S.s));
+          if (pool_used)
+            S.check(cudaMemcpyAsync(H.offsets, d_off.p, 4 * pool_used, cudaMemcpyDeviceToHost, S.s));
+        }
+      }
+    }
+    S.check(cudaStreamSynchronize(S.s));
+  }  // device buffers are returned to the pool here
+  if (S.s) {
+    cudaStreamSynchronize(S.s);
+    cudaStreamDestroy(S.s);
   }
-  std::vector<uint32_t> hpool(pool_used);
-  if (pool_used)
-    S.check(cudaMemcpyAsync(hpool.data(), pool.p, pool_used * 4, cudaMemcpyDeviceToHost, S.s));
-  pool.release();
-  S.check(cudaStreamSynchronize(S.s));
+  if (in_pool) pool_leave(dev);
   const cudaError_t e = S.err;
-  cudaStreamDestroy(S.s);
-  if (S.pool) cudaMemPoolDestroy(S.pool);
   if (limit_hit && e == cudaSuccess) return KDGR_ERR_LIMIT;
   if (e != cudaSuccess) {
+    cudaGetLastError();
     if (err.empty()) err = std::string("CUDA error in the device build: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? KDGR_ERR_OUT_OF_MEMORY : KDGR_ERR_CUDA;
   }
-  auto t2 = clk::now();
-  // number as the reference allocates: child pairs in depth-first,
-  // left-first order; leaf ID lists appended in the same order
-  out.nodes.assign(2, 0);
-  out.offsets.clear();
-  out.offsets.reserve(pool_used);
-  uint32_t n_leaves = 0, max_leaf = 0;
-  struct Item {
-    uint32_t rec, slot;
-  };
-  std::vector<Item> st{{0, 0}};
-  while (!st.empty()) {
-    const Item it = st.back();
-    st.pop_back();
-    const Rec& r = recs[it.rec];
-    if (r.axis < 0) {
-      out.nodes[2 * it.slot] = (r.leaf_cnt << 3) | 3u;
-      out.nodes[2 * it.slot + 1] = (uint32_t)out.offsets.size();
-      out.offsets.insert(out.offsets.end(), hpool.begin() + r.leaf_off, hpool.begin() + r.leaf_off + r.leaf_cnt);
-      ++n_leaves;
-      max_leaf = std::max(max_leaf, r.leaf_cnt);
-    } else {
-      const uint32_t c = (uint32_t)(out.nodes.size() / 2);
-      out.nodes.resize(out.nodes.size() + 4, 0);
-      uint32_t bits;
-      memcpy(&bits, &r.split, 4);
-      out.nodes[2 * it.slot] = (c << 3) | (uint32_t)r.axis;
-      out.nodes[2 * it.slot + 1] = bits;
-      st.push_back({r.first_child + 1, c + 1});
-      st.push_back({r.first_child, c});
-    }
+  if (!H.nodes || !H.offsets) throw std::bad_alloc();
+  out->nodes = static_cast<uint32_t*>(H.nodes);
+  out->offsets = static_cast<uint32_t*>(H.offsets);
+  out->valid = valid;
+  H.nodes = H.offsets = H.valid = nullptr;
+  out->n_nodes = n_nodes;
+  out->n_offsets = (uint32_t)pool_used;
+  for (int a = 0; a < 3; ++a) {
+    out->aabb[a] = box_lo[a];
+    out->aabb[3 + a] = box_hi[a];
   }
-  out.aabb[0] = box_lo[0];
-  out.aabb[1] = box_lo[1];
-  out.aabb[2] = box_lo[2];
-  out.aabb[3] = box_hi[0];
-  out.aabb[4] = box_hi[1];
-  out.aabb[5] = box_hi[2];
-  out.depth = depth;
-  out.n_leaves = n_leaves;
-  out.max_leaf = max_leaf;
+  out->depth = depth;
+  out->n_leaves = n_leaves;
+  out->max_leaf = max_leaf;
+  out->n_gaussians = n;
   auto t3 = clk::now();
   if (stats) {
     stats->build_s = std::chrono::duration<double>(t2 - t0).count() - stats->proxy_s;

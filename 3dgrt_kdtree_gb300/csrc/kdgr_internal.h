@@ -5,6 +5,8 @@
 #include <string>
 #include <vector>
 
+#include "kdgr.h"
+
 namespace kdgr {
 
 struct BuildParams {
@@ -40,8 +42,9 @@ bool proxy_kiso(const float* g, float* k_iso);
 // Unit icosahedron of the proxy mesh (Kd-treeConverterMain.cpp:1860-1922).
 extern const float kIcosaVerts[12][3];
 extern const int kIcosaFaces[20][3];
-// The same build on the current CUDA device (kdbuild_gpu.cu).
-int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, HostTree& out, BuildStats* stats,
+// The same build on the current CUDA device (kdbuild_gpu.cu); the arrays of
+// `out` are malloc'd on success and null otherwise.
+int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_tree* out, BuildStats* stats,
                    std::string& err);
 
 // .kdt v1 binary (Kd-treeConverter.cpp:297-342, 444-495)

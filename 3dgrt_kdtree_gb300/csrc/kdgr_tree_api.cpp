@@ -344,12 +344,11 @@ int kdgr_build_tree_gpu(const float* gaussians, uint32_t n_gaussians, const kdgr
     set_error("kdgr_build_tree_gpu: max_level must be in [0, 60]");
     return KDGR_ERR_INVALID_ARG;
   }
-  HostTree t;
   BuildStats bs;
   std::string err;
   int rc;
   try {
-    rc = build_tree_gpu(gaussians, n_gaussians, bp, t, &bs, err);
+    rc = build_tree_gpu(gaussians, n_gaussians, bp, out, &bs, err);
   } catch (const std::bad_alloc&) {
     set_error("kdgr_build_tree_gpu: host allocation failed");
     return KDGR_ERR_OUT_OF_MEMORY;
@@ -365,7 +364,7 @@ int kdgr_build_tree_gpu(const float* gaussians, uint32_t n_gaussians, const kdgr
     stats->n_valid = bs.n_valid;
     stats->serialize_s = bs.serialize_s;
   }
-  return fill_out(t, n_gaussians, out);
+  return KDGR_OK;
 }
 
 int kdgr_read_kdt(const char* path, kdgr_tree* out) {
