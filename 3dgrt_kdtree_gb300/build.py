@@ -30,10 +30,12 @@ CU_UNITS = {
     "render_fast.cu": [],
     "kdgr_noalloc.cu": [],
     "scene_pack.cu": ["--fmad=false", "-prec-div=true", "-prec-sqrt=true"],
+    "scene_tree.cu": [],
     "kdbuild_gpu.cu": ["--fmad=false", "-prec-div=true", "-prec-sqrt=true"],
 }
 CPP_UNITS = ["kdbuild.cpp", "kdgr_tree_api.cpp", "kdgr_api.cpp", "kdgr_batch_api.cpp", "kdgr_reference_api.cpp",
-             "kdgr_server.cpp", "kdgr_debug.cpp", "kdgr_ingest.cpp", "kdgr_hybrid.cpp"]
+             "kdgr_server.cpp", "kdgr_debug.cpp", "kdgr_ingest.cpp", "kdgr_hybrid.cpp",
+             "device_pool.cpp"]
 
 
 def _cuda_home() -> str:

@@ -59,10 +59,10 @@
 #include <chrono>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
+#include "device_pool.h"
 #include "kdgr.h"
 #include "kdgr_internal.h"
 
@@ -92,53 +92,9 @@ struct Params {
 };
 
 // ------------------------------------------------------------ device buffers
-// The builder's memory pool of a device.  It keeps what it has mapped while a
-// build runs (the level loop synchronises often, and the device's default
-// pool hands memory back at every synchronisation) and, when the last build
-// on the device has ended, up to kPoolKeep bytes for the next one: mapping
-// and unmapping them took longer than a 10k-Gaussian build's kernels.
-// Allocation and release are stream-ordered, so builds on several threads
-// (each on its own stream) may share it.
-constexpr size_t kPoolKeep = 256ull << 20;
-struct BuildPool {
-  std::mutex mu;
-  cudaMemPool_t pool[64] = {};
-  int users[64] = {};
-};
-BuildPool& build_pool() {
-  static BuildPool p;
-  return p;
-}
-cudaError_t pool_enter(int dev, cudaMemPool_t* out) {
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  BuildPool& B = build_pool();
-  std::lock_guard<std::mutex> lk(B.mu);
-  if (!B.pool[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    if (e != cudaSuccess) return e;
-    uint64_t keep = UINT64_MAX;
-    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return e;
-    }
-    B.pool[dev] = pool;
-  }
-  ++B.users[dev];
-  *out = B.pool[dev];
-  return cudaSuccess;
-}
-void pool_leave(int dev) {
-  BuildPool& B = build_pool();
-  std::lock_guard<std::mutex> lk(B.mu);
-  if (--B.users[dev] == 0) cudaMemPoolTrimTo(B.pool[dev], kPoolKeep);
-}
-
+// Work memory comes from the library's pool of the device (device_pool.h): it
+// keeps what it has mapped while a build runs, where the device's default
+// pool hands memory back at every synchronisation of the level loop.
 struct Stream {
   cudaStream_t s = nullptr;
   cudaMemPool_t pool = nullptr;
@@ -1367,7 +1323,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
   Stream S;
   int dev = 0;
   S.check(cudaGetDevice(&dev));
-  if (S.err == cudaSuccess) S.check(pool_enter(dev, &S.pool));
+  if (S.err == cudaSuccess) S.check(work_pool_enter(dev, &S.pool));
   const bool in_pool = S.pool != nullptr;
   if (in_pool) S.check(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
   const Params P{bp.max_level,  bp.force_split, bp.isect_cost,
@@ -1597,7 +1553,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
     cudaStreamSynchronize(S.s);
     cudaStreamDestroy(S.s);
   }
-  if (in_pool) pool_leave(dev);
+  if (in_pool) work_pool_leave(dev);
   const cudaError_t e = S.err;
   if (limit_hit && e == cudaSuccess) return KDGR_ERR_LIMIT;
   if (e != cudaSuccess) {

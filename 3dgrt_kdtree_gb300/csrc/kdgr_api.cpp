@@ -48,79 +48,6 @@ CamInfo make_caminfo(const kdgr_camera& cam, int width, int height) {
   return c;
 }
 
-void relayout_tree(const uint32_t* nodes, uint32_t n_nodes, int top_levels, std::vector<uint32_t>& out,
-                   uint32_t* top_count) {
-  std::vector<uint32_t> newidx(n_nodes, 0xFFFFFFFFu), order;
-  order.reserve(n_nodes);
-  struct Q {
-    uint32_t old, depth;
-  };
-  std::deque<Q> q;
-  newidx[0] = 0;
-  order.push_back(0);
-  q.push_back({0, 0});
-  std::vector<uint32_t> frontier;  // inner nodes at depth == top_levels
-  while (!q.empty()) {
-    Q it = q.front();
-    q.pop_front();
-    const uint32_t x = nodes[2 * it.old];
-    if ((x & 7u) == 3u) continue;
-    if ((int)it.depth >= top_levels) {
-      frontier.push_back(it.old);
-      continue;
-    }
-    const uint32_t c = x >> 3;
-    newidx[c] = (uint32_t)order.size();
-    order.push_back(c);
-    newidx[c + 1] = (uint32_t)order.size();
-    order.push_back(c + 1);
-    q.push_back({c, it.depth + 1});
-    q.push_back({c + 1, it.depth + 1});
-  }
-  *top_count = (uint32_t)order.size();
-  std::vector<uint32_t> st;
-  for (uint32_t f : frontier) {
-    st.push_back(f);
-    while (!st.empty()) {
-      const uint32_t o = st.back();
-      st.pop_back();
-      const uint32_t x = nodes[2 * o];
-      if ((x & 7u) == 3u) continue;
-      const uint32_t c = x >> 3;
-      newidx[c] = (uint32_t)order.size();
-      order.push_back(c);
-      newidx[c + 1] = (uint32_t)order.size();
-      order.push_back(c + 1);
-      st.push_back(c + 1);
-      st.push_back(c);
-    }
-  }
-  out.assign(2 * (size_t)order.size(), 0);
-  for (size_t n = 0; n < order.size(); ++n) {
-    const uint32_t o = order[n];
-    const uint32_t x = nodes[2 * o], y = nodes[2 * o + 1];
-    if ((x & 7u) == 3u) {
-      out[2 * n] = x;
-      out[2 * n + 1] = y;
-    } else {
-      out[2 * n] = (newidx[x >> 3] << 3) | (x & 3u);
-      out[2 * n + 1] = y;
-    }
-  }
-}
-
-void pad_leaf_pairs(std::vector<uint32_t>& relaid, const uint32_t* offsets, std::vector<uint32_t>& pair_gid) {
-  pair_gid.clear();
-  for (size_t n = 0; 2 * n < relaid.size(); ++n) {
-    const uint32_t x = relaid[2 * n];
-    if ((x & 7u) != 3u) continue;
-    const uint32_t cnt = x >> 3, off = relaid[2 * n + 1];
-    relaid[2 * n + 1] = (uint32_t)(pair_gid.size() / 2);
-    pair_gid.insert(pair_gid.end(), offsets + off, offsets + off + cnt);
-    if (cnt & 1u) pair_gid.push_back(kPadGid);
-  }
-}
-
 }  // namespace kdgr
 
 using namespace kdgr;
@@ -164,69 +91,96 @@ kdgr::FastView kdgr_scene_s::fast_view(bool packed) const {
   return v;
 }
 
-namespace {
-
-constexpr int kTopLevels = 10;  // 2047 nodes at most = 16 KB of shared memory
-
-}  // namespace
-
 namespace kdgr {
 
 // renderGaussianWithCudaSetup (cudaRenderer.cu:2557-2703) from device-resident
-// 64-float records: the per-Gaussian arrays of every requested form are
-// written by the packing kernel (scene_pack.cu), the tree is uploaded as
-// given (plain form) and relaid out with its leaf-order pair records (fast
-// forms).  The tree must have been validated.
+// 64-float records: the tree is copied to the device as given, checked,
+// relaid out and expanded into padded leaf order there (scene_tree.cu), and
+// the per-Gaussian arrays of every requested form are written by the packing
+// kernel (scene_pack.cu).  Work runs on the legacy default stream, so that
+// records another blocking stream is still writing are waited for.
 int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* offsets, uint32_t n_offsets,
-                      const float aabb[6], const float* d_g, uint32_t n, uint32_t flags, uint32_t depth,
-                      kdgr_scene_t* out, const char* who) {
+                      const float aabb[6], uint32_t n, uint32_t flags,
+                      const std::function<int(const float** d_gaussians)>& records, kdgr_scene_t* out,
+                      const char* who) {
   const std::string w(who);
   uint32_t forms = flags & (KDGR_FORM_EXACT | KDGR_FORM_FAST | KDGR_FORM_PACKED);
   if (forms == 0) forms = KDGR_FORM_EXACT | KDGR_FORM_FAST;
   const bool inverted = (flags & KDGR_SCALES_INVERTED) != 0;
+  const bool exact = (forms & KDGR_FORM_EXACT) != 0, fast = (forms & KDGR_FORM_FAST) != 0,
+             packed = (forms & KDGR_FORM_PACKED) != 0;
 
   std::unique_ptr<kdgr_scene_s> s(new kdgr_scene_s);
-  cudaGetDevice(&s->device);
+  WorkMem W(nullptr);
+  auto fail = [&](const char* where, cudaError_t e) {
+    for (void* p : s->blocks) cudaFree(p);
+    return cuda_fail(e != cudaSuccess ? e : cudaErrorUnknown, (w + ": " + where).c_str());
+  };
+  auto host_check = [&]() {  // names what is wrong with the tree
+    std::string err;
+    uint32_t depth = 0;
+    const int rc = validate_tree(nodes, n_nodes, offsets, n_offsets, n, err, &depth);
+    if (rc != KDGR_OK) set_error(w + ": " + err);
+    return rc;
+  };
+  if (W.err != cudaSuccess) {  // a malformed tree is refused as such also without a device
+    const int rc = host_check();
+    return rc != KDGR_OK ? rc : fail("work memory", W.err);
+  }
+  s->device = W.dev;
   s->forms = forms;
   s->n_nodes = n_nodes;
   s->n_offsets = n_offsets;
   s->n_gauss = n;
-  s->depth = depth;
   memcpy(s->aabb, aabb, sizeof(s->aabb));
-  for (uint32_t i = 0; i < n_nodes; ++i)
-    if ((nodes[2 * i] & 7u) == 3u) {
-      ++s->n_leaves;
-      if ((nodes[2 * i] >> 3) > s->max_leaf) s->max_leaf = nodes[2 * i] >> 3;
-    }
 
-  DevAlloc A;
-  std::vector<void*> staging;
-  auto fail = [&](const std::string& where, cudaError_t e = cudaSuccess) {
-    if (e == cudaSuccess) e = A.err != cudaSuccess ? A.err : cudaGetLastError();
-    for (void* p : staging) cudaFree(p);
-    A.release();
-    return cuda_fail(e, (w + ": " + where).c_str());
-  };
-  auto stage = [&](size_t bytes, void** p) {
-    const cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
-    if (e == cudaSuccess) staging.push_back(*p);
-    return e;
-  };
-  s->d_offsets = A.alloc<uint32_t>(n_offsets ? n_offsets : 1);
-  s->d_sh = A.alloc<float4>(12 * (size_t)n);
-  s->d_status = A.alloc<uint32_t>(1);
-  if (forms & KDGR_FORM_EXACT) {
-    s->d_nodes = A.alloc<uint2>(n_nodes);
-    s->d_test = A.alloc<float4>(4 * (size_t)n);
+  // the tree as given, and its checks
+  uint2* d_raw = W.take<uint2>(n_nodes);
+  uint32_t* d_ids = W.take<uint32_t>(n_offsets ? n_offsets : 1);
+  cudaError_t e = W.err;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_raw, nodes, 8ull * n_nodes, cudaMemcpyHostToDevice, W.st);
+  if (e == cudaSuccess && n_offsets)
+    e = cudaMemcpyAsync(d_ids, offsets, 4ull * n_offsets, cudaMemcpyHostToDevice, W.st);
+  TreeLists L;
+  if (e == cudaSuccess) e = tree_check(W, d_raw, n_nodes, d_ids, n_offsets, n, L);
+  if (e != cudaSuccess) return fail("tree upload", e);
+  if (!L.ok) {
+    const int rc = host_check();
+    if (rc != KDGR_OK) return rc;
+    set_error(w + ": the tree failed its device check");
+    return KDGR_ERR_FORMAT;
   }
-  if (forms & (KDGR_FORM_FAST | KDGR_FORM_PACKED)) s->d_opacity = A.alloc<float>(n);
-  if (forms & KDGR_FORM_PACKED) s->d_sh_bf16 = A.alloc<uint4>(6 * (size_t)n);
-  if (A.err != cudaSuccess) return fail("cudaMalloc");
-  if (n_offsets && cudaMemcpy(s->d_offsets, offsets, 4ull * n_offsets, cudaMemcpyHostToDevice) != cudaSuccess)
-    return fail("upload offsets");
-  if (s->d_nodes && cudaMemcpy(s->d_nodes, nodes, 8ull * n_nodes, cudaMemcpyHostToDevice) != cudaSuccess)
-    return fail("upload nodes");
-  if (cudaMemset(s->d_status, 0, 4) != cudaSuccess) return fail("status");
+  s->depth = L.levels - 1;
+  s->n_leaves = L.n_leaves;
+  s->max_leaf = L.max_leaf;
+  const float* d_g = nullptr;
+  const int rrc = records(&d_g);
+  if (rrc != KDGR_OK) return rrc;
+
+  Slab A;
+  A.add(s->d_offsets, n_offsets ? n_offsets : 1);
+  A.add(s->d_sh, 12 * (size_t)n);
+  A.add(s->d_status, 1);
+  if (exact) {
+    A.add(s->d_nodes, n_nodes);
+    A.add(s->d_test, 4 * (size_t)n);
+  }
+  if (fast || packed) {
+    A.add(s->d_opacity, n);
+    A.add(s->d_nodes_fast, n_nodes);
+  }
+  if (packed) {
+    A.add(s->d_sh_bf16, 6 * (size_t)n);
+    A.add(s->d_nodes_packed, n_nodes);
+    A.add(s->d_leaf_aux, n_nodes);
+  }
+  e = A.make(s->blocks);
+  if (e != cudaSuccess) return fail("cudaMalloc", e);
+  if (n_offsets) e = cudaMemcpyAsync(s->d_offsets, d_ids, 4ull * n_offsets, cudaMemcpyDeviceToDevice, W.st);
+  if (e == cudaSuccess && exact)
+    e = cudaMemcpyAsync(s->d_nodes, d_raw, 8ull * n_nodes, cudaMemcpyDeviceToDevice, W.st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->d_status, 0, 4, W.st);
+  if (e != cudaSuccess) return fail("tree arrays", e);
 
   // per-Gaussian arrays, packed on the device
   PackOut po{};
@@ -234,60 +188,72 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   po.test = s->d_test;
   po.opacity = s->d_opacity;
   po.sh_bf16 = s->d_sh_bf16;
-  float* d_giscl = nullptr;
-  float4* d_fast = nullptr;
-  uint32_t* d_packed = nullptr;
-  uint8_t* d_aniso = nullptr;
-  cudaError_t e = stage(12ull * n, (void**)&d_giscl);
-  if (e == cudaSuccess && (forms & KDGR_FORM_FAST)) e = stage(48ull * n, (void**)&d_fast);
-  if (e == cudaSuccess && (forms & KDGR_FORM_PACKED)) e = stage(32ull * n, (void**)&d_packed);
-  if (e == cudaSuccess && (forms & KDGR_FORM_PACKED)) e = stage(n, (void**)&d_aniso);
-  if (e != cudaSuccess) return fail("cudaMalloc (staging)", e);
-  po.giscl = d_giscl;
-  po.fast = d_fast;
-  po.packed = d_packed;
-  po.aniso = d_aniso;
-  e = launch_pack(d_g, n, inverted, po, nullptr);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (packed) po.giscl = W.take<float>(3 * (size_t)n);
+  if (fast) po.fast = W.take<float4>(3 * (size_t)n);
+  if (packed) po.packed = W.take<uint32_t>(8 * (size_t)n);
+  if (packed) po.aniso = W.take<uint8_t>(n);
+  if (W.err != cudaSuccess) return fail("cudaMalloc (staging)", W.err);
+  e = launch_pack(d_g, n, inverted, po, W.st);
   if (e != cudaSuccess) return fail("packing kernel", e);
 
-  std::vector<uint32_t> relaid, pair_gid;  // relaid fast tree, padded leaf order (fast forms)
-  if (forms & (KDGR_FORM_FAST | KDGR_FORM_PACKED)) {
-    relayout_tree(nodes, n_nodes, kTopLevels, relaid, &s->top_nodes);
-    pad_leaf_pairs(relaid, offsets, pair_gid);
-    if (pair_gid.size() > 0xFFFFFFF0ull) {
-      for (void* p : staging) cudaFree(p);
-      A.release();
+  Slab P;
+  if (fast || packed) {  // the relaid tree and its padded leaf order
+    s->top_nodes = L.top_nodes;
+    uint64_t *first = nullptr, n_pairs = 0;
+    e = tree_relayout(W, d_raw, L, s->d_nodes_fast);
+    if (e == cudaSuccess) e = tree_leaf_pairs(W, s->d_nodes_fast, L.n, &first, &n_pairs);
+    if (e != cudaSuccess) return fail("tree relayout", e);
+    if (2 * n_pairs > 0xFFFFFFF0ull) {
+      for (void* p : s->blocks) cudaFree(p);
       set_error(w + ": more than 2^32 leaf entries after pair padding");
       return KDGR_ERR_LIMIT;
     }
-    s->n_pair_entries = (uint32_t)pair_gid.size();
-    s->d_nodes_fast = A.alloc<uint2>(n_nodes);
-    s->d_pair_gid = A.alloc<uint32_t>(pair_gid.size() + 2);
-    if (A.err != cudaSuccess) return fail("cudaMalloc (tree)");
-    if (cudaMemcpy(s->d_nodes_fast, relaid.data(), 8ull * n_nodes, cudaMemcpyHostToDevice) != cudaSuccess ||
-        (!pair_gid.empty() && cudaMemcpy(s->d_pair_gid, pair_gid.data(), 4 * pair_gid.size(),
-                                         cudaMemcpyHostToDevice) != cudaSuccess))
-      return fail("upload (tree)");
-  }
-  if (forms & KDGR_FORM_FAST) {
+    s->n_pair_entries = (uint32_t)(2 * n_pairs);
+    P.add(s->d_pair_gid, s->n_pair_entries + 2ull);
+    if (fast) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
+    e = P.make(s->blocks);
+    if (e == cudaSuccess) e = tree_leaf_gids(W, s->d_nodes_fast, L.n, first, s->d_offsets, s->d_pair_gid);
     // the per-Gaussian rows are staging: the kernels read the leaf-order pairs
-    s->d_leaf_pairs = A.alloc<float4>(6 * ((size_t)s->n_pair_entries / 2 + 1));
-    if (A.err != cudaSuccess) return fail("cudaMalloc (fast)");
-    e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, d_fast, s->d_leaf_pairs);
-    if (e != cudaSuccess) return fail("leaf pairs (fast)", e);
+    if (e == cudaSuccess && fast)
+      e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, po.fast, s->d_leaf_pairs, W.st);
+    if (e != cudaSuccess) return fail("leaf order", e);
   }
-  if (forms & KDGR_FORM_PACKED) {
-    const int rc = pack_precision(s.get(), d_g, d_giscl, d_packed, d_aniso, relaid, pair_gid, A);
-    if (rc != KDGR_OK) {
-      for (void* p : staging) cudaFree(p);
-      A.release();
-      return rc;
+  Slab Q;
+  if (packed) {
+    // the flagged Gaussians get FP64-precomputed factors, and each leaf is
+    // laid out as its plain entries in FP16 pairs followed by its flagged
+    // entries in FP32 pairs of a second stream
+    uint32_t* aidx = nullptr;
+    uint64_t *first = nullptr, totals = 0;
+    e = aniso_index(W, po.aniso, n, &aidx, &s->n_aniso);
+    if (e == cudaSuccess)
+      e = tree_split_counts(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, &first, &totals);
+    if (e != cudaSuccess) return fail("packed leaf counts", e);
+    s->n_plain_entries = 2u * (uint32_t)totals;
+    s->n_flag_entries = 2u * (uint32_t)(totals >> 32);
+    Q.add(s->d_gid_plain, s->n_plain_entries + 2ull);
+    Q.add(s->d_gid_flag, s->n_flag_entries + 2ull);
+    Q.add(s->d_leaf_packed, 2 * (s->n_plain_entries + 2ull));
+    Q.add(s->d_flag_pairs, 3 * (s->n_flag_entries + 2ull));
+    e = Q.make(s->blocks);
+    if (e != cudaSuccess) return fail("cudaMalloc (packed)", e);
+    float* src = W.take<float>(10 * (size_t)s->n_aniso);
+    float4* table = W.take<float4>(3 * (size_t)s->n_aniso);
+    e = W.err;
+    if (e == cudaSuccess)
+      e = tree_split_fill(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, first, s->d_nodes_packed, s->d_leaf_aux,
+                          s->d_gid_plain, s->d_gid_flag);
+    if (e == cudaSuccess) e = build_packed_pairs(s->d_gid_plain, s->n_plain_entries, po.packed, s->d_leaf_packed, W.st);
+    if (e == cudaSuccess && s->n_aniso) {
+      e = launch_gather_aniso(d_g, po.giscl, aidx, n, src, W.st);
+      if (e == cudaSuccess) e = launch_aniso_fp64(src, s->n_aniso, table, W.st);
+      if (e == cudaSuccess) e = build_flag_pairs(s->d_gid_flag, s->n_flag_entries, aidx, table, s->d_flag_pairs, W.st);
     }
+    if (e != cudaSuccess) return fail("packed upload", e);
   }
-  for (void* p : staging) cudaFree(p);
-  s->device_bytes = A.bytes;
-  A.ptrs.clear();  // ownership moves to the scene
+  e = cudaStreamSynchronize(W.st);
+  if (e != cudaSuccess) return fail("upload", e);
+  s->device_bytes = A.bytes + P.bytes + Q.bytes;
   *out = s.release();
   return KDGR_OK;
 }
@@ -306,7 +272,10 @@ int kdgr_init(int device) {
 
 int kdgr_shutdown(void) {
   cudaError_t e = cudaDeviceSynchronize();
+  int dev = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "kdgr_shutdown");
+  work_pool_trim(dev);
   return KDGR_OK;
 }
 
@@ -317,24 +286,19 @@ int kdgr_scene_create(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     return KDGR_ERR_INVALID_ARG;
   }
   *out = nullptr;
-  std::string err;
-  uint32_t depth = 0;
-  int rc = validate_tree(nodes, n_nodes, offsets, n_offsets, n, err, &depth);
-  if (rc != KDGR_OK) {
-    set_error("kdgr_scene_create: " + err);
-    return rc;
-  }
   // the records go to the device as they are; the device packs every form
   float* d_rec = nullptr;
-  cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
-  if (e == cudaSuccess) e = cudaMemcpy(d_rec, g, 256ull * n, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    if (d_rec) cudaFree(d_rec);
-    return cuda_fail(e, "kdgr_scene_create: record upload");
-  }
-  rc = scene_create_impl(nodes, n_nodes, offsets, n_offsets, aabb, d_rec, n, flags, depth, out,
-                         "kdgr_scene_create");
-  cudaFree(d_rec);
+  const int rc = scene_create_impl(
+      nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
+      [&](const float** d) {
+        cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_rec, g, 256ull * n, cudaMemcpyHostToDevice, nullptr);
+        if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create: record upload");
+        *d = d_rec;
+        return (int)KDGR_OK;
+      },
+      out, "kdgr_scene_create");
+  if (d_rec) cudaFree(d_rec);
   return rc;
 }
 
@@ -345,26 +309,20 @@ int kdgr_scene_create_device(const uint32_t* nodes, uint32_t n_nodes, const uint
     return KDGR_ERR_INVALID_ARG;
   }
   *out = nullptr;
-  std::string err;
-  uint32_t depth = 0;
-  int rc = validate_tree(nodes, n_nodes, offsets, n_offsets, n, err, &depth);
-  if (rc != KDGR_OK) {
-    set_error("kdgr_scene_create_device: " + err);
-    return rc;
-  }
-  return scene_create_impl(nodes, n_nodes, offsets, n_offsets, aabb, d_g, n, flags, depth, out,
-                           "kdgr_scene_create_device");
+  return scene_create_impl(
+      nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
+      [&](const float** d) {
+        *d = d_g;
+        return (int)KDGR_OK;
+      },
+      out, "kdgr_scene_create_device");
 }
 
 int kdgr_scene_destroy(kdgr_scene_t s) {
   if (!s) return KDGR_ERR_INVALID_ARG;
   DeviceScope on(s->device);
-  void* ps[] = {s->d_nodes,     s->d_offsets, s->d_test,      s->d_sh,          s->d_nodes_fast,
-                s->d_opacity,   s->d_sh_bf16,     s->d_leaf_pairs,  s->d_leaf_packed, s->d_pair_gid,
-                s->d_nodes_packed, s->d_leaf_aux, s->d_gid_plain, s->d_gid_flag, s->d_flag_pairs,
-                s->d_status};
   cudaError_t first = cudaSuccess;
-  for (void* p : ps)
+  for (void* p : s->blocks)
     if (p) {
       cudaError_t e = cudaFree(p);
       if (first == cudaSuccess) first = e;

@@ -366,24 +366,19 @@ extern "C" int kdgr_scene_create_from_files(const char* ply_path, const char* kd
     return rc;
   }
   const uint32_t n_nodes = (uint32_t)(t.nodes.size() / 2), n_offsets = (uint32_t)t.offsets.size();
-  uint32_t depth = 0;
-  rc = validate_tree(t.nodes.data(), n_nodes, t.offsets.data(), n_offsets, n, err, &depth);
-  if (rc != KDGR_OK) {
-    set_error("kdgr_scene_create_from_files: " + err);
-    return rc;
-  }
   float* d_rec = nullptr;
-  cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
-  if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create_from_files: cudaMalloc");
-  uint32_t n2 = 0;
-  rc = read_ply_device(ply_path, d_rec, n, &n2, nullptr, err);
-  if (rc != KDGR_OK) {
-    cudaFree(d_rec);
-    set_error("kdgr_scene_create_from_files: " + err);
-    return rc;
-  }
-  rc = scene_create_impl(t.nodes.data(), n_nodes, t.offsets.data(), n_offsets, t.aabb, d_rec, n, flags, depth, out,
-                         "kdgr_scene_create_from_files");
-  cudaFree(d_rec);
+  rc = scene_create_impl(
+      t.nodes.data(), n_nodes, t.offsets.data(), n_offsets, t.aabb, n, flags,
+      [&](const float** d) {
+        const cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
+        if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create_from_files: cudaMalloc");
+        uint32_t n2 = 0;
+        const int prc = read_ply_device(ply_path, d_rec, n, &n2, nullptr, err);
+        if (prc != KDGR_OK) set_error("kdgr_scene_create_from_files: " + err);
+        *d = d_rec;
+        return prc;
+      },
+      out, "kdgr_scene_create_from_files");
+  if (d_rec) cudaFree(d_rec);
   return rc;
 }

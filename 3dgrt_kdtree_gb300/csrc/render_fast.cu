@@ -1364,91 +1364,6 @@ cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& c, const ViewD
   return cudaGetLastError();
 }
 
-// The precision form from the device packing kernel's outputs (d_packed:
-// FP32 mean + FP16 M per Gaussian; d_aniso: flagged Gaussians; BF16 SH and
-// opacity already in the scene): the flagged Gaussians get FP64-precomputed
-// factors (k_aniso_fp64) and each leaf is laid out as its plain entries in
-// FP16 pairs followed by its flagged entries in FP32 pairs of a second stream.
-int pack_precision(kdgr_scene_s* s, const float* d_rec, const float* d_giscl, const uint32_t* d_packed,
-                   const uint8_t* d_aniso, const std::vector<uint32_t>& relaid,
-                   const std::vector<uint32_t>& pair_gid, DevAlloc& A) {
-  const size_t n = s->n_gauss;
-  std::vector<uint8_t> flag(n);
-  if (cudaMemcpy(flag.data(), d_aniso, n, cudaMemcpyDeviceToHost) != cudaSuccess)
-    return cuda_fail(cudaGetLastError(), "kdgr_scene_create: aniso flags");
-  std::vector<uint32_t> aidx(n, 0xFFFFFFFFu);
-  uint32_t n_aniso = 0;
-  for (size_t i = 0; i < n; ++i)
-    if (flag[i]) aidx[i] = n_aniso++;
-  // The packed form's leaf layout: per leaf its plain entries in FP16 pairs,
-  // then its flagged entries in FP32 pairs of a second stream, both padded
-  // to whole pairs; the leaf words and per-node aux words say where.
-  std::vector<uint32_t> nodes_p(relaid), gid_plain, gid_flag;
-  std::vector<uint32_t> aux(relaid.size(), 0u);
-  std::vector<uint32_t> plain, flagged;
-  for (size_t nd = 0; 2 * nd < relaid.size(); ++nd) {
-    const uint32_t x = relaid[2 * nd];
-    if ((x & 7u) != 3u) continue;
-    const uint32_t cnt = x >> 3, e0 = 2 * relaid[2 * nd + 1];
-    plain.clear();
-    flagged.clear();
-    for (uint32_t k = 0; k < cnt; ++k) {
-      const uint32_t gid = pair_gid[e0 + k];
-      (aidx[gid] == 0xFFFFFFFFu ? plain : flagged).push_back(gid);
-    }
-    nodes_p[2 * nd] = ((uint32_t)plain.size() << 3) | 3u;
-    nodes_p[2 * nd + 1] = (uint32_t)(gid_plain.size() / 2);
-    aux[2 * nd] = (uint32_t)(gid_flag.size() / 2);
-    aux[2 * nd + 1] = (uint32_t)flagged.size();
-    gid_plain.insert(gid_plain.end(), plain.begin(), plain.end());
-    if (plain.size() & 1u) gid_plain.push_back(kPadGid);
-    gid_flag.insert(gid_flag.end(), flagged.begin(), flagged.end());
-    if (flagged.size() & 1u) gid_flag.push_back(kPadGid);
-  }
-  if (gid_plain.size() > 0xFFFFFFF0ull || gid_flag.size() > 0xFFFFFFF0ull) {
-    set_error("kdgr_scene_create: more than 2^32 leaf entries after pair padding");
-    return KDGR_ERR_LIMIT;
-  }
-  s->n_plain_entries = (uint32_t)gid_plain.size();
-  s->n_flag_entries = (uint32_t)gid_flag.size();
-  s->n_aniso = n_aniso;
-  s->d_nodes_packed = A.alloc<uint2>(relaid.size() / 2);
-  s->d_leaf_aux = A.alloc<uint2>(relaid.size() / 2);
-  s->d_gid_plain = A.alloc<uint32_t>(gid_plain.size() + 2);
-  s->d_gid_flag = A.alloc<uint32_t>(gid_flag.size() + 2);
-  s->d_leaf_packed = A.alloc<uint4>(2 * (gid_plain.size() + 2));
-  s->d_flag_pairs = A.alloc<float4>(3 * (gid_flag.size() + 2));
-  if (A.err != cudaSuccess) return cuda_fail(A.err, "kdgr_scene_create: cudaMalloc (packed)");
-  uint32_t* d_aidx = nullptr;
-  float* d_src = nullptr;
-  float4* d_table = nullptr;
-  auto up = [](void* dst, const void* src, size_t bytes) {
-    return bytes ? cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
-  cudaError_t e = up(s->d_nodes_packed, nodes_p.data(), nodes_p.size() * 4);
-  if (e == cudaSuccess) e = up(s->d_leaf_aux, aux.data(), aux.size() * 4);
-  if (e == cudaSuccess) e = up(s->d_gid_plain, gid_plain.data(), gid_plain.size() * 4);
-  if (e == cudaSuccess) e = up(s->d_gid_flag, gid_flag.data(), gid_flag.size() * 4);
-  if (e == cudaSuccess) e = build_packed_pairs(s->d_gid_plain, s->n_plain_entries, d_packed, s->d_leaf_packed);
-  if (e == cudaSuccess && n_aniso) {
-    e = cudaMalloc(&d_src, 40ull * n_aniso);
-    if (e == cudaSuccess) e = cudaMalloc(&d_table, 3 * sizeof(float4) * n_aniso);
-    if (e == cudaSuccess) e = cudaMalloc(&d_aidx, aidx.size() * 4);
-    if (e == cudaSuccess) e = up(d_aidx, aidx.data(), aidx.size() * 4);
-    if (e == cudaSuccess) e = launch_gather_aniso(d_rec, d_giscl, d_aidx, (uint32_t)n, d_src, nullptr);
-    if (e == cudaSuccess) {
-      k_aniso_fp64<<<(n_aniso + 127) / 128, 128>>>(d_src, n_aniso, d_table);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = build_flag_pairs(s->d_gid_flag, s->n_flag_entries, d_aidx, d_table, s->d_flag_pairs);
-  }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  for (void* q : {(void*)d_src, (void*)d_table, (void*)d_aidx})
-    if (q) cudaFree(q);
-  if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create: packed upload");
-  return KDGR_OK;
-}
-
 // Pair p of the packed plain records (layout at PPairRec) from the
 // per-Gaussian staging words: mean x, y, z (FP32), half2 (M22, 0),
 // half2 (M00, M01), (M02, M10), (M11, M12), (M20, M21).  Padding entries
@@ -1509,27 +1424,33 @@ __global__ void k_build_pairs(const uint32_t* __restrict__ gid, uint32_t n, cons
   }
 }
 
-cudaError_t build_leaf_pairs(const uint32_t* d_gid, uint32_t n_entries, const float4* test, float4* pairs) {
+cudaError_t build_leaf_pairs(const uint32_t* d_gid, uint32_t n_entries, const float4* test, float4* pairs,
+                             cudaStream_t st) {
   if (n_entries == 0) return cudaSuccess;
   const size_t np = (size_t)n_entries / 2;
-  k_build_pairs<<<(unsigned)((np + 255) / 256), 256>>>(d_gid, n_entries, test, pairs);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  return e;
+  k_build_pairs<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(d_gid, n_entries, test, pairs);
+  return cudaGetLastError();
 }
 
-cudaError_t build_packed_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* src, uint4* pairs) {
+cudaError_t build_packed_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* src, uint4* pairs,
+                               cudaStream_t st) {
   if (n_entries == 0) return cudaSuccess;
   const size_t np = (size_t)n_entries / 2;
-  k_build_ppairs<<<(unsigned)((np + 255) / 256), 256>>>(d_gid, n_entries, src, pairs);
+  k_build_ppairs<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(d_gid, n_entries, src, pairs);
   return cudaGetLastError();
 }
 
 cudaError_t build_flag_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* aidx, const float4* table,
-                             float4* pairs) {
+                             float4* pairs, cudaStream_t st) {
   if (n_entries == 0) return cudaSuccess;
   const size_t np = (size_t)n_entries / 2;
-  k_build_flag_pairs<<<(unsigned)((np + 255) / 256), 256>>>(d_gid, n_entries, aidx, table, pairs);
+  k_build_flag_pairs<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(d_gid, n_entries, aidx, table, pairs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_aniso_fp64(const float* src, uint32_t n, float4* table, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  k_aniso_fp64<<<(n + 127) / 128, 128, 0, st>>>(src, n, table);
   return cudaGetLastError();
 }
 

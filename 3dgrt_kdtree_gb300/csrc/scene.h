@@ -4,11 +4,14 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <functional>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "device_common.cuh"
+#include "device_pool.h"
 #include "kdgr.h"
 
 struct kdgr_scene_s {
@@ -49,6 +52,7 @@ struct kdgr_scene_s {
   // per-scene status word written by kernels (error bits)
   uint32_t* d_status = nullptr;
   size_t device_bytes = 0;
+  std::vector<void*> blocks;  // device allocations that hold the arrays above
   std::mutex mu;
 
   kdgr::ExactView exact_view() const;
@@ -74,49 +78,101 @@ struct DeviceScope {
   DeviceScope& operator=(const DeviceScope&) = delete;
 };
 
-// Allocation helper that records bytes and frees everything on failure.
-struct DevAlloc {
-  std::vector<void*> ptrs;
+// Arrays laid out in one device allocation (a cudaMalloc and its cudaFree
+// take 35 to 100 us each): add every array, then make() sets the pointers.
+struct Slab {
+  std::vector<std::pair<void**, size_t>> at;
   size_t bytes = 0;
-  cudaError_t err = cudaSuccess;
   template <typename T>
-  T* alloc(size_t count) {
-    if (err != cudaSuccess) return nullptr;
-    void* p = nullptr;
-    const size_t b = count * sizeof(T) + 16;
-    err = cudaMalloc(&p, b);
-    if (err != cudaSuccess) return nullptr;
-    ptrs.push_back(p);
-    bytes += b;
-    return static_cast<T*>(p);
+  void add(T*& p, size_t count) {
+    at.push_back({reinterpret_cast<void**>(&p), bytes});
+    bytes += (count * sizeof(T) + 16 + 255) & ~size_t(255);
   }
-  void release() {
-    for (void* p : ptrs) cudaFree(p);
-    ptrs.clear();
+  cudaError_t make(std::vector<void*>& blocks) {
+    void* base = nullptr;
+    const cudaError_t e = cudaMalloc(&base, bytes ? bytes : 256);
+    if (e != cudaSuccess) return e;
+    blocks.push_back(base);
+    for (auto& a : at) *a.first = static_cast<char*>(base) + a.second;
+    return cudaSuccess;
   }
 };
 
+// Buffers of one call from the library's work pool, all on one stream,
+// returned (stream-ordered) when the object ends.
+struct WorkMem {
+  cudaStream_t st = nullptr;
+  cudaMemPool_t pool = nullptr;
+  int dev = -1;
+  cudaError_t err = cudaSuccess;
+  std::vector<void*> ptrs;
+  explicit WorkMem(cudaStream_t stream) : st(stream) {
+    err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) err = work_pool_enter(dev, &pool);
+  }
+  ~WorkMem() {
+    for (void* p : ptrs) cudaFreeAsync(p, st);
+    if (!pool) return;
+    if (!ptrs.empty()) cudaStreamSynchronize(st);  // so that the pool can trim
+    work_pool_leave(dev);
+  }
+  template <typename T>
+  T* take(size_t count) {
+    if (err != cudaSuccess) return nullptr;
+    void* p = nullptr;
+    err = cudaMallocFromPoolAsync(&p, count * sizeof(T) + 16, pool, st);
+    if (err != cudaSuccess) return nullptr;
+    ptrs.push_back(p);
+    return static_cast<T*>(p);
+  }
+  WorkMem(const WorkMem&) = delete;
+  WorkMem& operator=(const WorkMem&) = delete;
+};
+
 int cuda_fail(cudaError_t e, const char* where);
-// Fast-form tree relayout: top levels breadth-first, rest depth-first.
-void relayout_tree(const uint32_t* nodes, uint32_t n_nodes, int top_levels, std::vector<uint32_t>& out,
-                   uint32_t* top_count);
-// Packed precision form from the packing kernel's outputs: the FP64
-// upload-time factors of flagged Gaussians and the form's own leaf layout.
-int pack_precision(kdgr_scene_s* s, const float* d_rec, const float* d_giscl, const uint32_t* d_packed,
-                   const uint8_t* d_aniso, const std::vector<uint32_t>& relaid,
-                   const std::vector<uint32_t>& pair_gid, DevAlloc& A);
-// Fast-form leaf layout: rewrites the leaf words of the relaid tree
-// (y = first pair) and returns the padded per-entry Gaussian IDs.
-void pad_leaf_pairs(std::vector<uint32_t>& relaid, const uint32_t* offsets, std::vector<uint32_t>& pair_gid);
+// The tree side of an upload, on the device (scene_tree.cu).  The nodes
+// reached from the root, listed level by level:
+struct TreeLists {
+  uint32_t *list = nullptr, *cpos = nullptr, *ls = nullptr;  // node, list position of its left child, level starts
+  std::vector<uint32_t> starts;                              // host copy of ls
+  uint32_t n = 0, levels = 0, top_nodes = 0;
+  uint32_t n_leaves = 0, max_leaf = 0;  // over all nodes given
+  bool ok = false;                      // every check of validate_tree holds
+};
+cudaError_t tree_check(WorkMem& W, const uint2* d_nodes, uint32_t n_nodes, const uint32_t* d_offsets,
+                       uint32_t n_offsets, uint32_t n_gauss, TreeLists& L);
+// Fast-form node order into out[0 .. L.n): top levels breadth-first, rest
+// depth-first; leaf words as given.
+cudaError_t tree_relayout(WorkMem& W, const uint2* d_nodes, const TreeLists& L, uint2* out);
+// First pair of every relaid leaf (exclusive sums, n + 1 of them) and the
+// number of pairs; synchronises.
+cudaError_t tree_leaf_pairs(WorkMem& W, const uint2* relaid, uint32_t n, uint64_t** first, uint64_t* n_pairs);
+// Padded leaf-order IDs; leaf word y of the relaid tree becomes its first pair.
+cudaError_t tree_leaf_gids(WorkMem& W, uint2* relaid, uint32_t n, const uint64_t* first, const uint32_t* d_offsets,
+                           uint32_t* gid);
+// Table index of every flagged Gaussian (0xFFFFFFFF for the others); n_aniso
+// is set once the stream has been synchronised.
+cudaError_t aniso_index(WorkMem& W, const uint8_t* flag, uint32_t n, uint32_t** aidx, uint32_t* n_aniso);
+// Packed form: first plain pair (low word) and first flagged pair (high
+// word) of every relaid leaf, and the totals; synchronises.
+cudaError_t tree_split_counts(WorkMem& W, const uint2* relaid, uint32_t n, const uint32_t* gid, const uint8_t* flag,
+                              uint64_t** first, uint64_t* totals);
+cudaError_t tree_split_fill(WorkMem& W, const uint2* relaid, uint32_t n, const uint32_t* gid, const uint8_t* flag,
+                            const uint64_t* first, uint2* nodes_p, uint2* aux, uint32_t* gid_plain,
+                            uint32_t* gid_flag);
 constexpr uint32_t kPadGid = 0xFFFFFFFFu;
 // Pair records in padded leaf order (entry j = Gaussian gid[j], zero for
 // padding): FP32 from 3 float4 per Gaussian (rows of M and b), packed from
 // 8 words per Gaussian, flagged FP32 pairs from the FP64-precomputed table
-// (entry aidx[gid]).  The packed builders do not synchronize.
-cudaError_t build_leaf_pairs(const uint32_t* d_gid, uint32_t n_entries, const float4* test, float4* pairs);
-cudaError_t build_packed_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* src, uint4* pairs);
+// (entry aidx[gid]).  Asynchronous on `st`.
+cudaError_t build_leaf_pairs(const uint32_t* d_gid, uint32_t n_entries, const float4* test, float4* pairs,
+                             cudaStream_t st);
+cudaError_t build_packed_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* src, uint4* pairs,
+                               cudaStream_t st);
 cudaError_t build_flag_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* aidx, const float4* table,
-                             float4* pairs);
+                             float4* pairs, cudaStream_t st);
+// The FP64 factors of n flagged Gaussians (k_aniso_fp64).
+cudaError_t launch_aniso_fp64(const float* src, uint32_t n, float4* table, cudaStream_t st);
 // Batched rendering (render_fast.cu).
 // totals: 8x4 tiles, 16x8 blocks and 32x16 super-blocks over all views.
 int make_view_table(const kdgr_view* views, int n_views, std::vector<ViewDesc>& out, uint32_t totals[3]);
@@ -178,9 +234,10 @@ struct PlyLayout {
 int parse_ply_header(FILE* fp, PlyLayout& lay, uint64_t& n_vertices, uint32_t& stride, std::string& err);
 cudaError_t launch_ply_activate(const uint8_t* d_raw, uint32_t n, uint32_t stride, const PlyLayout& lay,
                                 float* d_rec, cudaStream_t st);
-// Device records -> scene (all forms); the tree arrays are host arrays,
-// validated by the caller.
+// Records and tree -> scene (all forms).  The tree arrays are host arrays,
+// checked here before `records` is called for the device records.
 int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* offsets, uint32_t n_offsets,
-                      const float aabb[6], const float* d_gaussians, uint32_t n, uint32_t flags, uint32_t depth,
-                      kdgr_scene_t* out, const char* who);
+                      const float aabb[6], uint32_t n, uint32_t flags,
+                      const std::function<int(const float** d_gaussians)>& records, kdgr_scene_t* out,
+                      const char* who);
 }  // namespace kdgr
