@@ -21,10 +21,12 @@ CamInfo make_caminfo(const kdgr_camera& cam, int width, int height);
 // Device arrays of the oracle-matching (plain drop-in) form.
 //   nodes:   the reference's 8-byte nodes, in the file's order;
 //   offsets: leaf Gaussian-ID lists;
-//   test:    4 x float4 per Gaussian, the fields the ray-Gaussian test reads:
-//            (pos.xyz, opacity) (1/s.xyz, s.x) (s.y, s.z, q.w, q.x) (q.y, q.z, 0, 0)
-//            with 1/s the reference's uploaded (inverted) scale and s its
-//            IEEE reciprocal, the value rayPrimIntersect computes per call;
+//   test:    kTestWords x float4 per Gaussian, the values the ray-Gaussian test
+//            reads: (pos.xyz, opacity) (1/s.xyz, s.x) (s.y, s.z, r00, r01)
+//            (r02, r10, r11, r12) (r20, r21, r22, 0) with 1/s the reference's
+//            uploaded (inverted) scale, s its IEEE reciprocal and r the rows of
+//            quaternionWXYZToMatrixTranspose in FP32: what rayPrimIntersect
+//            computes per call, computed once by the same operations;
 //   sh:      12 x float4 per Gaussian, coefficient-major RGB (k*3 + c).
 struct ExactView {
   const uint2* nodes;
@@ -32,6 +34,23 @@ struct ExactView {
   const float4* test;
   const float4* sh;
   uint32_t n_nodes, n_offsets, n_gauss;
+  float bmin[3], bmax[3];
+};
+
+constexpr uint32_t kTestWords = 5;
+
+// The plain form's leaf-order arrays for the packet walk: the fast form's
+// relaid tree, padded ID list and FP32 pairs, and per pair the constants of
+// the filter's tolerance (Ce lo, Ce hi, Cmu lo, Cmu hi; render_packet.cuh).
+// leaf_tol is null when they were not materialised.
+struct PlainView {
+  const uint2* nodes;
+  const uint32_t* offsets;
+  const float4* leaf_pairs;
+  const float4* leaf_tol;
+  const float4* test;
+  const float4* sh;
+  uint32_t n_offsets, n_gauss;
   float bmin[3], bmax[3];
 };
 
@@ -59,8 +78,8 @@ struct ExactView {
 //   leaf_aux:   packed form, per node: at a leaf (first flagged pair, number
 //               of flagged entries); flag_offsets their Gaussian IDs (n_flag).
 //   A leaf's hit index runs over its main-stream entries, then (packed) its
-//   flagged entries.  Padding entries hold zero records: M = 0 gives
-//   |grdu|^2 = 0 and t* = 0 * inf = NaN, which no leaf interval accepts.
+//   flagged entries.  Padding entries have M = 0: |grdu|^2 = 0 and
+//   grdu . ng = 0, which no leaf interval accepts.
 struct FastView {
   const uint2* nodes;
   const uint32_t* offsets;
@@ -130,7 +149,10 @@ struct HybridView {
 cudaError_t launch_hybrid(const ExactView& s, const CamInfo& cam, int width, int height, const HybridView& m,
                           float* rgb, uint32_t* status, cudaStream_t stream);
 
-cudaError_t launch_exact(const ExactView& s, const CamInfo& cam, int width, int height, float* rgb, float* alpha,
-                         float* depth, kdgr_ray_trace* trace, uint32_t* status, int kbuf, cudaStream_t stream);
+// Plain render; the packet walk over `plain` when it is materialised and no
+// trace is asked for, one thread per ray over `s` otherwise.
+cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamInfo& cam, int width, int height,
+                         float* rgb, float* alpha, float* depth, kdgr_ray_trace* trace, uint32_t* status,
+                         cudaStream_t stream);
 
 }  // namespace kdgr

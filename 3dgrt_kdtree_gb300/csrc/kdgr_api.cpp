@@ -91,6 +91,23 @@ kdgr::FastView kdgr_scene_s::fast_view(bool packed) const {
   return v;
 }
 
+kdgr::PlainView kdgr_scene_s::plain_view() const {
+  PlainView v;
+  v.nodes = d_nodes_fast;
+  v.offsets = d_pair_gid;
+  v.leaf_pairs = d_leaf_pairs;
+  v.leaf_tol = d_leaf_tol;
+  v.test = d_test;
+  v.sh = d_sh;
+  v.n_offsets = n_pair_entries;
+  v.n_gauss = n_gauss;
+  for (int i = 0; i < 3; ++i) {
+    v.bmin[i] = aabb[i];
+    v.bmax[i] = aabb[3 + i];
+  }
+  return v;
+}
+
 namespace kdgr {
 
 // renderGaussianWithCudaSetup (cudaRenderer.cu:2557-2703) from device-resident
@@ -163,12 +180,10 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   A.add(s->d_status, 1);
   if (exact) {
     A.add(s->d_nodes, n_nodes);
-    A.add(s->d_test, 4 * (size_t)n);
+    A.add(s->d_test, kTestWords * (size_t)n);
   }
-  if (fast || packed) {
-    A.add(s->d_opacity, n);
-    A.add(s->d_nodes_fast, n_nodes);
-  }
+  A.add(s->d_nodes_fast, n_nodes);
+  if (fast || packed) A.add(s->d_opacity, n);
   if (packed) {
     A.add(s->d_sh_bf16, 6 * (size_t)n);
     A.add(s->d_nodes_packed, n_nodes);
@@ -189,33 +204,56 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   po.opacity = s->d_opacity;
   po.sh_bf16 = s->d_sh_bf16;
   if (packed) po.giscl = W.take<float>(3 * (size_t)n);
-  if (fast) po.fast = W.take<float4>(3 * (size_t)n);
+  if (fast || exact) po.fast = W.take<float4>(3 * (size_t)n);
+  if (exact) po.tol = W.take<float2>(n);
   if (packed) po.packed = W.take<uint32_t>(8 * (size_t)n);
   if (packed) po.aniso = W.take<uint8_t>(n);
   if (W.err != cudaSuccess) return fail("cudaMalloc (staging)", W.err);
   e = launch_pack(d_g, n, inverted, po, W.st);
   if (e != cudaSuccess) return fail("packing kernel", e);
 
+  // the relaid tree and its padded leaf order
+  uint64_t *first = nullptr, n_pairs = 0;
+  e = tree_relayout(W, d_raw, L, s->d_nodes_fast);
+  if (e == cudaSuccess) e = tree_leaf_pairs(W, s->d_nodes_fast, L.n, &first, &n_pairs);
+  if (e != cudaSuccess) return fail("tree relayout", e);
+  const bool fits = 2 * n_pairs <= 0xFFFFFFF0ull;
+  if ((fast || packed) && !fits) {
+    for (void* p : s->blocks) cudaFree(p);
+    set_error(w + ": more than 2^32 leaf entries after pair padding");
+    return KDGR_ERR_LIMIT;
+  }
+  if (fast || packed) s->top_nodes = L.top_nodes;
+  auto leaf_arrays = [&](bool plain, Slab& P) {
+    P.add(s->d_pair_gid, 2 * n_pairs + 2);
+    if (fast || plain) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
+    if (plain) P.add(s->d_leaf_tol, n_pairs + 1);
+    return P.make(s->blocks);
+  };
   Slab P;
-  if (fast || packed) {  // the relaid tree and its padded leaf order
-    s->top_nodes = L.top_nodes;
-    uint64_t *first = nullptr, n_pairs = 0;
-    e = tree_relayout(W, d_raw, L, s->d_nodes_fast);
-    if (e == cudaSuccess) e = tree_leaf_pairs(W, s->d_nodes_fast, L.n, &first, &n_pairs);
-    if (e != cudaSuccess) return fail("tree relayout", e);
-    if (2 * n_pairs > 0xFFFFFFF0ull) {
-      for (void* p : s->blocks) cudaFree(p);
-      set_error(w + ": more than 2^32 leaf entries after pair padding");
-      return KDGR_ERR_LIMIT;
+  bool plain = exact && fits;
+  if (plain || fast || packed) {
+    e = leaf_arrays(plain, P);
+    if (e != cudaSuccess && plain) {
+      // no room for the plain form's leaf order: its frames are then walked
+      // one thread per ray over the tree as given
+      cudaGetLastError();
+      plain = false;
+      s->d_pair_gid = nullptr;
+      s->d_leaf_pairs = s->d_leaf_tol = nullptr;
+      P = Slab();
+      e = fast || packed ? leaf_arrays(false, P) : cudaSuccess;
     }
+    if (e != cudaSuccess) return fail("cudaMalloc (leaf order)", e);
+  }
+  if (plain || fast || packed) {
     s->n_pair_entries = (uint32_t)(2 * n_pairs);
-    P.add(s->d_pair_gid, s->n_pair_entries + 2ull);
-    if (fast) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
-    e = P.make(s->blocks);
-    if (e == cudaSuccess) e = tree_leaf_gids(W, s->d_nodes_fast, L.n, first, s->d_offsets, s->d_pair_gid);
+    e = tree_leaf_gids(W, s->d_nodes_fast, L.n, first, s->d_offsets, s->d_pair_gid);
     // the per-Gaussian rows are staging: the kernels read the leaf-order pairs
-    if (e == cudaSuccess && fast)
+    if (e == cudaSuccess && s->d_leaf_pairs)
       e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, po.fast, s->d_leaf_pairs, W.st);
+    if (e == cudaSuccess && s->d_leaf_tol)
+      e = build_leaf_tol(s->d_pair_gid, s->n_pair_entries, po.tol, s->d_leaf_tol, W.st);
     if (e != cudaSuccess) return fail("leaf order", e);
   }
   Slab Q;
@@ -224,10 +262,10 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     // laid out as its plain entries in FP16 pairs followed by its flagged
     // entries in FP32 pairs of a second stream
     uint32_t* aidx = nullptr;
-    uint64_t *first = nullptr, totals = 0;
+    uint64_t *split = nullptr, totals = 0;
     e = aniso_index(W, po.aniso, n, &aidx, &s->n_aniso);
     if (e == cudaSuccess)
-      e = tree_split_counts(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, &first, &totals);
+      e = tree_split_counts(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, &split, &totals);
     if (e != cudaSuccess) return fail("packed leaf counts", e);
     s->n_plain_entries = 2u * (uint32_t)totals;
     s->n_flag_entries = 2u * (uint32_t)(totals >> 32);
@@ -241,7 +279,7 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     float4* table = W.take<float4>(3 * (size_t)s->n_aniso);
     e = W.err;
     if (e == cudaSuccess)
-      e = tree_split_fill(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, first, s->d_nodes_packed, s->d_leaf_aux,
+      e = tree_split_fill(W, s->d_nodes_fast, L.n, s->d_pair_gid, po.aniso, split, s->d_nodes_packed, s->d_leaf_aux,
                           s->d_gid_plain, s->d_gid_flag);
     if (e == cudaSuccess) e = build_packed_pairs(s->d_gid_plain, s->n_plain_entries, po.packed, s->d_leaf_packed, W.st);
     if (e == cudaSuccess && s->n_aniso) {
@@ -384,7 +422,7 @@ static int render_common(kdgr_scene_t s, const kdgr_camera* cam, int W, int H, f
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
   }
-  cudaError_t e = launch_exact(s->exact_view(), ci, W, H, rgb, alpha, depth, trace, s->d_status, 8, st);
+  cudaError_t e = launch_exact(s->exact_view(), s->plain_view(), ci, W, H, rgb, alpha, depth, trace, s->d_status, st);
   if (e != cudaSuccess) {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);

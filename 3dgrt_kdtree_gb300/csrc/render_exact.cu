@@ -11,130 +11,36 @@
 // instead of rsqrtf, the project exponential instead of CUDA expf -- are the
 // oracle's as well.
 //
-// GB300 layout choices, none of which change a result:
-//   * one thread per ray; a warp covers an 8x4 pixel tile, a 128-thread
-//     block a 16x8 tile, so the 32 rays of a warp start coherent;
-//   * the 12-entry ring short stack (cudaRenderer.cu:184-210, restart from
-//     the root when it runs dry, :1694-1708) lives in shared memory laid out
-//     [slot][thread], bank-conflict free;
-//   * Gaussians are split SoA: a 64-byte test record (the fields the test
-//     reads, with the reciprocal of the inverted scale precomputed by the same
-//     IEEE division) and a separate 192-byte SH record read only for
-//     composited hits;
-//   * the reference collects every hit of a leaf into a 256-entry local array
-//     (no overflow check, :1126-1133) and insertion-sorts it.  Here a K-entry
-//     register buffer keeps the K smallest (t, leaf position) keys; a leaf
-//     with more than K accepted hits is re-scanned for the next K keys, so
-//     any leaf size gives the same stable t order with no overflow.
+// Two walks give these results:
+//   * over the tree as given, one thread per ray (k_render_exact), for traces,
+//     bounced rays and scenes without the leaf-order arrays: a warp covers an
+//     8x4 pixel tile; the 12-entry ring short stack (cudaRenderer.cu:184-210,
+//     restart from the root when it runs dry, :1694-1708) lives in shared
+//     memory laid out [slot][thread]; Gaussians are an 80-byte test record
+//     (reciprocal scale and rotation rows precomputed by the same operations)
+//     and a separate 192-byte SH record read only for composited hits;
+//   * over the fast form's relaid tree and leaf-order pairs (k_render_plain,
+//     render_packet.cuh), as warp packets, independent rays or rays shared by
+//     lanes: candidates that certainly miss are discarded two at a time in
+//     FP32x2 arithmetic with a proven tolerance, the others take the same
+//     test as above.  What bounds it is the issue rate, as in the fast form:
+//     of 65.1k warp instructions per 8x4 tile (1280x720, 300k Gaussians) the
+//     filter on t* leaves 44k and that on the response 34k; 1080p on the 1M
+//     scene 4.26 -> 2.39 ms.
+// The reference collects every hit of a leaf into a 256-entry local array
+// (no overflow check, :1126-1133) and insertion-sorts it.  Here a K-entry
+// register buffer keeps the K smallest (t, leaf position) keys; a leaf
+// with more than K accepted hits is re-scanned for the next K keys, so any
+// leaf size gives the same stable t order with no overflow.
 #include <cfloat>
 #include <cstdint>
 
-#include "device_common.cuh"
-#include "kdgr_math.h"
+#include "render_packet.cuh"
 
 namespace kdgr {
 namespace {
 
-struct F3 {
-  float x, y, z;
-};
-__device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ float fq(float a) { return __fsqrt_rn(a); }
-__device__ __forceinline__ F3 mk(float x, float y, float z) { return F3{x, y, z}; }
-__device__ __forceinline__ F3 add(F3 a, F3 b) { return mk(fa(a.x, b.x), fa(a.y, b.y), fa(a.z, b.z)); }
-__device__ __forceinline__ F3 sub(F3 a, F3 b) { return mk(fs(a.x, b.x), fs(a.y, b.y), fs(a.z, b.z)); }
-__device__ __forceinline__ F3 mulv(F3 a, F3 b) { return mk(fm(a.x, b.x), fm(a.y, b.y), fm(a.z, b.z)); }
-__device__ __forceinline__ F3 muls(F3 a, float s) { return mk(fm(a.x, s), fm(a.y, s), fm(a.z, s)); }
-__device__ __forceinline__ float dot(F3 a, F3 b) { return fa(fa(fm(a.x, b.x), fm(a.y, b.y)), fm(a.z, b.z)); }
-__device__ __forceinline__ F3 cross(F3 a, F3 b) {
-  return mk(fs(fm(a.y, b.z), fm(a.z, b.y)), fs(fm(a.z, b.x), fm(a.x, b.z)), fs(fm(a.x, b.y), fm(a.y, b.x)));
-}
-
-// quaternionWXYZToMatrixTranspose (cudaRenderer.cu:808-828)
-__device__ __forceinline__ void quat_rt(float r, float x, float y, float z, F3 m[3]) {
-  const float xx = fm(x, x), yy = fm(y, y), zz = fm(z, z);
-  const float xy = fm(x, y), xz = fm(x, z), yz = fm(y, z);
-  const float rx = fm(r, x), ry = fm(r, y), rz = fm(r, z);
-  m[0] = mk(fs(1.f, fm(2.f, fa(yy, zz))), fm(2.f, fa(xy, rz)), fm(2.f, fs(xz, ry)));
-  m[1] = mk(fm(2.f, fs(xy, rz)), fs(1.f, fm(2.f, fa(xx, zz))), fm(2.f, fa(yz, rx)));
-  m[2] = mk(fm(2.f, fa(xz, ry)), fm(2.f, fs(yz, rx)), fs(1.f, fm(2.f, fa(xx, yy))));
-}
-__device__ __forceinline__ F3 mat_mul(F3 p, const F3 m[3]) { return mk(dot(m[0], p), dot(m[1], p), dot(m[2], p)); }
-
-// rayPrimIntersect with VOLUME_ISECT (cudaRenderer.cu:1070-1135).
-__device__ __forceinline__ bool exact_test(F3 o, F3 d, const float4* __restrict__ rec, float t_near, float t_far,
-                                           float* t_out, float* gray_out) {
-  const float4 r0 = __ldg(rec), r1 = __ldg(rec + 1), r2 = __ldg(rec + 2), r3 = __ldg(rec + 3);
-  const F3 pos = mk(r0.x, r0.y, r0.z);
-  const F3 giscl = mk(r1.x, r1.y, r1.z);
-  const F3 pscale = mk(r1.w, r2.x, r2.y);
-  F3 rt[3];
-  quat_rt(r2.z, r2.w, r3.x, r3.y, rt);
-  const F3 gposc = sub(o, pos);
-  const F3 gposcr = mat_mul(gposc, rt);
-  const F3 gro = mulv(giscl, gposcr);
-  const F3 ray_dir_r = mat_mul(d, rt);
-  const F3 grdu = mulv(ray_dir_r, giscl);
-  // safe_normalize with rsqrtf -> 1/sqrtf
-  const float l = fa(fa(fm(grdu.x, grdu.x), fm(grdu.y, grdu.y)), fm(grdu.z, grdu.z));
-  const F3 grd = l > 0.f ? muls(grdu, fd(1.f, fq(l))) : grdu;
-  const float grp = -dot(grd, gro);
-  const F3 grds = muls(mulv(pscale, grd), grp);
-  const float t = fm(grp < 0.f ? -1.f : 1.f, fq(dot(grds, grds)));
-  if (t < t_near || t > t_far) return false;
-  const F3 gcrod = cross(grd, gro);
-  const float gray = dot(gcrod, gcrod);
-  *t_out = t;
-  *gray_out = gray;
-  return gray < 8.f;
-}
-
-// eval_sh_final(3, dir, g) (cudaRenderer.cu:487-558), constants
-// cudaRenderer.h:33-48.
-__device__ __forceinline__ F3 eval_sh(F3 d, const float4* __restrict__ shp) {
-  float c[48];
-#pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    const float4 v = __ldg(shp + i);
-    c[4 * i] = v.x;
-    c[4 * i + 1] = v.y;
-    c[4 * i + 2] = v.z;
-    c[4 * i + 3] = v.w;
-  }
-#define SH(k) mk(c[3 * (k)], c[3 * (k) + 1], c[3 * (k) + 2])
-  const float C0 = 0.28209479177387814f, C1 = 0.4886025119029199f;
-  const float C20 = 1.0925484305920792f, C21 = -1.0925484305920792f, C22 = 0.31539156525252005f,
-              C23 = -1.0925484305920792f, C24 = 0.5462742152960396f;
-  const float C30 = -0.5900435899266435f, C31 = 2.890611442640554f, C32 = -0.4570457994644658f,
-              C33 = 0.3731763325901154f, C34 = -0.4570457994644658f, C35 = 1.445305721320277f,
-              C36 = -0.5900435899266435f;
-  F3 rad = muls(SH(0), C0);
-  const float x = d.x, y = d.y, z = d.z;
-  rad = sub(add(sub(rad, muls(SH(1), fm(C1, y))), muls(SH(2), fm(C1, z))), muls(SH(3), fm(C1, x)));
-  const float xx = fm(x, x), yy = fm(y, y), zz = fm(z, z);
-  const float xy = fm(x, y), yz = fm(y, z), xz = fm(x, z);
-  rad = add(rad, muls(SH(4), fm(C20, xy)));
-  rad = add(rad, muls(SH(5), fm(C21, yz)));
-  rad = add(rad, muls(SH(6), fm(C22, fs(fs(fm(2.f, zz), xx), yy))));
-  rad = add(rad, muls(SH(7), fm(C23, xz)));
-  rad = add(rad, muls(SH(8), fm(C24, fs(xx, yy))));
-  rad = add(rad, muls(SH(9), fm(fm(C30, y), fs(fm(3.f, xx), yy))));
-  rad = add(rad, muls(SH(10), fm(fm(C31, xy), z)));
-  rad = add(rad, muls(SH(11), fm(fm(C32, y), fs(fs(fm(4.f, zz), xx), yy))));
-  rad = add(rad, muls(SH(12), fm(fm(C33, z), fs(fs(fm(2.f, zz), fm(3.f, xx)), fm(3.f, yy)))));
-  rad = add(rad, muls(SH(13), fm(fm(C34, x), fs(fs(fm(4.f, zz), xx), yy))));
-  rad = add(rad, muls(SH(14), fm(fm(C35, z), fs(xx, yy))));
-  rad = add(rad, muls(SH(15), fm(fm(C36, x), fs(xx, fm(3.f, yy)))));
-#undef SH
-  rad = add(rad, mk(0.5f, 0.5f, 0.5f));
-  return mk(fmaxf(rad.x, 0.f), fmaxf(rad.y, 0.f), fmaxf(rad.z, 0.f));
-}
-
-constexpr int kStack = 12;       // SHORT_STACK_DEPTH, Kd-treeConverter.h:117
-constexpr int kBlock = 128;
+constexpr int kBlock = kThreads;
 
 // Trace-mode counters and sequence hashes of one ray (kdgr_ray_trace).
 struct RayStats {
@@ -152,19 +58,8 @@ template <int K, bool TRACE>
 __device__ __forceinline__ bool trace_exact(const ExactView& S, const F3 o, const F3 d, const float max_t, F3& acc,
                                             float& A, float& D, RayStats& rs, uint32_t (*s_id)[kBlock],
                                             float (*s_t)[kBlock], const int tid, uint32_t* status) {
-  // BoundsRayIntersect (cudaRenderer.cu:379-399) with IEEE division
-  float tmin = 1e-2f, tmax = FLT_MAX;
-  {
-    const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float l1 = fd(fs(S.bmin[a], oo[a]), dd[a]);
-      const float l2 = fd(fs(S.bmax[a], oo[a]), dd[a]);
-      tmin = fmaxf(fminf(l1, l2), tmin);
-      tmax = fminf(fmaxf(l1, l2), tmax);
-    }
-  }
-  if (!((tmax >= tmin) & (tmax >= 0.f))) return true;
+  float tmin, tmax;
+  if (!exact_bounds(S.bmin, S.bmax, o, d, &tmin, &tmax)) return true;
   tmax = fminf(tmax, max_t);
   if (tmin > tmax) return true;
   const float t_scene_far = tmax;
@@ -236,7 +131,7 @@ __device__ __forceinline__ bool trace_exact(const ExactView& S, const F3 o, cons
             return false;
           }
           float t, g;
-          if (!exact_test(o, d, S.test + 4ull * gid, t_near, t_far, &t, &g)) continue;
+          if (!exact_test(o, d, S.test + kTestWords * (size_t)gid, t_near, t_far, &t, &g)) continue;
           if (TRACE && !have_last) ++n_acc;
           if (have_last && !(t > last_t || (t == last_t && i > last_i))) continue;
           float ct = t, cg = g;
@@ -268,15 +163,7 @@ __device__ __forceinline__ bool trace_exact(const ExactView& S, const F3 o, cons
             ++rs.n_hit;
             rs.hh = fnv_add(rs.hh, gid);
           }
-          const float opacity = __ldg(&S.test[4ull * gid].w);
-          const float gres = kdgr_expf(fm(fm(-0.0555555555556f, bg[k]), bg[k]));
-          const float alpha = fminf(0.99f, fm(opacity, gres));
-          if (gres < 0.0113f || alpha < 1.0f / 255.0f) continue;
-          const F3 c = eval_sh(d, S.sh + 12ull * gid);
-          const float w = fm(alpha, fs(1.f, A));
-          acc = add(acc, muls(muls(c, alpha), fs(1.f, A)));
-          D = fa(D, fm(bt[k], w));
-          A = fa(A, fm(alpha, fs(1.f, A)));
+          if (!exact_blend(S.test + kTestWords * (size_t)gid, S.sh + 12ull * gid, d, bt[k], bg[k], acc, A, D)) continue;
           if (TRACE) {
             ++rs.n_blend;
             rs.hb = fnv_add(rs.hb, gid);
@@ -317,7 +204,7 @@ __device__ __forceinline__ bool trace_exact(const ExactView& S, const F3 o, cons
 }
 
 // Pixel of thread `tid` in a 16x8 block: warps cover 8x4 tiles.
-__device__ __forceinline__ void block_pixel(int tid, int* x, int* y) {
+__device__ __forceinline__ void thread_pixel(int tid, int* x, int* y) {
   const int lane = tid & 31, warp = tid >> 5;
   *x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
   *y = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
@@ -337,6 +224,50 @@ __device__ __forceinline__ F3 primary_dir(const CamInfo& C, int x, int y) {
 
 __device__ __forceinline__ F3 normalize3(F3 v) { return muls(v, fd(1.f, fq(dot(v, v)))); }
 
+// The plain form (render_packet.cuh): each warp renders one 8x4 tile, or with
+// LPR lanes per ray a tile of 32 / LPR rays, of its 16x8 block, as packets
+// (PKT) or each lane its own ray.
+template <int LPR, int MINB, bool PKT>
+__global__ void __launch_bounds__(kThreads, MINB) k_render_plain(PlainView S, CamInfo C, int W, int H, uint32_t n_items,
+                                                                 float* __restrict__ rgb,
+                                                                 float* __restrict__ alpha_out,
+                                                                 float* __restrict__ depth_out, uint32_t* status) {
+  __shared__ uint32_t s_id[kStack][kThreads];
+  __shared__ float s_t[kStack][kThreads];
+  __shared__ PktEnt s_ent[kStack][kWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t it = blockIdx.x * kWarps + warp;
+  if (it >= n_items) return;
+  const uint32_t blk = it / (4u * LPR), q = it % (4u * LPR), nx = (uint32_t)((W + kBlockW - 1) / kBlockW);
+  const int bx = (int)(blk % nx) * kBlockW, by = (int)(blk / nx) * kBlockH;
+  int x, y;
+  if constexpr (LPR == 1) block_pixel(KDGR_TILE_8X4, bx, by, (int)q, lane, x, y);
+  else group_pixel<LPR>(bx, by, (int)q, lane, x, y);
+  const bool inimg = x < W && y < H;
+  Ray R;
+  R.A = 0.f;
+  *acc_slot() = make_float4(0.f, 0.f, 0.f, 0.f);
+  const F3 d = primary_dir(C, inimg ? x : 0, inimg ? y : 0);
+  const bool live = ray_init_plain(S, mk(C.eye[0], C.eye[1], C.eye[2]), d, FLT_MAX, R) && inimg;
+  if constexpr (PKT) {
+    trace_packets<kHits, kFormPlain, LPR>(S, R, live, sign_bits(d), s_id, s_t, s_ent, tid, status);
+  } else if (live) {
+    R.cur = R.steps = 0;
+    R.top = kStack - 1;
+    R.quant = 0;
+    while (R.A < 0.99f && !leaf_step<kHits, kFormPlain, LPR>(S, s_id, s_t, tid, R, status)) {
+    }
+  }
+  if (!inimg || (tid & (LPR - 1)) != 0) return;
+  const size_t idx = (size_t)(H - 1 - y) * W + x;  // rows flipped (cudaRenderer.cu:2370)
+  const float4 v = *acc_slot();
+  rgb[3 * idx] = v.x;
+  rgb[3 * idx + 1] = v.y;
+  rgb[3 * idx + 2] = v.z;
+  if (alpha_out) alpha_out[idx] = R.A;
+  if (depth_out) depth_out[idx] = v.w;
+}
+
 template <int K, bool TRACE>
 __global__ void __launch_bounds__(kBlock) k_render_exact(ExactView S, CamInfo C, int W, int H, float* __restrict__ rgb,
                                                          float* __restrict__ alpha_out, float* __restrict__ depth_out,
@@ -345,7 +276,7 @@ __global__ void __launch_bounds__(kBlock) k_render_exact(ExactView S, CamInfo C,
   __shared__ float s_t[kStack][kBlock];
   const int tid = threadIdx.x;
   int x, y;
-  block_pixel(tid, &x, &y);
+  thread_pixel(tid, &x, &y);
   if (x >= W || y >= H) return;
   const F3 o = mk(C.eye[0], C.eye[1], C.eye[2]);
   const F3 d = primary_dir(C, x, y);
@@ -470,7 +401,7 @@ __global__ void __launch_bounds__(kBlock) k_render_hybrid(ExactView S, CamInfo C
   __shared__ float s_t[kStack][kBlock];
   const int tid = threadIdx.x;
   int x, y;
-  block_pixel(tid, &x, &y);
+  thread_pixel(tid, &x, &y);
   if (x >= W || y >= H) return;
   F3 o = mk(C.eye[0], C.eye[1], C.eye[2]);
   F3 d = primary_dir(C, x, y);
@@ -519,29 +450,52 @@ __global__ void __launch_bounds__(kBlock) k_render_hybrid(ExactView S, CamInfo C
   rgb[3 * idx + 2] = fminf(fin.z, 1.0f);
 }
 
-template <int K>
-cudaError_t launch_k(const ExactView& s, const CamInfo& cam, int W, int H, float* rgb, float* alpha, float* depth,
-                     kdgr_ray_trace* trace, uint32_t* status, cudaStream_t st) {
-  dim3 grid((W + 15) / 16, (H + 7) / 8);
-  if (trace)
-    k_render_exact<K, true><<<grid, kBlock, 0, st>>>(s, cam, W, H, rgb, alpha, depth, trace, status);
-  else
-    k_render_exact<K, false><<<grid, kBlock, 0, st>>>(s, cam, W, H, rgb, alpha, depth, trace, status);
+template <int LPR, int MINB, bool PKT>
+cudaError_t launch_plain(const PlainView& s, const CamInfo& cam, int W, int H, float* rgb, float* alpha, float* depth,
+                         uint32_t* status, cudaStream_t st) {
+  const uint64_t blocks = (uint64_t)((W + kBlockW - 1) / kBlockW) * ((H + kBlockH - 1) / kBlockH);
+  if (blocks * LPR > 0x3FFFFFFFull) return cudaErrorInvalidValue;
+  k_render_plain<LPR, MINB, PKT><<<(unsigned)(blocks * LPR), kThreads, 0, st>>>(s, cam, W, H, (uint32_t)(blocks * 4 * LPR),
+                                                                           rgb, alpha, depth, status);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_exact(const ExactView& s, const CamInfo& cam, int W, int H, float* rgb, float* alpha, float* depth,
-                         kdgr_ray_trace* trace, uint32_t* status, int kbuf, cudaStream_t st) {
-  switch (kbuf) {
-    case 4:
-      return launch_k<4>(s, cam, W, H, rgb, alpha, depth, trace, status, st);
-    case 16:
-      return launch_k<16>(s, cam, W, H, rgb, alpha, depth, trace, status, st);
-    default:
-      return launch_k<8>(s, cam, W, H, rgb, alpha, depth, trace, status, st);
+cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamInfo& cam, int W, int H, float* rgb,
+                         float* alpha, float* depth, kdgr_ray_trace* trace, uint32_t* status, cudaStream_t st) {
+  if (!trace && plain.leaf_tol) {
+    // How the rays are laid on the lanes, by their number (GB300: 152 SMs, 24
+    // or 32 resident warps each).  Few rays leave the chip idle and a frame
+    // takes as long as its longest ray, so lanes share rays; many rays keep it
+    // busy, and the packet walk saves loads and instructions once a tile's
+    // rays meet mostly the same leaves.  us over cluster scenes of 10k / 100k
+    // / 300k Gaussians, one thread per ray over the tree as given first:
+    //   10k rays   257 / 490 / 510   8 lanes, own walk 112 / 196 / 225
+    //   40k rays   265 / 486 / 526   4 lanes, packets  176 / 340 / 376   (8 lanes 198 / 437 / 520)
+    //   110k rays  246 / 547 / 726   1 lane, own walk  178 / 405 / 475   (packets 233 / 633 / 572)
+    //   400k rays  477 / 1215 / 1472 packets           305 / 757 / 880   (own walk 281 / 821 / 1011)
+    //   2.1M rays  (1M Gaussians) 4260, packets 2504, with 64 registers 2394
+    const uint64_t rays = (uint64_t)W * H;
+    // Gaussians that sit in more than 64 leaves each: their leaf-order copies
+    // outgrow L2 where the records themselves do not (100k overlapping
+    // Gaussians, 175 leaves each: 980 MB against 8 MB), so the walk over the
+    // tree as given is the faster one unless rays are few (65k rays: 410 us,
+    // 4 lanes per ray 360; 250k rays: 540, packets 950, own walk 560).
+    const bool copies = s.n_offsets / 64u > s.n_gauss;
+    if (rays < 30000) return launch_plain<8, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (copies && rays < 70000) return launch_plain<4, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies && rays < 60000) return launch_plain<4, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies && rays < 300000) return launch_plain<1, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies && rays < 1000000) return launch_plain<1, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
   }
+  dim3 grid((W + 15) / 16, (H + 7) / 8);
+  if (trace)
+    k_render_exact<8, true><<<grid, kBlock, 0, st>>>(s, cam, W, H, rgb, alpha, depth, trace, status);
+  else
+    k_render_exact<8, false><<<grid, kBlock, 0, st>>>(s, cam, W, H, rgb, alpha, depth, trace, status);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_hybrid(const ExactView& s, const CamInfo& cam, int W, int H, const HybridView& m, float* rgb,

@@ -37,7 +37,8 @@ struct kdgr_scene_s {
   // records are zero)
   uint32_t* d_pair_gid = nullptr;
   uint32_t n_pair_entries = 0;     // even
-  float4* d_leaf_pairs = nullptr;  // FP32 form, 6 x float4 per pair of entries
+  float4* d_leaf_pairs = nullptr;  // FP32 and plain forms, 6 x float4 per pair of entries
+  float4* d_leaf_tol = nullptr;    // plain form, 1 x float4 per pair of entries
   uint4* d_leaf_packed = nullptr;  // packed form, 4 x uint4 per pair of plain entries
   // The packed form's own leaf layout: a leaf's plain entries in FP16 pairs
   // (d_leaf_packed), its flagged entries (scale ratio > 1e3 or factors beyond
@@ -57,6 +58,7 @@ struct kdgr_scene_s {
 
   kdgr::ExactView exact_view() const;
   kdgr::FastView fast_view(bool packed) const;
+  kdgr::PlainView plain_view() const;
 };
 
 namespace kdgr {
@@ -167,6 +169,8 @@ constexpr uint32_t kPadGid = 0xFFFFFFFFu;
 // (entry aidx[gid]).  Asynchronous on `st`.
 cudaError_t build_leaf_pairs(const uint32_t* d_gid, uint32_t n_entries, const float4* test, float4* pairs,
                              cudaStream_t st);
+cudaError_t build_leaf_tol(const uint32_t* d_gid, uint32_t n_entries, const float2* tol, float4* out,
+                           cudaStream_t st);
 cudaError_t build_packed_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* src, uint4* pairs,
                                cudaStream_t st);
 cudaError_t build_flag_pairs(const uint32_t* d_gid, uint32_t n_entries, const uint32_t* aidx, const float4* table,
@@ -211,7 +215,8 @@ constexpr double kAnisoRatio = 1e3;
 struct PackOut {
   float* giscl;         // 3 per Gaussian: inverse scale as uploaded by the reference's caller
   float4* sh;           // 12 per Gaussian: FP32 SH, coefficient-major
-  float4* test;         // 4 per Gaussian: the plain kernel's test record
+  float4* test;         // kTestWords per Gaussian: the plain form's test record
+  float2* tol;          // 1 per Gaussian: the plain form's filter tolerance (Ce, Cmu)
   float4* fast;         // 3 per Gaussian: rows of M and b (FP64 -> FP32)
   float* opacity;       // 1 per Gaussian
   uint32_t* packed;     // 8 per Gaussian: FP32 mean + FP16 entries of M (precision form staging)

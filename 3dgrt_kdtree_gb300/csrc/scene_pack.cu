@@ -10,8 +10,9 @@
 //     Kd-treeConverterMain.cpp:3636-3650 unless the records are inverted);
 //   * SH coefficients coefficient-major (f_dc, then f_rest channel-major
 //     re-ordered, cudaRenderer.cu:494-499);
-//   * the plain kernel's 64-byte test record: position, opacity, inverse
-//     scale, its IEEE reciprocal (cudaRenderer.cu:1091) and the quaternion;
+//   * the plain form's 80-byte test record: position, opacity, inverse scale,
+//     its IEEE reciprocal (cudaRenderer.cu:1091) and the rotation's FP32 rows,
+//     and the constants of its candidate filter's tolerance;
 //   * the fast form's rows of M = diag(1/s) R^T and b = M mu, computed in
 //     FP64 from R^T of quaternionWXYZToMatrixTranspose (cudaRenderer.cu:
 //     808-828) and stored FP32; the opacity array;
@@ -63,6 +64,25 @@ __device__ __forceinline__ void quat_rt_d(const float* q, double m[3][3]) {
   m[2][2] = ds(1.0, dm(2.0, da(xx, yy)));
 }
 
+// The same in FP32, in the order of the reference's operations.
+__device__ __forceinline__ void quat_rt_f(const float* q, float m[9]) {
+  auto mul = [](float a, float b) { return __fmul_rn(a, b); };
+  auto add = [](float a, float b) { return __fadd_rn(a, b); };
+  auto sub = [](float a, float b) { return __fsub_rn(a, b); };
+  const float r = q[0], x = q[1], y = q[2], z = q[3];
+  const float xx = mul(x, x), yy = mul(y, y), zz = mul(z, z), xy = mul(x, y), xz = mul(x, z), yz = mul(y, z);
+  const float rx = mul(r, x), ry = mul(r, y), rz = mul(r, z);
+  m[0] = sub(1.f, mul(2.f, add(yy, zz)));
+  m[1] = mul(2.f, add(xy, rz));
+  m[2] = mul(2.f, sub(xz, ry));
+  m[3] = mul(2.f, sub(xy, rz));
+  m[4] = sub(1.f, mul(2.f, add(xx, zz)));
+  m[5] = mul(2.f, add(yz, rx));
+  m[6] = mul(2.f, add(xz, ry));
+  m[7] = mul(2.f, sub(yz, rx));
+  m[8] = sub(1.f, mul(2.f, add(xx, yy)));
+}
+
 __global__ void k_pack(const float* __restrict__ rec, uint32_t n, int inverted, PackOut o) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -96,11 +116,30 @@ __global__ void k_pack(const float* __restrict__ rec, uint32_t n, int inverted, 
     for (int c = 0; c < 3; ++c) o.giscl[3ull * i + c] = gs[c];
   }
   if (o.test) {  // particleScale = 1 / giscl, cudaRenderer.cu:1091
-    float4* d = o.test + 4ull * i;
+    float m[9];
+    quat_rt_f(r + 8, m);
+    float4* d = o.test + (size_t)kTestWords * i;
     d[0] = make_float4(r[0], r[1], r[2], r[3]);
     d[1] = make_float4(gs[0], gs[1], gs[2], __fdiv_rn(1.0f, gs[0]));
-    d[2] = make_float4(__fdiv_rn(1.0f, gs[1]), __fdiv_rn(1.0f, gs[2]), r[8], r[9]);
-    d[3] = make_float4(r[10], r[11], 0.f, 0.f);
+    d[2] = make_float4(__fdiv_rn(1.0f, gs[1]), __fdiv_rn(1.0f, gs[2]), m[0], m[1]);
+    d[3] = make_float4(m[2], m[3], m[4], m[5]);
+    d[4] = make_float4(m[6], m[7], m[8], 0.f);
+  }
+  if (o.tol) {
+    // constants of the plain form's filter tolerance (render_packet.cuh);
+    // infinite (the filter never discards) outside the ranges its bound covers
+    const double q2 = (double)r[8] * r[8] + (double)r[9] * r[9] + (double)r[10] * r[10] + (double)r[11] * r[11];
+    const double mu2 = (double)r[0] * r[0] + (double)r[1] * r[1] + (double)r[2] * r[2];
+    double g2 = 0.0;
+    bool covered = fabs(q2 - 1.0) <= 2e-6 && mu2 < 1e16;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      g2 += (double)gs[c] * gs[c];
+      covered = covered && fabsf(gs[c]) >= 1e-8f && fabsf(gs[c]) <= 1e8f;
+    }
+    const double ce = g2 * 4.656612873077393e-10;  // 2^-31
+    const float inf = __int_as_float(0x7f800000);
+    o.tol[i] = covered ? make_float2(__double2float_ru(ce), __double2float_ru(ce * mu2)) : make_float2(inf, inf);
   }
   if (o.opacity) o.opacity[i] = r[3];
   double m[3][3];
