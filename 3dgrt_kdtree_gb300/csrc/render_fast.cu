@@ -227,8 +227,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_render_batch(FastView S, con
 // quarters of 16x8 blocks; queue word 1 + k counts the claims of strip k.
 // outs[v] is view v's output base (the device arena, or a request's
 // page-locked host buffer); the view's out_off counts pixels from it.
-template <bool PACKED>
-__global__ void __launch_bounds__(kThreads, 8) k_render_multi(const __grid_constant__ SceneTable scenes,
+// PKT, LPR: the walk, as in k_render_batch.
+template <bool PACKED, int MINB, bool PKT, int LPR>
+__global__ void __launch_bounds__(kThreads, MINB) k_render_multi(const __grid_constant__ SceneTable scenes,
                                                               const ViewDesc* __restrict__ views, int n_views,
                                                               uint32_t total_items, float* const* __restrict__ outs,
                                                               uint32_t* queue, uint32_t* status, int n_strips) {
@@ -251,15 +252,17 @@ __global__ void __launch_bounds__(kThreads, 8) k_render_multi(const __grid_const
       if (k >= n) break;
       continue;
     }
-    const uint32_t blk = it >> 2;
+    const uint32_t blk = it / (4u * LPR), q = it % (4u * LPR);
     const int vi = find_view(views, n_views, blk, KDGR_SCHED_CTA_BLOCKS);
     const ViewDesc& V = views[vi];
     const FastView& S = scenes.s[__ldg(&V.scene) & (kSceneSlots - 1)];
     float* const rgb = outs[vi];
     const uint32_t lb = blk - __ldg(&V.cb_base), nx = __ldg(&V.cb_x);
     int x, y;
-    block_pixel(KDGR_TILE_8X4, (int)(lb % nx) * kBlockW, (int)(lb / nx) * kBlockH, (int)(it & 3u), lane, x, y);
-    render_px<kHits, PACKED ? kFormPacked : kFormFp32, true, 1>(S, V, x, y, s_id, s_t, s_ent, tid, rgb, nullptr, nullptr, status);
+    const int bx = (int)(lb % nx) * kBlockW, by = (int)(lb / nx) * kBlockH;
+    if constexpr (LPR == 1) block_pixel(KDGR_TILE_8X4, bx, by, (int)q, lane, x, y);
+    else group_pixel<LPR>(bx, by, (int)q, lane, x, y);
+    render_px<kHits, PACKED ? kFormPacked : kFormFp32, PKT, LPR>(S, V, x, y, s_id, s_t, s_ent, tid, rgb, nullptr, nullptr, status);
   }
 }
 
@@ -299,9 +302,10 @@ KernelFn pick_minb(int minb) {
   return k_render_batch<PACKED, SCHED, 0, KB, PKT, LPR>;
 }
 
-// Lanes per ray: 32 / rays_per_warp (warp-strip schedule only).
+// Lanes per ray: 32 / rays_per_warp (warp-strip schedule only; 4 rays per
+// warp only from choose_walk).
 int lanes_per_ray(const kdgr_batch_config& c) {
-  return c.rays_per_warp == 8 ? 4 : c.rays_per_warp == 16 ? 2 : 1;
+  return c.rays_per_warp == 4 ? 8 : c.rays_per_warp == 8 ? 4 : c.rays_per_warp == 16 ? 2 : 1;
 }
 
 template <bool PACKED, int KB, bool PKT>
@@ -309,6 +313,8 @@ KernelFn pick_sched_k(const kdgr_batch_config& c) {
   if (c.schedule == KDGR_SCHED_CTA_BLOCKS) return pick_minb<PACKED, KDGR_SCHED_CTA_BLOCKS, KB, PKT, 1>(c.min_blocks);
   if (c.schedule == KDGR_SCHED_SM_STRIPS) return pick_minb<PACKED, KDGR_SCHED_SM_STRIPS, KB, PKT, 1>(c.min_blocks);
   if (c.schedule == KDGR_SCHED_WARP_STRIPS) {
+    if constexpr (KB == kHits && PKT)  // choose_walk's small launches only
+      if (lanes_per_ray(c) == 8) return k_render_batch<PACKED, KDGR_SCHED_WARP_STRIPS, 6, KB, PKT, 8>;
     if (lanes_per_ray(c) == 4) return pick_minb<PACKED, KDGR_SCHED_WARP_STRIPS, KB, PKT, 4>(c.min_blocks);
     if (lanes_per_ray(c) == 2) return pick_minb<PACKED, KDGR_SCHED_WARP_STRIPS, KB, PKT, 2>(c.min_blocks);
     return pick_minb<PACKED, KDGR_SCHED_WARP_STRIPS, KB, PKT, 1>(c.min_blocks);
@@ -468,10 +474,41 @@ int check_batch_config(kdgr_scene_t s, const kdgr_batch_config& c) {
   return KDGR_OK;
 }
 
+// How few rays a launch may have before its walk changes.  One frame of R rays
+// on the default walk (packets of 32 rays, 64 registers) takes as long as its
+// longest packet when R is small; us on a GB300, default first, over cluster
+// scenes of 10k / 100k / 300k Gaussians and a dense uniform one (100k):
+//   10k rays   349 / 891 / 799 / 1670   4-ray packets 115 / 206 / 200 / 270
+//   40k rays   246 / 596 / 535 / 1438   own walk      160 / 298 / 334 / 293   (4-ray packets 177 / 325 / 356 / 312)
+//   160k rays  234 / 526 / 458 / 1099   own walk      194 / 424 / 446 / 401
+//   400k rays  282 / 629 / 696 / 783    own walk      282 / 650 / 748 / 521
+// A scene whose Gaussians sit in more than 64 leaves each (the last one) has
+// leaves far smaller than a tile: its rays share too few of them for packets
+// up to a full frame (1.1M rays: 924 us, own walk 850).
+constexpr uint64_t kFewRays = 30000, kSomeRays = 250000, kSomeRaysDense = 1200000;
+
+// The configuration a launch runs with: a caller's own choice as it is; the
+// default one (precision apart) with the walk that suits the number of rays.
+// Every walk gives the same pixels bit for bit.
+kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64_t rays) {
+  kdgr_batch_config d;
+  kdgr_batch_config_default(&d);
+  d.precision = c.precision;
+  if (memcmp(&d, &c, sizeof d) != 0) return c;
+  const bool dense = s->n_pair_entries / 64u > s->n_gauss;
+  if (rays >= (dense ? kSomeRaysDense : kSomeRays)) return c;
+  d.schedule = KDGR_SCHED_WARP_STRIPS;
+  d.min_blocks = 6;
+  if (rays < kFewRays) d.rays_per_warp = 4;
+  else d.traversal = KDGR_TRAV_RAY;
+  return d;
+}
+
 // Launch the persistent kernel.  `queue` must read 0 when the kernel starts.
-cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& c, const ViewDesc* d_views, int n_views,
+cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& cc, const ViewDesc* d_views, int n_views,
                          const uint32_t totals[3], float* rgb, float* alpha, float* depth, uint32_t* queue,
                          cudaStream_t st) {
+  const kdgr_batch_config c = choose_walk(s, cc, 32ull * totals[0]);
   const uint32_t total_tiles = totals[0], total_blocks = totals[1];
   KernelFn fn = pick_kernel(c);
   int per_sm = c.blocks_per_sm;
@@ -643,16 +680,21 @@ cudaError_t stage_views(const ViewDesc* views, int n_views, ViewDesc* d_views, u
 cudaError_t launch_multi(const SceneTable& scenes, bool packed, const ViewDesc* d_views, int n_views,
                          uint32_t total_blocks, float* const* d_outs, uint32_t* queue, uint32_t* status,
                          cudaStream_t st) {
-  auto fn = packed ? k_render_multi<true> : k_render_multi<false>;
+  // the walk by the number of rays, as choose_walk (the scenes may differ)
+  const uint64_t rays = (uint64_t)kBlockW * kBlockH * total_blocks;
+  const uint32_t lpr = rays < kFewRays ? 8 : 1;
+  auto fn = packed ? k_render_multi<true, 8, true, 1> : k_render_multi<false, 8, true, 1>;
+  if (lpr == 8) fn = packed ? k_render_multi<true, 6, true, 8> : k_render_multi<false, 6, true, 8>;
+  else if (rays < kSomeRays) fn = packed ? k_render_multi<true, 6, false, 1> : k_render_multi<false, 6, false, 1>;
   int occ = 0;
   cudaError_t e = resident_ctas(reinterpret_cast<const void*>(fn), &occ);
   if (e != cudaSuccess) return e;
   if (total_blocks > 0x3FFFFFFFu) return cudaErrorInvalidValue;
-  const uint32_t quarters = 4u * total_blocks;
+  const uint32_t items = 4u * lpr * total_blocks;
   uint64_t blocks = (uint64_t)num_sms() * (occ > 0 ? occ : 1);
-  const uint64_t cap = ((uint64_t)quarters + kWarps - 1) / kWarps;
+  const uint64_t cap = ((uint64_t)items + kWarps - 1) / kWarps;
   if (blocks > cap) blocks = cap > 0 ? cap : 1;
-  fn<<<(unsigned)blocks, kThreads, 0, st>>>(scenes, d_views, n_views, quarters, d_outs, queue, status,
+  fn<<<(unsigned)blocks, kThreads, 0, st>>>(scenes, d_views, n_views, items, d_outs, queue, status,
                                             std::min(num_sms(), kMaxStrips));
   return cudaGetLastError();
 }
