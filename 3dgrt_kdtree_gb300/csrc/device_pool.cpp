@@ -11,6 +11,7 @@ struct Pools {
   std::mutex mu;
   cudaMemPool_t pool[kMaxDevices] = {};
   int users[kMaxDevices] = {};
+  size_t keep[kMaxDevices] = {};
 };
 Pools& pools() {
   static Pools p;
@@ -36,6 +37,9 @@ cudaError_t work_pool_enter(int dev, cudaMemPool_t* out) {
       cudaMemPoolDestroy(pool);
       return e;
     }
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) total = 0;
+    P.keep[dev] = total / kWorkPoolShare;
     P.pool[dev] = pool;
   }
   ++P.users[dev];
@@ -47,7 +51,7 @@ void work_pool_leave(int dev) {
   if (dev < 0 || dev >= kMaxDevices) return;
   Pools& P = pools();
   std::lock_guard<std::mutex> lk(P.mu);
-  if (--P.users[dev] == 0) cudaMemPoolTrimTo(P.pool[dev], kWorkPoolKeep);
+  if (--P.users[dev] == 0) cudaMemPoolTrimTo(P.pool[dev], P.keep[dev]);
 }
 
 void work_pool_trim(int dev) {

@@ -39,8 +39,11 @@
 // sequential sweep does, took a global 64-bit radix sort of all edges per
 // level and about 60 FP64 operations per edge on a chip with two FP64 lanes
 // per SM; events are 3 to 20 times fewer than edges, and FP64 is left for a
-// handful of candidates per node.  Measured on a GB300, whole call: 10k
-// Gaussians 15.5 -> 4.9 ms, 500k 337 -> 87 ms, 1M 723 -> 180 ms.
+// handful of candidates per node -- for none where a single position is left.
+// Measured on a GB300, whole call: 10k Gaussians 15.5 -> 4.0 ms, 500k 337 ->
+// 61 ms, 1M 723 -> 134 ms.  Of the 500k build's 49 ms of kernels the partition
+// takes 11 (3.4 TB/s), the searches 15, the scans 7, the sorts of large nodes
+// 4; small builds are bound by their levels' launches and latencies.
 //
 // This unit is compiled with --fmad=false and IEEE division, so every float
 // and double expression rounds as on the host (compiled -ffp-contract=off).
@@ -60,7 +63,11 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 #include "device_pool.h"
 #include "kdgr.h"
@@ -78,9 +85,10 @@ constexpr uint32_t kFaces = 20;      // triangles per proxy: triangle t belongs 
 
 // Relative slack between FP32 and FP64 scores.  Every term of a score is
 // positive (costs and extents; other parameters switch the FP32 filter off),
-// so the FP32 value of its at most 20 roundings is within 1.3e-6; the gap
-// bound adds as much again.
-constexpr float kMargin = 5e-5f;
+// so an FP32 score, at most 16 roundings from the same float inputs, is within
+// 1e-6 of the FP64 one: a candidate that is not worse than the best in FP64 is
+// at most 2e-6 above it in FP32.  Twice that is allowed.
+constexpr float kMargin = 4e-6f;
 
 struct Params {
   int max_level;
@@ -353,12 +361,16 @@ struct Decision {
 // a 512-thread block 86 KB, two per SM; beyond that a node alone keeps many
 // blocks busy and its keys go through the device-wide sort.
 constexpr uint32_t kWarpIds = 64, kMidIds = 256, kBlockIds = 1024;
+// A level of few nodes takes as long as its slowest node: below this many
+// nodes every one gets a 128-thread block (10k Gaussians: a warp took up to
+// 130 us for a node of 64 IDs).
+constexpr uint32_t kFewNodes = 4096;
 
 // Per node: its first run, its ID count, the class lists of its split search
 // (nodes of up to kWarpIds need no list) and a leaf decision to begin with.
 // counts: [0] kMidIds nodes, [1] kBlockIds nodes, [2] larger nodes.
 __global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ ridx, uint32_t N,
-                             int level, int max_level, uint32_t* rb, Decision* dec, uint32_t* is_split,
+                             int level, int max_level, uint32_t warp_ids, uint32_t* rb, Decision* dec, uint32_t* is_split,
                              uint32_t* list_mid, uint32_t* list_block, uint32_t* counts, uint32_t* eG) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n > N) return;
@@ -371,7 +383,7 @@ __global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __
   dec[n] = Decision{-1, 0.f, 0};
   is_split[n] = 0u;
   const bool elig = level < max_level && G > kMinPrim;
-  if (elig && G > kWarpIds && G <= kMidIds) list_mid[atomicAdd(&counts[0], 1u)] = n;
+  if (elig && G > warp_ids && G <= kMidIds) list_mid[atomicAdd(&counts[0], 1u)] = n;
   if (elig && G > kMidIds && G <= kBlockIds) list_block[atomicAdd(&counts[1], 1u)] = n;
   if (eG) {
     const bool big = elig && G > kBlockIds;
@@ -538,6 +550,8 @@ struct SearchMem {
   uint32_t pl[3][CAP];      // planar positions, unsorted
   float cost[6][CAP], bound[6][CAP];
   uint32_t n_pl[3], hull_lo[3], hull_hi[3];
+  uint64_t cand[CAP];       // candidates within the margin: axis << 32 | ordf(position)
+  uint32_t n_cand;
   float red[NT / 32];
   double best_c[NT / 32];
   uint64_t best_k[NT / 32];
@@ -549,55 +563,76 @@ __device__ __forceinline__ void group_sync() {
   else __syncthreads();
 }
 
-// tid: index inside the group.  n: node; runs [r0, r0 + G), triangles [t0, t1).
+// tid: index inside the group.  n: node; runs [r0, r0 + G), triangles [t0, t1); ridx[t + 1] - 1: run of triangle t.
 template <int NT, int CAP>
 __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, const Params& P, uint32_t n, uint32_t r0,
                                             uint32_t G, uint32_t t0, uint32_t t1,
-                                            const uint32_t* __restrict__ run_start, const TriView& V,
+                                            const uint32_t* __restrict__ ridx, const TriView& V,
                                             const float* __restrict__ nlo, const float* __restrict__ nhi,
                                             Decision* dec, uint32_t* is_split) {
   const float kInf = __int_as_float(0x7f800000);
-  uint32_t M = 32;
-  while (M < G) M <<= 1;
+  uint32_t M = 32, shift = 5;
+  while (M < G) {
+    M <<= 1;
+    ++shift;
+  }
+  if (tid == 0) S.n_cand = 0u;
   if (tid < 3) {
     S.n_pl[tid] = 0u;
     S.hull_lo[tid] = 0xFFFFFFFFu;
     S.hull_hi[tid] = 0u;
   }
   group_sync<NT>();
-  for (uint32_t r = tid; r < M; r += NT) {
-    uint32_t km[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
-    if (r < G) {
-      const uint32_t a0 = run_start[r0 + r], a1 = r + 1 < G ? run_start[r0 + r + 1] : t1;
-      float mn[3], mx[3];
+  for (uint32_t r = tid; r < M; r += NT)
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        mn[a] = V.lo[a * V.cap + a0];
-        mx[a] = V.hi[a * V.cap + a0];
-      }
-      for (uint32_t t = a0 + 1; t < a1; ++t)
+    for (int a = 0; a < 3; ++a) {
+      S.k[a][r] = 0xFFFFFFFFu;
+      S.k[3 + a][r] = r < G ? 0u : 0xFFFFFFFFu;
+    }
+  group_sync<NT>();
+  // Interval of every ID: a warp takes 32 triangles at a time, coalesced,
+  // reduces each run's part of them by shuffles and the run's first lane
+  // merges it.
+  for (uint32_t b = t0 + (tid & ~31u); b < t1; b += NT) {
+    const uint32_t t = b + (tid & 31u), tc = min(t, t1 - 1);
+    const uint32_t r = ridx[tc + 1] - 1u - r0;
+    uint32_t v[6];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float l = V.lo[a * V.cap + t], h = V.hi[a * V.cap + t];
-          if (l < mn[a]) mn[a] = l;
-          if (h > mx[a]) mx[a] = h;
-        }
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        km[a] = ordz(mn[a]);
-        km[3 + a] = ordz(mx[a]);
-        if (mn[a] == mx[a]) S.pl[a][atomicAdd(&S.n_pl[a], 1u)] = km[a];
-      }
+    for (int a = 0; a < 3; ++a) {
+      v[a] = ordz(V.lo[a * V.cap + tc]);
+      v[3 + a] = ordz(V.hi[a * V.cap + tc]);
     }
 #pragma unroll
-    for (int l = 0; l < 6; ++l) S.k[l][r] = km[l];
+    for (int o = 1; o < 32; o <<= 1) {
+      // runs are contiguous: lane + o is in this lane's run if its index is the same
+      const bool same = __shfl_down_sync(0xFFFFFFFFu, r, o) == r && (tid & 31u) + o < 32u;
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        const uint32_t w = __shfl_down_sync(0xFFFFFFFFu, v[l], o);
+        if (same) v[l] = l < 3 ? min(v[l], w) : max(v[l], w);
+      }
+    }
+    const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, r, 1);
+    const bool head = (tid & 31u) == 0u || before != r;
+    if (head && t < t1) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        atomicMin(&S.k[a][r], v[a]);
+        atomicMax(&S.k[3 + a][r], v[3 + a]);
+      }
+    }
   }
+  group_sync<NT>();
+  for (uint32_t r = tid; r < G; r += NT)
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      if (S.k[a][r] == S.k[3 + a][r]) S.pl[a][atomicAdd(&S.n_pl[a], 1u)] = S.k[a][r];
   group_sync<NT>();
   // bitonic sort of the six lists
   for (uint32_t size = 2; size <= M; size <<= 1)
     for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
       for (uint32_t i = tid; i < 6 * (M / 2); i += NT) {
-        const uint32_t l = i / (M / 2), j = i & (M / 2 - 1);
+        const uint32_t l = i >> (shift - 1), j = i & (M / 2 - 1);
         const uint32_t x = 2 * j - (j & (stride - 1)), y = x + stride;
         const uint32_t u = S.k[l][x], v = S.k[l][y];
         if ((u > v) == ((x & size) == 0)) {
@@ -619,16 +654,30 @@ __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, cons
   };
   // events: FP32 score, and a lower bound over the gap up to the next event
   float best32 = c.init;
-  for (uint32_t i = tid; i < 6 * G; i += NT) {
-    const uint32_t l = i / G, j = i - l * G;
-    const int a = (int)(l % 3);
+  for (uint32_t i = tid; i < 6 * M; i += NT) {
+    const uint32_t l = i >> shift, j = i & (M - 1);
+    if (j >= G) continue;
+    const int a = (int)(l < 3 ? l : l - 3);
     const uint32_t kp = S.k[l][j];
     const float p = unordf(kp);
     float cost = kInf, bound = kInf;
     if (!(j > 0 && S.k[l][j - 1] == kp)) {  // equal events score once
-      const Counts k = counts_at(a, kp);
-      if (in_limits(c, a, p)) cost = score32(P, c, a, p, k);
-      const uint32_t le_mn = upper(S.k[a], G, kp), le_mx = k.close + k.eq_max;
+      // the event is the first of its value in its own list: only the other
+      // list is searched
+      const uint32_t* const own = S.k[l];
+      const uint32_t* const other = S.k[l < 3 ? l + 3 : l - 3];
+      uint32_t own_le = j + 1;
+      while (own_le < G && own[own_le] == kp) ++own_le;
+      const uint32_t lt = lower(other, G, kp);
+      uint32_t le = lt;
+      while (le < G && other[le] == kp) ++le;
+      Counts k{l < 3 ? j : lt, l < 3 ? lt : j, 0u, 0u};
+      const uint32_t le_mn = l < 3 ? own_le : le, le_mx = l < 3 ? le : own_le;
+      k.eq_max = le_mx - k.close;
+      if (in_limits(c, a, p)) {
+        for (uint32_t i2 = 0; i2 < S.n_pl[a]; ++i2) k.planar += S.pl[a][i2] == kp ? 1u : 0u;
+        cost = score32(P, c, a, p, k);
+      }
       const uint32_t nmn = le_mn < G ? S.k[a][le_mn] : 0xFFFFFFFFu, nmx = le_mx < G ? S.k[3 + a][le_mx] : 0xFFFFFFFFu;
       const uint32_t kn = min(nmn, nmx);
       if (kn != 0xFFFFFFFFu) {
@@ -666,14 +715,22 @@ __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, cons
       }
     }
   };
+  // Candidates within the margin are gathered first and scored in FP64 side by
+  // side: the SM's two FP64 lanes take some 1100 cycles for one score, whether
+  // one thread of a warp or all of them ask for it.
+  auto gather = [&](int a, float p) {
+    const uint32_t at = atomicAdd(&S.n_cand, 1u);
+    if (at < (uint32_t)CAP) S.cand[at] = (uint64_t)a << 32 | ordf(p);
+  };
   // events and gaps that are not worse than the best by more than the margin
-  for (uint32_t i = tid; i < 6 * G; i += NT) {
-    const uint32_t l = i / G, j = i - l * G;
-    const int a = (int)(l % 3);
+  for (uint32_t i = tid; i < 6 * M; i += NT) {
+    const uint32_t l = i >> shift, j = i & (M - 1);
+    if (j >= G) continue;
+    const int a = (int)(l < 3 ? l : l - 3);
     const float cost = S.cost[l][j], bound = S.bound[l][j];
     if (!(cost > limit) && cost != kInf) {
       const uint32_t kp = S.k[l][j];
-      consider(a, unordf(kp), counts_at(a, kp));
+      gather(a, unordf(kp));
       if (kp == kZeroKey) {  // the edges at zero say which zero it is
         atomicMin(&S.hull_lo[a], kp);
         atomicMax(&S.hull_hi[a], kp);
@@ -690,21 +747,55 @@ __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, cons
   group_sync<NT>();
   // triangle edges inside the surviving gaps (interval ends among them: their
   // own bits decide between -0 and +0)
-  for (int a = 0; a < 3; ++a) {
-    const uint32_t hl = S.hull_lo[a], hh = S.hull_hi[a];
-    if (hl > hh) continue;
-    for (uint32_t t = t0 + tid; t < t1; t += NT) {
-      const float e[2] = {V.lo[a * V.cap + t], V.hi[a * V.cap + t]};
+  auto edges = [&](auto take) {
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t hl = S.hull_lo[a], hh = S.hull_hi[a];
+      if (hl > hh) continue;
+      for (uint32_t t = t0 + tid; t < t1; t += NT) {
+        const float e[2] = {V.lo[a * V.cap + t], V.hi[a * V.cap + t]};
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const float p = e[s];
-        const uint32_t kp = ordz(p);
-        if (kp < hl || kp > hh || !in_limits(c, a, p)) continue;
-        const Counts k = counts_at(a, kp);
-        if (score32(P, c, a, p, k) > limit) continue;
-        consider(a, p, k);
+        for (int s = 0; s < 2; ++s) {
+          const float p = e[s];
+          const uint32_t kp = ordz(p);
+          if (kp < hl || kp > hh || !in_limits(c, a, p)) continue;
+          const Counts k = counts_at(a, kp);
+          if (score32(P, c, a, p, k) > limit) continue;
+          take(a, p, k);
+        }
       }
     }
+  };
+  edges([&](int a, float p, const Counts&) { gather(a, p); });
+  group_sync<NT>();
+  const uint32_t m = S.n_cand;
+  if (m > 0u && m <= (uint32_t)CAP) {
+    const uint64_t c0 = S.cand[0];
+    const int a = (int)(c0 >> 32);
+    const float p = unordf((uint32_t)c0);
+    bool same = true;
+    for (uint32_t i = tid; i < m; i += NT) same = same && S.cand[i] == c0;
+    same = NT == 32 ? __all_sync(0xFFFFFFFFu, same) : __syncthreads_and(same);
+    const Counts k0 = counts_at(a, ordz(p));
+    if (same && k0.planar == 0 && (double)score32(P, c, a, p, k0) * (1.0 + kMargin) < init) {
+      // one position is left and it certainly beats the leaf: its cost decides
+      // nothing more, and without planar IDs both sides score the same
+      best_k = cand_key(a, p, 0);
+    } else {
+      for (uint32_t i = tid; i < m; i += NT) {
+        const uint64_t ci = S.cand[i];
+        const int ai = (int)(ci >> 32);
+        consider(ai, unordf((uint32_t)ci), counts_at(ai, ordz(unordf((uint32_t)ci))));
+      }
+    }
+  } else if (m > (uint32_t)CAP) {  // more than the list holds (no filter, or a flat node): each on the spot
+    for (uint32_t i = tid; i < 6 * M; i += NT) {
+      const uint32_t l = i >> shift, j = i & (M - 1);
+      if (j >= G) continue;
+      const int a = (int)(l < 3 ? l : l - 3);
+      const float cost = S.cost[l][j];
+      if (!(cost > limit) && cost != kInf) consider(a, unordf(S.k[l][j]), counts_at(a, S.k[l][j]));
+    }
+    edges(consider);
   }
   for (int o = 16; o > 0; o >>= 1) {
     const double oc = __shfl_xor_sync(0xFFFFFFFFu, best, o);
@@ -736,7 +827,7 @@ __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, cons
 constexpr int kSearchWarps = 4;
 __global__ void __launch_bounds__(32 * kSearchWarps)
     k_search_warp(Params P, uint32_t N, int level, const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb,
-                  const uint32_t* __restrict__ run_start, TriView V, const float* __restrict__ nlo,
+                  const uint32_t* __restrict__ ridx, TriView V, const float* __restrict__ nlo,
                   const float* __restrict__ nhi, Decision* dec, uint32_t* is_split) {
   __shared__ SearchMem<32, kWarpIds> S[kSearchWarps];
   const int w = threadIdx.x >> 5;
@@ -744,7 +835,7 @@ __global__ void __launch_bounds__(32 * kSearchWarps)
   if (n >= N || level >= P.max_level) return;
   const uint32_t r0 = rb[n], G = rb[n + 1] - r0;
   if (G <= kMinPrim || G > kWarpIds) return;
-  search_node<32, (int)kWarpIds>(S[w], threadIdx.x & 31, P, n, r0, G, tb[n], tb[n + 1], run_start, V, nlo, nhi, dec,
+  search_node<32, (int)kWarpIds>(S[w], threadIdx.x & 31, P, n, r0, G, tb[n], tb[n + 1], ridx, V, nlo, nhi, dec,
                                  is_split);
 }
 
@@ -753,13 +844,13 @@ template <int NT, int CAP>
 __global__ void __launch_bounds__(NT)
     k_search_block(Params P, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
                    const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb,
-                   const uint32_t* __restrict__ run_start, TriView V, const float* __restrict__ nlo,
+                   const uint32_t* __restrict__ ridx, TriView V, const float* __restrict__ nlo,
                    const float* __restrict__ nhi, Decision* dec, uint32_t* is_split) {
   extern __shared__ __align__(16) unsigned char raw[];
   SearchMem<NT, CAP>& S = *reinterpret_cast<SearchMem<NT, CAP>*>(raw);
   for (uint32_t i = blockIdx.x; i < *count; i += gridDim.x) {
     const uint32_t n = list[i], r0 = rb[n];
-    search_node<NT, CAP>(S, threadIdx.x, P, n, r0, rb[n + 1] - r0, tb[n], tb[n + 1], run_start, V, nlo, nhi, dec,
+    search_node<NT, CAP>(S, threadIdx.x, P, n, r0, rb[n + 1] - r0, tb[n], tb[n + 1], ridx, V, nlo, nhi, dec,
                          is_split);
     __syncthreads();
   }
@@ -824,10 +915,20 @@ __device__ __forceinline__ Counts big_counts(const Big& B, int a, uint32_t n, ui
 // State of a large node's search: best FP32 event (float bits; scores are
 // positive where the filter is on), best FP64 cost, its first candidate, and
 // per axis the hull of the surviving gaps.
+// The candidates scored in FP64 are listed (there are few within the margin),
+// so that choosing among those of equal cost does not score them again; only
+// when the list overflows (no FP32 filter) do the two scoring passes run twice.
+struct Scored {
+  unsigned long long cost, key;
+  uint32_t node;
+};
+constexpr uint32_t kScoredCap = 1u << 20;
 struct BigState {
   uint32_t* best32;
   unsigned long long *best64, *key;
   uint32_t *hull_lo, *hull_hi;
+  Scored* list;
+  uint32_t* n_list;
 };
 // order-preserving map of a double to unsigned
 __device__ __forceinline__ unsigned long long ordd(double d) {
@@ -896,19 +997,22 @@ __device__ __forceinline__ void big_consider(const Params& P, const Big& B, cons
   if (!(cst < init_cost(P, B.eGn[n], tb[n + 1] - tb[n]))) return;
   const unsigned long long o = ordd(cst);
   if (FIRST) {
-    if (o < st.best64[n]) atomicMin(&st.best64[n], o);
+    if (o > st.best64[n]) return;  // only ever decreases
+    atomicMin(&st.best64[n], o);
+    const uint32_t at = atomicAdd(st.n_list, 1u);
+    if (at < kScoredCap) st.list[at] = Scored{o, cand_key(a, p, side), n};
   } else if (o == st.best64[n]) {
     atomicMin(&st.key[n], (unsigned long long)cand_key(a, p, side));
   }
 }
 
-// Pass 2 (FIRST) and 4: events within the margin; pass 2 also gathers the
+// Pass 2 (FIRST; again if the list overflowed): events within the margin; pass 2 also gathers the
 // hull of the gaps whose bound is.
 template <bool FIRST>
 __global__ void k_event_exact(Params P, Big B, const uint32_t* __restrict__ tb, const float* __restrict__ nlo,
                               const float* __restrict__ nhi, const float2* __restrict__ scores, BigState st) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 6 * B.eG) return;
+  if (i >= 6 * B.eG || (!FIRST && *st.n_list <= kScoredCap)) return;
   const float kInf = __int_as_float(0x7f800000);
   const bool is_max = i >= 3 * B.eG;
   const uint64_t key = is_max ? B.kmax[i - 3 * B.eG] : B.kmin[i];
@@ -936,12 +1040,12 @@ __global__ void k_event_exact(Params P, Big B, const uint32_t* __restrict__ tb, 
   }
 }
 
-// Pass 3 (FIRST) and 5: triangle edges inside the hulls.
+// Pass 3 (FIRST; again if the list overflowed): triangle edges inside the hulls.
 template <bool FIRST>
 __global__ void k_edge_exact(Params P, Big B, TriView V, size_t T, const uint32_t* __restrict__ tb,
                              const float* __restrict__ nlo, const float* __restrict__ nhi, BigState st) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T) return;
+  if (t >= T || (!FIRST && *st.n_list <= kScoredCap)) return;
   const uint32_t n = V.node[t];
   if (B.eGn[n] == 0u) return;
   for (int a = 0; a < 3; ++a) {
@@ -972,6 +1076,16 @@ __global__ void k_big_init(const Params P, Big B, const uint32_t* __restrict__ t
   for (int a = 0; a < 3; ++a) {
     st.hull_lo[3ull * n + a] = 0xFFFFFFFFu;
     st.hull_hi[3ull * n + a] = 0u;
+  }
+}
+
+// First candidate of each node's smallest cost, from the list.
+__global__ void k_scored_first(BigState st) {
+  const uint32_t m = *st.n_list;
+  if (m > kScoredCap) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    const Scored c = st.list[i];
+    if (c.cost == st.best64[c.node]) atomicMin(&st.key[c.node], c.key);
   }
 }
 
@@ -1267,12 +1381,42 @@ __global__ void k_place(const Rec* __restrict__ rec, uint32_t N, const uint2* __
 
 template <int NT, int CAP>
 void launch_search_block(Stream& S, const Params& P, const uint32_t* list, const uint32_t* count, uint32_t most,
-                         const uint32_t* tb, const uint32_t* rb, const uint32_t* run_start, const TriView& V,
+                         const uint32_t* tb, const uint32_t* rb, const uint32_t* ridx, const TriView& V,
                          const float* nlo, const float* nhi, Decision* dec, uint32_t* is_split) {
   const int bytes = (int)sizeof(SearchMem<NT, CAP>);
   S.check(cudaFuncSetAttribute(k_search_block<NT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   const unsigned grid = std::max(1u, std::min(most, 4096u));
-  k_search_block<NT, CAP><<<grid, NT, bytes, S.s>>>(P, list, count, tb, rb, run_start, V, nlo, nhi, dec, is_split);
+  k_search_block<NT, CAP><<<grid, NT, bytes, S.s>>>(P, list, count, tb, rb, ridx, V, nlo, nhi, dec, is_split);
+}
+
+// Host threads of the steps around the build.  Reading 500k records for their
+// proxies took 6.0 ms on one thread and 1 ms on eight; the first touch of the
+// result's pages by the copy engine 2.4 ms for 40 MB against 0.8.
+constexpr uint32_t kHostThreads = 8;
+template <typename F>
+void host_parallel(uint32_t n, F fn) {
+  std::vector<std::thread> t;
+  t.reserve(n);
+  uint32_t r = 1;
+  try {
+    for (; r < n; ++r) t.emplace_back(fn, r);
+  } catch (const std::system_error&) {  // no more threads: the rest runs here
+  }
+  fn(0u);
+  for (uint32_t k = r; k < n; ++k) fn(k);
+  for (auto& x : t) x.join();
+}
+
+// malloc with the pages of a large array touched by several threads.
+void* host_array(size_t bytes) {
+  char* p = static_cast<char*>(malloc(bytes));
+  if (!p || bytes < (4u << 20)) return p;
+  const long page = std::max(4096l, sysconf(_SC_PAGESIZE));
+  host_parallel(kHostThreads, [=](uint32_t r) {
+    const size_t lo = bytes / kHostThreads * r, hi = r + 1 == kHostThreads ? bytes : bytes / kHostThreads * (r + 1);
+    for (size_t i = lo; i < hi; i += (size_t)page) reinterpret_cast<volatile char*>(p)[i] = 0;
+  });
+  return p;
 }
 
 }  // namespace
@@ -1294,23 +1438,35 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
   H.valid = calloc((size_t)n + 1, 1);
   if (!H.valid) throw std::bad_alloc();
   uint8_t* valid = static_cast<uint8_t*>(H.valid);
-  // per-Gaussian proxy scale on the host (the host builder's function)
-  std::vector<float> gv;
-  std::vector<float> kiso;
-  std::vector<uint32_t> ids;
-  gv.reserve((size_t)n * 10);
-  kiso.reserve(n);
-  ids.reserve(n);
-  for (uint32_t i = 0; i < n; ++i) {
-    const float* g = gauss + (size_t)i * 64;
-    float k;
-    if (!proxy_kiso(g, &k)) continue;
-    valid[i] = 1;
-    gv.insert(gv.end(), {g[0], g[1], g[2], g[4], g[5], g[6], g[8], g[9], g[10], g[11]});
-    kiso.push_back(k);
-    ids.push_back(i);
-  }
-  const uint32_t n_valid = (uint32_t)ids.size();
+  // per-Gaussian proxy scale on the host (the host builder's function), in
+  // ranges: the scales first, then each range's fields after those before it
+  std::vector<float> kall(n);
+  const uint32_t n_ranges = std::max(1u, std::min(kHostThreads, n / 16384u));
+  std::vector<uint32_t> first(n_ranges + 1, 0u);
+  auto range_lo = [&](uint32_t r) { return (uint32_t)((uint64_t)n * r / n_ranges); };
+  host_parallel(n_ranges, [&](uint32_t r) {
+    uint32_t c = 0;
+    for (uint32_t i = range_lo(r); i < range_lo(r + 1); ++i) {
+      valid[i] = proxy_kiso(gauss + (size_t)i * 64, &kall[i]) ? 1 : 0;
+      c += valid[i];
+    }
+    first[r + 1] = c;
+  });
+  for (uint32_t r = 0; r < n_ranges; ++r) first[r + 1] += first[r];
+  const uint32_t n_valid = first[n_ranges];
+  std::vector<float> gv((size_t)n_valid * 10), kiso(n_valid);
+  std::vector<uint32_t> ids(n_valid);
+  host_parallel(n_ranges, [&](uint32_t r) {
+    size_t j = first[r];
+    for (uint32_t i = range_lo(r); i < range_lo(r + 1); ++i) {
+      if (!valid[i]) continue;
+      const float* g = gauss + (size_t)i * 64;
+      const float f[10] = {g[0], g[1], g[2], g[4], g[5], g[6], g[8], g[9], g[10], g[11]};
+      memcpy(&gv[10 * j], f, sizeof f);
+      kiso[j] = kall[i];
+      ids[j++] = i;
+    }
+  });
   if (n_valid == 0) {
     err = "every Gaussian is below the opacity cut; nothing to build";
     return KDGR_ERR_INVALID_ARG;
@@ -1392,15 +1548,18 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
       }
       if (S.err != cudaSuccess) break;
       counts.zero();
-      k_node_setup<<<grid_for((size_t)N + 1, 128), 128, 0, S.s>>>(tb.p, ridx.p, N, level, P.max_level, rb.p, dec.p,
-                                                                  is_split.p, lists.p, lists.p + N, counts.p, eG.p);
-      k_search_warp<<<grid_for(N, kSearchWarps), 32 * kSearchWarps, 0, S.s>>>(P, N, level, tb.p, rb.p, run_start.p, V,
-                                                                              nlo.p, nhi.p, dec.p, is_split.p);
-      if (max_ids > kWarpIds)
-        launch_search_block<128, (int)kMidIds>(S, P, lists.p, counts.p, N, tb.p, rb.p, run_start.p, V, nlo.p, nhi.p,
-                                               dec.p, is_split.p);
+      const uint32_t warp_ids = N < kFewNodes ? 0u : kWarpIds;
+      k_node_setup<<<grid_for((size_t)N + 1, 128), 128, 0, S.s>>>(tb.p, ridx.p, N, level, P.max_level, warp_ids, rb.p,
+                                                                  dec.p, is_split.p, lists.p, lists.p + N, counts.p,
+                                                                  eG.p);
+      if (warp_ids)
+        k_search_warp<<<grid_for(N, kSearchWarps), 32 * kSearchWarps, 0, S.s>>>(
+            P, N, level, tb.p, rb.p, ridx.p, V, nlo.p, nhi.p, dec.p, is_split.p);
+      if (max_ids > std::max(warp_ids, kMinPrim))
+        launch_search_block<128, (int)kMidIds>(S, P, lists.p, counts.p, N, tb.p, rb.p, ridx.p, V, nlo.p, nhi.p, dec.p,
+                                               is_split.p);
       if (max_ids > kMidIds)
-        launch_search_block<512, (int)kBlockIds>(S, P, lists.p + N, counts.p + 1, N, tb.p, rb.p, run_start.p, V,
+        launch_search_block<512, (int)kBlockIds>(S, P, lists.p + N, counts.p + 1, N, tb.p, rb.p, ridx.p, V,
                                                  nlo.p, nhi.p, dec.p, is_split.p);
       if (may_be_big) {
         DBuf<uint32_t> grb(S, (size_t)N + 1);
@@ -1421,8 +1580,11 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
           DBuf<uint32_t> pl_fill(S, 1), best32(S, N), hull(S, 6 * (size_t)N);
           DBuf<unsigned long long> best64(S, 2 * (size_t)N);
           DBuf<float2> scores(S, 6 * (size_t)eGT);
+          DBuf<Scored> scored(S, kScoredCap);
+          DBuf<uint32_t> n_scored(S, 1);
           if (S.err != cudaSuccess) break;
           pl_fill.zero();
+          n_scored.zero();
           k_run_bounds<<<grid_for(T, 128), 128, 0, S.s>>>(run_start.p, run_node.p, rb.p, N, T, V, B, kmin.p, kmax.p,
                                                           kpl.p, pl_fill.p);
           S.check(cudaMemcpyAsync(&B.n_pl, pl_fill.p, 4, cudaMemcpyDeviceToHost, S.s));
@@ -1434,12 +1596,13 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
           B.kmin = kmin.p;
           B.kmax = kmax.p;
           B.kpl = kpl.p;
-          BigState st{best32.p, best64.p, best64.p + N, hull.p, hull.p + 3 * (size_t)N};
+          BigState st{best32.p, best64.p, best64.p + N, hull.p, hull.p + 3 * (size_t)N, scored.p, n_scored.p};
           const unsigned ge = grid_for(6 * (size_t)eGT, 256), gt = grid_for(T, 256), gn = grid_for(N, 128);
           k_big_init<<<gn, 128, 0, S.s>>>(P, B, tb.p, N, st);
           k_event_scores<<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
           k_event_exact<true><<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
           k_edge_exact<true><<<gt, 256, 0, S.s>>>(P, B, V, T, tb.p, nlo.p, nhi.p, st);
+          k_scored_first<<<256, 256, 0, S.s>>>(st);
           k_event_exact<false><<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
           k_edge_exact<false><<<gt, 256, 0, S.s>>>(P, B, V, T, tb.p, nlo.p, nhi.p, st);
           k_big_choose<<<gn, 128, 0, S.s>>>(B, N, st, dec.p, is_split.p);
@@ -1538,8 +1701,8 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
           at = std::move(next);
         }
         S.check(cudaGetLastError());
-        H.nodes = malloc(8ull * n_nodes + 4);
-        H.offsets = malloc(4 * pool_used + 4);
+        H.nodes = host_array(8ull * n_nodes + 4);
+        H.offsets = host_array(4 * pool_used + 4);
         if (H.nodes && H.offsets && S.err == cudaSuccess) {
           S.check(cudaMemcpyAsync(H.nodes, d_nodes.p, 8ull * n_nodes, cudaMemcpyDeviceToHost, S.s));
           if (pool_used)

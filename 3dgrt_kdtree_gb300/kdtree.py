@@ -30,15 +30,32 @@ class KdTree:
         return int(self.nodes.shape[0])
 
 
+class _Owner:
+    """Frees a library-owned tree when the last array over its memory goes."""
+
+    def __init__(self, t: capi.Tree):
+        self._t, self._free = t, capi.lib().kdgr_tree_free
+
+    def __del__(self):
+        self._free(ctypes.byref(self._t))
+
+
+def _array(owner: _Owner, ptr, ctype, n: int) -> np.ndarray:
+    """The library's array itself (no copy), keeping its owner alive."""
+    if n == 0:
+        return np.zeros(0, ctype)
+    buf = (ctype * n).from_address(ctypes.addressof(ptr.contents))
+    buf._owner = owner
+    return np.frombuffer(buf, dtype=ctype)
+
+
 def _take(t: capi.Tree) -> KdTree:
-    nodes = np.ctypeslib.as_array(t.nodes, shape=(t.n_nodes * 2,)).copy().reshape(t.n_nodes, 2)
-    offsets = (np.ctypeslib.as_array(t.offsets, shape=(t.n_offsets,)).copy() if t.n_offsets
-               else np.zeros(0, np.uint32))
-    valid = (np.ctypeslib.as_array(t.valid, shape=(t.n_gaussians,)).copy() if t.n_gaussians else None)
-    out = KdTree(nodes, offsets, np.array(list(t.aabb), np.float32), int(t.depth), int(t.n_leaves),
-                 int(t.max_leaf), valid)
-    capi.lib().kdgr_tree_free(ctypes.byref(t))
-    return out
+    own = _Owner(t)
+    nodes = _array(own, t.nodes, ctypes.c_uint32, t.n_nodes * 2).reshape(t.n_nodes, 2)
+    offsets = _array(own, t.offsets, ctypes.c_uint32, t.n_offsets)
+    valid = _array(own, t.valid, ctypes.c_uint8, t.n_gaussians) if t.n_gaussians else None
+    return KdTree(nodes, offsets, np.array(list(t.aabb), np.float32), int(t.depth), int(t.n_leaves),
+                  int(t.max_leaf), valid)
 
 
 def build(gaussians: np.ndarray, max_level: int = 24, force_split: int = 16, isect_cost: float = 5.0,
