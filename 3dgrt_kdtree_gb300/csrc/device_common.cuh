@@ -137,8 +137,13 @@ constexpr uint32_t kMaxRaySteps = 1u << 22;
 //   spheres: 10 floats each (center xyz, radius, material word, reflectivity,
 //            ior, color rgb); the material word is an int stored bitwise;
 //   tris:    9 floats each (three vertices), one material for all of them
-//            (tri_material: the 6 material floats, device pointer).
+//            (tri_material: the 6 material floats, device pointer);
+//   groups:  bounds of every kTriGroup consecutive triangles, then of every
+//            kTriGroup * kTriGroup (8 floats each: centre xyz, radius, margin
+//            factor, longest edge, 0, 0; see intersect_secondary).
+constexpr uint32_t kTriGroup = 8;
 struct HybridView {
+  const float* groups;
   const float* spheres;
   const float* tris;
   const float* tri_material;
@@ -146,8 +151,9 @@ struct HybridView {
   uint32_t n_tris;
 };
 
-cudaError_t launch_hybrid(const ExactView& s, const CamInfo& cam, int width, int height, const HybridView& m,
-                          float* rgb, uint32_t* status, cudaStream_t stream);
+// The walk over `plain` when it is materialised, over `s` otherwise.
+cudaError_t launch_hybrid(const ExactView& s, const PlainView& plain, const CamInfo& cam, int width, int height,
+                          const HybridView& m, float* rgb, uint32_t* status, cudaStream_t stream);
 
 // Plain render; the packet walk over `plain` when it is materialised and no
 // trace is asked for, one thread per ray over `s` otherwise.

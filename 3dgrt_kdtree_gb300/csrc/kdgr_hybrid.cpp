@@ -5,10 +5,12 @@
 // loadSecondaryMesh, Kd-treeConverterMain.cpp:179-221).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -21,6 +23,7 @@ using namespace kdgr;
 struct kdgr_secondary_s {
   float* d_spheres = nullptr;
   float* d_tris = nullptr;
+  float* d_groups = nullptr;
   float* d_tri_material = nullptr;
   int n_spheres = 0;
   uint32_t n_tris = 0;
@@ -49,6 +52,46 @@ bool obj_index(const char* tok, long n_pos, long* out) {
   if (k < 0 || k >= n_pos) return false;
   *out = k;
   return true;
+}
+
+// Bounds of every kTriGroup consecutive triangles, then of every kTriGroup
+// groups (HybridView::groups): a sphere around the vertices, the longest edge
+// E, and the factor 0.33 E^2 of the margin that makes the sphere test
+// conservative against the triangle test's rounding (infinite, never skipped,
+// for edges so long that the bound behind it does not hold).
+std::vector<float> tri_groups(const float* verts, uint32_t n_tris) {
+  std::vector<float> out;
+  for (uint32_t per : {kTriGroup, kTriGroup * kTriGroup})
+    for (uint32_t first = 0; first < n_tris; first += per) {
+      const uint32_t end = std::min(n_tris, first + per);
+      double lo[3], hi[3], r2 = 0.0, e2 = 0.0;
+      for (int d = 0; d < 3; ++d) lo[d] = hi[d] = verts[9ull * first + d];
+      for (size_t k = 3ull * first; k < 3ull * end; ++k)
+        for (int d = 0; d < 3; ++d) {
+          lo[d] = std::min(lo[d], (double)verts[3 * k + d]);
+          hi[d] = std::max(hi[d], (double)verts[3 * k + d]);
+        }
+      const float c[3] = {(float)(0.5 * (lo[0] + hi[0])), (float)(0.5 * (lo[1] + hi[1])), (float)(0.5 * (lo[2] + hi[2]))};
+      bool finite = true;
+      for (size_t k = 3ull * first; k < 3ull * end; ++k) {
+        const float* v = verts + 3 * k;
+        const float* w = verts + 3 * (k % 3 == 2 ? k - 2 : k + 1);
+        double r = 0.0, e = 0.0;
+        for (int d = 0; d < 3; ++d) {
+          r += ((double)v[d] - c[d]) * ((double)v[d] - c[d]);
+          e += ((double)v[d] - w[d]) * ((double)v[d] - w[d]);
+        }
+        finite = finite && std::isfinite(r) && std::isfinite(e);
+        r2 = std::max(r2, r);
+        e2 = std::max(e2, e);
+      }
+      const double E = std::sqrt(e2) * 1.0001;
+      const float inf = std::numeric_limits<float>::infinity();
+      const bool covered = finite && E <= 3.4;
+      out.insert(out.end(), {c[0], c[1], c[2], covered ? (float)(std::sqrt(r2) * 1.0001) : inf,
+                             covered ? (float)(0.33 * E * E) : inf, covered ? (float)E : 0.f, 0.f, 0.f});
+    }
+  return out;
 }
 
 }  // namespace
@@ -183,11 +226,17 @@ int kdgr_secondary_create(const kdgr_sphere* spheres, int n_spheres, const float
     e = cudaMalloc(&s->d_tris, 36ull * n_tris);
     if (e == cudaSuccess) e = cudaMemcpy(s->d_tris, tri_verts, 36ull * n_tris, cudaMemcpyHostToDevice);
   }
+  if (e == cudaSuccess && n_tris > 0) {
+    const std::vector<float> groups = tri_groups(tri_verts, n_tris);
+    e = cudaMalloc(&s->d_groups, groups.size() * 4);
+    if (e == cudaSuccess) e = cudaMemcpy(s->d_groups, groups.data(), groups.size() * 4, cudaMemcpyHostToDevice);
+  }
   if (e == cudaSuccess) e = cudaMalloc(&s->d_tri_material, sizeof tm);
   if (e == cudaSuccess) e = cudaMemcpy(s->d_tri_material, tm, sizeof tm, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(s->d_spheres);
     cudaFree(s->d_tris);
+    cudaFree(s->d_groups);
     cudaFree(s->d_tri_material);
     delete s;
     return cuda_fail(e, "kdgr_secondary_create");
@@ -200,6 +249,7 @@ int kdgr_secondary_destroy(kdgr_secondary_t s) {
   if (!s) return KDGR_OK;
   cudaFree(s->d_spheres);
   cudaFree(s->d_tris);
+  cudaFree(s->d_groups);
   cudaFree(s->d_tri_material);
   delete s;
   return KDGR_OK;
@@ -219,14 +269,14 @@ int kdgr_render_hybrid(kdgr_scene_t s, const kdgr_camera* cam, int W, int H, kdg
   if (on.err != cudaSuccess) return cuda_fail(on.err, "kdgr_render_hybrid");
   const cudaStream_t st = (cudaStream_t)stream;
   const CamInfo ci = make_caminfo(*cam, W, H);
-  HybridView m{sec->d_spheres, sec->d_tris, sec->d_tri_material, sec->n_spheres, sec->n_tris};
+  HybridView m{sec->d_groups, sec->d_spheres, sec->d_tris, sec->d_tri_material, sec->n_spheres, sec->n_tris};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ms_out) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
   }
-  cudaError_t e = launch_hybrid(s->exact_view(), ci, W, H, m, rgb, s->d_status, st);
+  cudaError_t e = launch_hybrid(s->exact_view(), s->plain_view(), ci, W, H, m, rgb, s->d_status, st);
   if (e == cudaSuccess && ms_out) {
     cudaEventRecord(e1, st);
     e = cudaEventSynchronize(e1);

@@ -342,7 +342,26 @@ __device__ __forceinline__ void sec_set_normal(SecHit& h, const F3 d, F3 n) {
   }
 }
 
-__device__ SecHit intersect_secondary(const HybridView& M, const F3 o, const F3 d) {
+// Whether a group of triangles may be hit: the line (o, d) passes its sphere
+// within a margin.  A triangle test accepts barycentrics in [0, 1] up to its
+// rounding, which dividing by |a| >= 1e-5 magnifies: with edges E <= 3.4 and
+// s = o - v0 they are off by at most 0.11 E (E + |s|), so a line that the test
+// accepts passes the triangle within 3 E times that.
+__device__ __forceinline__ bool near_group(const float* __restrict__ g, const F3 o, const F3 d) {
+  const float4 c = __ldg(reinterpret_cast<const float4*>(g));
+  const float2 e = __ldg(reinterpret_cast<const float2*>(g + 4));  // margin factor, longest edge
+  const F3 oc = mk(o.x - c.x, o.y - c.y, o.z - c.z);
+  const F3 x = mk(oc.y * d.z - oc.z * d.y, oc.z * d.x - oc.x * d.z, oc.x * d.y - oc.y * d.x);
+  const float oc2 = oc.x * oc.x + oc.y * oc.y + oc.z * oc.z;
+  const float r = c.w + e.x * (e.y + c.w + sqrtf(oc2));
+  return !(x.x * x.x + x.y * x.y + x.z * x.z > 1.001f * r * r + 1e-5f * oc2);
+}
+
+// Closest secondary primitive of every active lane's ray; the warp calls it
+// together and skips the groups of triangles that none of its rays comes near
+// (of 320 triangles of a mirror ball, most tiles of a 720p frame test none:
+// 11k of 55k warp instructions per tile before).
+__device__ __forceinline__ SecHit intersect_secondary(const HybridView& M, const F3 o, const F3 d, bool active) {
   SecHit h;
   h.hit = false;
   h.t = 1e8f;
@@ -367,55 +386,115 @@ __device__ SecHit intersect_secondary(const HybridView& M, const F3 o, const F3 
       }
     }
   }
-  for (uint32_t i = 0; i < M.n_tris; ++i) {
-    const float* v = M.tris + 9ull * i;
-    const F3 v0 = mk(v[0], v[1], v[2]), v1 = mk(v[3], v[4], v[5]), v2 = mk(v[6], v[7], v[8]);
-    const F3 e1 = sub(v1, v0), e2 = sub(v2, v0);
-    const F3 hv = cross(d, e2);
-    const float a = dot(e1, hv);
-    if (a > -kEps && a < kEps) continue;
-    const float f = fd(1.0f, a);
-    const F3 sv = sub(o, v0);
-    const float u = fm(f, dot(sv, hv));
-    if (u < 0.0f || u > 1.0f) continue;
-    const F3 q = cross(sv, e1);
-    const float vv = fm(f, dot(d, q));
-    if (vv < 0.0f || fa(u, vv) > 1.0f) continue;
-    const float t = fm(f, dot(e2, q));
-    if (!(t > kEps)) continue;
-    if (t < h.t) {
-      h.hit = true;
-      h.t = t;
-      h.p = add(o, muls(d, t));
-      sec_set_normal(h, d, normalize3(cross(sub(v1, v0), sub(v2, v0))));
-      sec_material(h, M.tri_material);
+  constexpr uint32_t kSuper = kTriGroup * kTriGroup;
+  const uint32_t n_groups = (M.n_tris + kTriGroup - 1) / kTriGroup;
+  for (uint32_t first = 0; first < M.n_tris; first += kTriGroup) {
+    if (first % kSuper == 0 &&
+        !__any_sync(0xFFFFFFFFu, active && near_group(M.groups + 8ull * (n_groups + first / kSuper), o, d))) {
+      first += kSuper - kTriGroup;
+      continue;
     }
+    if (!__any_sync(0xFFFFFFFFu, active && near_group(M.groups + 8ull * (first / kTriGroup), o, d))) continue;
+    for (uint32_t i = first; i < min(first + kTriGroup, M.n_tris); ++i) {
+      const float* v = M.tris + 9ull * i;
+      const F3 v0 = mk(v[0], v[1], v[2]), v1 = mk(v[3], v[4], v[5]), v2 = mk(v[6], v[7], v[8]);
+      const F3 e1 = sub(v1, v0), e2 = sub(v2, v0);
+      const F3 hv = cross(d, e2);
+      const float a = dot(e1, hv);
+      if (a > -kEps && a < kEps) continue;
+      const float f = fd(1.0f, a);
+      const F3 sv = sub(o, v0);
+      const float u = fm(f, dot(sv, hv));
+      if (u < 0.0f || u > 1.0f) continue;
+      const F3 q = cross(sv, e1);
+      const float vv = fm(f, dot(d, q));
+      if (vv < 0.0f || fa(u, vv) > 1.0f) continue;
+      const float t = fm(f, dot(e2, q));
+      if (!(t > kEps)) continue;
+      if (t < h.t) {
+        h.hit = true;
+        h.t = t;
+        h.p = add(o, muls(d, t));
+        sec_set_normal(h, d, normalize3(cross(sub(v1, v0), sub(v2, v0))));
+        sec_material(h, M.tri_material);
+      }
+    }
+    __syncwarp();
   }
   return h;
 }
 
-template <int K>
-__global__ void __launch_bounds__(kBlock) k_render_hybrid(ExactView S, CamInfo C, int W, int H, HybridView M,
-                                                          float* __restrict__ rgb, uint32_t* status) {
+// WALK: how the Gaussian passes run -- 0: one thread per ray over the tree as
+// given; 1: independent rays over the leaf-order pairs; 2: the primary rays as
+// packets, bounced ones independently.  A warp's lanes stay together through
+// the bounces; a lane whose ray has ended only waits.  What a pass does not
+// need (the running colour, throughput and the hit) waits in shared memory
+// meanwhile: in registers it spilled 600 bytes around the walk.
+template <int WALK>
+__global__ void __launch_bounds__(kBlock, WALK == 0 ? 0 : 6)
+    k_render_hybrid(ExactView S, PlainView L, CamInfo C, int W, int H, HybridView M, float* __restrict__ rgb,
+                    uint32_t* status) {
   __shared__ uint32_t s_id[kStack][kBlock];
   __shared__ float s_t[kStack][kBlock];
   const int tid = threadIdx.x;
   int x, y;
   thread_pixel(tid, &x, &y);
-  if (x >= W || y >= H) return;
+  const bool inimg = x < W && y < H;
   F3 o = mk(C.eye[0], C.eye[1], C.eye[2]);
-  F3 d = primary_dir(C, x, y);
+  F3 d = primary_dir(C, inimg ? x : 0, inimg ? y : 0);
   F3 fin = mk(0.f, 0.f, 0.f), thr = mk(1.f, 1.f, 1.f), acc = mk(0.f, 0.f, 0.f);
-  float A = 0.f, D = 0.f;
-  RayStats rs;
+  constexpr int kKeep = sizeof(SecHit) / 4 + 6;
+  static_assert(sizeof(SecHit) % 4 == 0, "SecHit is kept as words");
+  __shared__ uint32_t s_keep[WALK == 0 ? 1 : kKeep][kBlock];
+  Ray R;  // its opacity, and colour and depth in acc_slot(), carry over between bounces
+  R.A = 0.f;
+  float D = 0.f;
+  if constexpr (WALK != 0) *acc_slot() = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool active = inimg;
   for (int bounce = 0; bounce < 5; ++bounce) {
-    const SecHit h = intersect_secondary(M, o, d);
+    if (!__any_sync(0xFFFFFFFFu, active)) break;
+    SecHit h = intersect_secondary(M, o, d, active);
     const float max_t = h.hit ? h.t : 1e8f;
-    if (!trace_exact<K, false>(S, o, d, max_t, acc, A, D, rs, s_id, s_t, tid, status)) break;
+    if constexpr (WALK == 0) {
+      RayStats rs;
+      if (active && !trace_exact<8, false>(S, o, d, max_t, acc, R.A, D, rs, s_id, s_t, tid, status)) active = false;
+    } else {
+      const bool live = active && ray_init_plain(L, o, d, max_t, R) && R.A < 0.99f;
+      uint32_t keep[kKeep];
+      memcpy(keep, &h, sizeof h);
+      memcpy(keep + sizeof(h) / 4, &fin, 12);
+      memcpy(keep + sizeof(h) / 4 + 3, &thr, 12);
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k) s_keep[k][tid] = keep[k];
+      if (WALK == 2 && bounce == 0) {
+        __shared__ PktEnt s_ent[kStack][kWarps];
+        trace_packets<kHits, kFormPlain, 1>(L, R, live, sign_bits(d), s_id, s_t, s_ent, tid, status);
+      } else if (live) {
+        R.cur = R.steps = 0;
+        R.top = kStack - 1;
+        R.quant = 0;
+        while (R.A < 0.99f && !leaf_step<kHits, kFormPlain, 1>(L, s_id, s_t, tid, R, status)) {
+        }
+      }
+      __syncwarp();
+      const float4 v = *acc_slot();
+      acc = mk(v.x, v.y, v.z);
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k) keep[k] = *(volatile uint32_t*)&s_keep[k][tid];
+      memcpy(&h, keep, sizeof h);
+      memcpy(&fin, keep + sizeof(h) / 4, 12);
+      memcpy(&thr, keep + sizeof(h) / 4 + 3, 12);
+      o = R.o;
+      d = R.d;
+    }
+    if (!active) continue;
+    const float A = R.A;
     fin = add(fin, mulv(thr, acc));
     thr = muls(thr, fs(1.0f, A));
-    if (thr.x < 0.01f && thr.y < 0.01f && thr.z < 0.01f) break;
-    if (!h.hit) break;
+    if ((thr.x < 0.01f && thr.y < 0.01f && thr.z < 0.01f) || !h.hit) {
+      active = false;
+      continue;
+    }
     const F3 N = h.n, I = d;
     if (h.mat == 1) {  // mirror
       const F3 rdir = sub(I, muls(muls(N, 2.0f), dot(I, N)));
@@ -441,9 +520,10 @@ __global__ void __launch_bounds__(kBlock) k_render_hybrid(ExactView S, CamInfo C
       thr = mulv(thr, h.color);
     } else {  // opaque
       fin = add(fin, mulv(thr, h.color));
-      break;
+      active = false;
     }
   }
+  if (!inimg) return;
   const size_t idx = (size_t)(H - 1 - y) * W + x;
   rgb[3 * idx] = fminf(fin.x, 1.0f);
   rgb[3 * idx + 1] = fminf(fin.y, 1.0f);
@@ -498,10 +578,21 @@ cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamIn
   return cudaGetLastError();
 }
 
-cudaError_t launch_hybrid(const ExactView& s, const CamInfo& cam, int W, int H, const HybridView& m, float* rgb,
-                          uint32_t* status, cudaStream_t st) {
-  dim3 grid((W + 15) / 16, (H + 7) / 8);
-  k_render_hybrid<8><<<grid, kBlock, 0, st>>>(s, cam, W, H, m, rgb, status);
+cudaError_t launch_hybrid(const ExactView& s, const PlainView& plain, const CamInfo& cam, int W, int H,
+                          const HybridView& m, float* rgb, uint32_t* status, cudaStream_t st) {
+  // The walk as in launch_exact; lanes are not shared here (bounced rays part).
+  // us with 320 triangles, 100k / 10k Gaussians, one thread per ray first:
+  // 256x256 765 / 731, own walk 657 / 599; 1280x720 2352 / 1203, packets
+  // 1277 / 967 (own walk 1532 / 933); without groups of triangles to skip the
+  // 1280x720 frame took 3400.
+  const dim3 grid((W + 15) / 16, (H + 7) / 8);
+  const bool leaf = plain.leaf_tol && !(s.n_offsets / 64u > s.n_gauss);
+  if (!leaf)
+    k_render_hybrid<0><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
+  else if ((uint64_t)W * H < 300000)
+    k_render_hybrid<1><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
+  else
+    k_render_hybrid<2><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
   return cudaGetLastError();
 }
 
