@@ -105,7 +105,7 @@ struct ViewDesc {
   uint32_t cb_x, cb_base;  // 16x8 blocks per row; first global block
   uint64_t out_off;
   uint32_t scene;          // scene slot (multi-scene launches of the serving loop)
-  uint32_t pad;
+  uint32_t grp_base;       // first group of blocks of the view (groups schedule)
 };
 
 __host__ __device__ inline uint64_t fnv_add(uint64_t h, uint32_t v) {

@@ -224,11 +224,11 @@ void kdgr_server_s::scheduler() {
         d.cb_base = (uint32_t)cbase;
         d.out_off = (r->direct ? 0 : r->dev_off) + v.out_offset;
         d.scene = (uint32_t)r->slot;
-        d.pad = 0;
         cbase += (uint64_t)d.cb_x * (uint64_t)((v.height + 7) / 8);
       }
       ++slots[r->slot].inflight;
     }
+    const uint32_t groups = number_groups(L.h_views, (int)k, 4 * cbase);
     const Clock::time_point now = Clock::now();
     for (Request* r : admitted) r->t_launch = now;
     L.busy = true;
@@ -242,7 +242,7 @@ void kdgr_server_s::scheduler() {
     cudaError_t e = cudaMemcpyAsync(L.d_views, L.h_views, k * kTableEntry, cudaMemcpyHostToDevice, L.st);
     if (e == cudaSuccess) e = cudaMemsetAsync(L.d_queue, 0, kQueueBytes, L.st);
     if (e == cudaSuccess)
-      e = launch_multi(tbl, packed, L.d_views, (int)k, (uint32_t)cbase,
+      e = launch_multi(tbl, packed, L.d_views, (int)k, (uint32_t)cbase, groups,
                        reinterpret_cast<float* const*>(L.d_views + k), L.d_queue, d_status, L.st);
     if (e == cudaSuccess) e = cudaEventRecord(L.ev, L.st);
     lk.lock();

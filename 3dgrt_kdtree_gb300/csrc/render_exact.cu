@@ -206,8 +206,8 @@ __device__ __forceinline__ bool trace_exact(const ExactView& S, const F3 o, cons
 // Pixel of thread `tid` in a 16x8 block: warps cover 8x4 tiles.
 __device__ __forceinline__ void thread_pixel(int tid, int* x, int* y) {
   const int lane = tid & 31, warp = tid >> 5;
-  *x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-  *y = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
+  *x = (int)middle_out(blockIdx.x, gridDim.x) * 16 + (warp & 1) * 8 + (lane & 7);
+  *y = (int)middle_out(blockIdx.y, gridDim.y) * 8 + (warp >> 1) * 4 + (lane >> 3);
 }
 
 // Ray generation (cudaRenderer.cu:2336-2339): direction through the pixel
@@ -238,8 +238,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_render_plain(PlainView S, Ca
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t it = blockIdx.x * kWarps + warp;
   if (it >= n_items) return;
-  const uint32_t blk = it / (4u * LPR), q = it % (4u * LPR), nx = (uint32_t)((W + kBlockW - 1) / kBlockW);
-  const int bx = (int)(blk % nx) * kBlockW, by = (int)(blk / nx) * kBlockH;
+  const uint32_t blk = it / (4u * LPR), q = it % (4u * LPR), nx = (uint32_t)((W + kBlockW - 1) / kBlockW),
+                 ny = (uint32_t)((H + kBlockH - 1) / kBlockH);
+  const int bx = (int)middle_out(blk % nx, nx) * kBlockW, by = (int)middle_out(blk / nx, ny) * kBlockH;
   int x, y;
   if constexpr (LPR == 1) block_pixel(KDGR_TILE_8X4, bx, by, (int)q, lane, x, y);
   else group_pixel<LPR>(bx, by, (int)q, lane, x, y);

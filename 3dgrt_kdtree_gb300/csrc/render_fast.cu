@@ -87,18 +87,14 @@ __device__ __forceinline__ uint32_t strip_lo(uint32_t total, uint32_t n, uint32_
 // may be exhausted by the time the caller claims from it; the caller then
 // asks again, and since a counter only grows, every failed claim closes a
 // strip for good.
-__device__ __forceinline__ uint32_t next_open_strip(const uint32_t* queue, uint32_t total, uint32_t n, uint32_t k,
-                                                    unsigned lane) {
+template <typename Open>
+__device__ __forceinline__ uint32_t next_open(uint32_t n, uint32_t k, unsigned lane, Open is_open) {
   constexpr int kRounds = (kMaxStrips + 31) / 32;
   bool open[kRounds];
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
     const uint32_t off = 1u + 32u * r + lane;  // off == n is k itself
-    open[r] = false;
-    if (off <= n) {
-      const uint32_t j = (k + off) % n;
-      open[r] = __ldcg(queue + 1 + j) < strip_lo(total, n, j + 1) - strip_lo(total, n, j);
-    }
+    open[r] = off <= n && is_open((k + off) % n);
   }
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
@@ -107,6 +103,71 @@ __device__ __forceinline__ uint32_t next_open_strip(const uint32_t* queue, uint3
   }
   return n;
 }
+__device__ __forceinline__ uint32_t next_open_strip(const uint32_t* queue, uint32_t total, uint32_t n, uint32_t k,
+                                                    unsigned lane) {
+  return next_open(n, k, lane, [&](uint32_t j) {
+    return __ldcg(queue + 1 + j) < strip_lo(total, n, j + 1) - strip_lo(total, n, j);
+  });
+}
+
+// Groups schedule (default configurations; no public value): blocks in groups
+// of 2x1 to 2x4, a view's groups numbered by rows and columns from its middle
+// outwards and dealt to the SMs in turn, warps claiming quarter blocks of
+// their SM's next group and then of the following SMs'.  Against one
+// contiguous strip of the block list per SM: every SM gets its share of the
+// expensive middle, the packets that start last are the short ones at the
+// border, and an SM's resident warps share a squarer piece of the image.  us
+// on a GB300, strips first: 640x480 of 100k Gaussians 628 -> 544, 1080p of 1M
+// 1768 -> 1693, 16 mixed views of 300k 10991 -> 10416, packed 4x1080p 7085 ->
+// 6926; smaller groups balance small launches better, larger ones share more
+// of the L1 (640x480: 2x1 541, 2x2 574, 2x4 592; mixed: 10582, 10453, 10393).
+struct GroupShape {
+  uint32_t lx, ly;  // blocks of a group, as powers of two
+};
+GroupShape group_shape(uint64_t tiles) {  // by the launch's 8x4 tiles
+  return tiles < 16384u ? GroupShape{1, 0} : tiles < 131072u ? GroupShape{1, 1} : GroupShape{1, 2};
+}
+// `chunk` argument of a groups launch: SMs, lx, ly.
+int group_arg(int sms, GroupShape g) { return sms | (int)(g.lx << 16 | g.ly << 20); }
+
+// A warp's place in the dealt groups.
+struct GroupWalk {
+  uint32_t n, lx, ly, groups, per;  // SMs, group shape, groups of the launch, items of a group
+  uint32_t k, fails;                // whose groups the warp claims from; exhausted ones it has met
+  __device__ __forceinline__ GroupWalk(int arg, uint32_t total, uint32_t items_per_block)
+      : n((uint32_t)arg & 0xFFFFu), lx(((uint32_t)arg >> 16) & 15u), ly((uint32_t)arg >> 20), groups(total),
+        per(items_per_block << (lx + ly)), fails(0) {
+    uint32_t smid;
+    asm("mov.u32 %0, %%smid;" : "=r"(smid));
+    k = smid % n;
+  }
+  __device__ __forceinline__ uint32_t items(uint32_t j) const { return j < groups ? (groups - j + n - 1) / n * per : 0u; }
+  // The warp's next item: its group and its number inside; false when every
+  // group is taken.  queue word 1 + j counts the claims from SM j's groups; an
+  // exhausted SM is followed by the first with items left, as next_open_strip.
+  __device__ __forceinline__ bool next(uint32_t* queue, unsigned lane, uint32_t& group, uint32_t& sub) {
+    while (fails <= n) {
+      uint32_t c = 0;
+      if (lane == 0) c = atomicAdd(queue + 1 + k, 1u);
+      c = __shfl_sync(0xFFFFFFFFu, c, 0);
+      if (c < items(k)) {
+        group = c / per * n + k;
+        sub = c % per;
+        return true;
+      }
+      ++fails;
+      k = next_open(n, k, lane, [&](uint32_t j) { return __ldcg(queue + 1 + j) < items(j); });
+      if (k >= n) return false;
+    }
+    return false;
+  }
+  // Top-left pixel of block `b` of group `lg` of a W x H view.
+  __device__ __forceinline__ void block(uint32_t lg, uint32_t b, int W, int H, int& bx, int& by) const {
+    const uint32_t gx = ((uint32_t)W + (16u << lx) - 1) >> (4 + lx), gy = ((uint32_t)H + (8u << ly) - 1) >> (3 + ly);
+    bx = (int)(middle_out(lg % gx, gx) << (4 + lx)) + (int)(b & ((1u << lx) - 1u)) * kBlockW;
+    by = (int)(middle_out(lg / gx, gy) << (3 + ly)) + (int)(b >> lx) * kBlockH;
+  }
+};
 
 template <bool PACKED, int SCHED, int MINB, int KB, bool PKT, int LPR>
 __global__ void __launch_bounds__(kThreads, MINB) k_render_batch(FastView S, const ViewDesc* __restrict__ views,
@@ -120,7 +181,22 @@ __global__ void __launch_bounds__(kThreads, MINB) k_render_batch(FastView S, con
   __shared__ PktEnt s_ent[kStack][kWarps];
   __shared__ uint32_t s_work;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if constexpr (SCHED == KDGR_SCHED_WARP_STRIPS) {
+  if constexpr (SCHED == kSchedGroups) {
+    GroupWalk G(chunk, total_items, 4u * LPR);
+    uint32_t g, sub;
+    while (G.next(queue, (unsigned)lane, g, sub)) {
+      const ViewDesc& V = views[find_view(views, n_views, g, kSchedGroups)];
+      const int W = __ldg(&V.W), H = __ldg(&V.H);
+      int bx, by, x, y;
+      G.block(g - __ldg(&V.grp_base), sub / (4u * LPR), W, H, bx, by);
+      if (bx >= W || by >= H) continue;  // a group's blocks beyond the image
+      const int q = (int)(sub % (4u * LPR));
+      if constexpr (LPR == 1) block_pixel(tile, bx, by, q, lane, x, y);
+      else group_pixel<LPR>(bx, by, q, lane, x, y);
+      render_px<KB, PACKED ? kFormPacked : kFormFp32, PKT, LPR>(S, V, x, y, s_id, s_t, s_ent, tid, rgb, alpha_out,
+                                                                depth_out, status);
+    }
+  } else if constexpr (SCHED == KDGR_SCHED_WARP_STRIPS) {
     // items are quarters of 16x8 blocks (warp tiles in block order), or with
     // LPR lanes per ray 4 LPR tiles of 32 / LPR rays; each warp claims the
     // next item of its SM's strip, no CTA barrier
@@ -219,50 +295,64 @@ __global__ void __launch_bounds__(kThreads, MINB) k_render_batch(FastView S, con
   }
 }
 
-// Multi-scene form of the warp-strip schedule for the serving loop: every
-// view names a scene slot and each warp renders its quarter-block against
-// that slot's arrays (the slot table travels in the launch parameters, so
-// the warp-uniform field reads hit the constant cache).  One persistent launch
-// serves the requests of all resident scenes queued in a tick.  Items are
-// quarters of 16x8 blocks; queue word 1 + k counts the claims of strip k.
-// outs[v] is view v's output base (the device arena, or a request's
-// page-locked host buffer); the view's out_off counts pixels from it.
-// PKT, LPR: the walk, as in k_render_batch.
+// Multi-scene form for the serving loop: every view names a scene slot and
+// each warp renders its quarter-block against that slot's arrays (the slot
+// table travels in the launch parameters, so the warp-uniform field reads hit
+// the constant cache).  One persistent launch serves the requests of all
+// resident scenes queued in a tick.  outs[v] is view v's output base (the
+// device arena, or a request's page-locked host buffer); the view's out_off
+// counts pixels from it.  PKT, LPR: the walk, as in k_render_batch; items are
+// dealt by groups, or with lanes sharing rays taken from warp strips (`share`
+// and `total` as the schedules' chunk and total_items).
 template <bool PACKED, int MINB, bool PKT, int LPR>
 __global__ void __launch_bounds__(kThreads, MINB) k_render_multi(const __grid_constant__ SceneTable scenes,
                                                               const ViewDesc* __restrict__ views, int n_views,
-                                                              uint32_t total_items, float* const* __restrict__ outs,
-                                                              uint32_t* queue, uint32_t* status, int n_strips) {
+                                                              uint32_t total, float* const* __restrict__ outs,
+                                                              uint32_t* queue, uint32_t* status, int share) {
   __shared__ uint32_t s_id[kStack][kThreads];
   __shared__ float s_t[kStack][kThreads];
   __shared__ PktEnt s_ent[kStack][kWarps];
   const int tid = threadIdx.x, lane = tid & 31;
-  uint32_t smid;
-  asm("mov.u32 %0, %%smid;" : "=r"(smid));
-  const uint32_t n = (uint32_t)n_strips;
-  uint32_t k = smid % n, fails = 0;
-  while (fails <= n) {  // a warp's claims fail at most once per strip
-    const uint32_t b0 = strip_lo(total_items, n, k), b1 = strip_lo(total_items, n, k + 1);
-    uint32_t it = 0;
-    if (lane == 0) it = b0 + atomicAdd(queue + 1 + k, 1u);
-    it = __shfl_sync(0xFFFFFFFFu, it, 0);
-    if (it >= b1) {
-      ++fails;
-      k = next_open_strip(queue, total_items, n, k, (unsigned)lane);
-      if (k >= n) break;
-      continue;
-    }
-    const uint32_t blk = it / (4u * LPR), q = it % (4u * LPR);
-    const int vi = find_view(views, n_views, blk, KDGR_SCHED_CTA_BLOCKS);
+  auto render = [&](int vi, int bx, int by, int q) {
     const ViewDesc& V = views[vi];
     const FastView& S = scenes.s[__ldg(&V.scene) & (kSceneSlots - 1)];
-    float* const rgb = outs[vi];
-    const uint32_t lb = blk - __ldg(&V.cb_base), nx = __ldg(&V.cb_x);
     int x, y;
-    const int bx = (int)(lb % nx) * kBlockW, by = (int)(lb / nx) * kBlockH;
-    if constexpr (LPR == 1) block_pixel(KDGR_TILE_8X4, bx, by, (int)q, lane, x, y);
-    else group_pixel<LPR>(bx, by, (int)q, lane, x, y);
-    render_px<kHits, PACKED ? kFormPacked : kFormFp32, PKT, LPR>(S, V, x, y, s_id, s_t, s_ent, tid, rgb, nullptr, nullptr, status);
+    if constexpr (LPR == 1) block_pixel(KDGR_TILE_8X4, bx, by, q, lane, x, y);
+    else group_pixel<LPR>(bx, by, q, lane, x, y);
+    render_px<kHits, PACKED ? kFormPacked : kFormFp32, PKT, LPR>(S, V, x, y, s_id, s_t, s_ent, tid, outs[vi], nullptr,
+                                                                nullptr, status);
+  };
+  if constexpr (LPR == 1) {
+    GroupWalk G(share, total, 4u);
+    uint32_t g, sub;
+    while (G.next(queue, (unsigned)lane, g, sub)) {
+      const int vi = find_view(views, n_views, g, kSchedGroups);
+      const int W = __ldg(&views[vi].W), H = __ldg(&views[vi].H);
+      int bx, by;
+      G.block(g - __ldg(&views[vi].grp_base), sub / 4u, W, H, bx, by);
+      if (bx < W && by < H) render(vi, bx, by, (int)(sub % 4u));
+    }
+  } else {
+    uint32_t smid;
+    asm("mov.u32 %0, %%smid;" : "=r"(smid));
+    const uint32_t n = (uint32_t)share;
+    uint32_t k = smid % n, fails = 0;
+    while (fails <= n) {  // a warp's claims fail at most once per strip
+      const uint32_t b0 = strip_lo(total, n, k), b1 = strip_lo(total, n, k + 1);
+      uint32_t it = 0;
+      if (lane == 0) it = b0 + atomicAdd(queue + 1 + k, 1u);
+      it = __shfl_sync(0xFFFFFFFFu, it, 0);
+      if (it >= b1) {
+        ++fails;
+        k = next_open_strip(queue, total, n, k, (unsigned)lane);
+        if (k >= n) break;
+        continue;
+      }
+      const uint32_t blk = it / (4u * LPR);
+      const int vi = find_view(views, n_views, blk, KDGR_SCHED_CTA_BLOCKS);
+      const uint32_t lb = blk - __ldg(&views[vi].cb_base), nx = __ldg(&views[vi].cb_x);
+      render(vi, (int)(lb % nx) * kBlockW, (int)(lb / nx) * kBlockH, (int)(it % (4u * LPR)));
+    }
   }
 }
 
@@ -310,6 +400,8 @@ int lanes_per_ray(const kdgr_batch_config& c) {
 
 template <bool PACKED, int KB, bool PKT>
 KernelFn pick_sched_k(const kdgr_batch_config& c) {
+  if constexpr (KB == kHits)  // choose_walk's launches only: packets with 64 registers, independent rays with 80
+    if (c.schedule == kSchedGroups) return k_render_batch<PACKED, kSchedGroups, PKT ? 8 : 6, KB, PKT, 1>;
   if (c.schedule == KDGR_SCHED_CTA_BLOCKS) return pick_minb<PACKED, KDGR_SCHED_CTA_BLOCKS, KB, PKT, 1>(c.min_blocks);
   if (c.schedule == KDGR_SCHED_SM_STRIPS) return pick_minb<PACKED, KDGR_SCHED_SM_STRIPS, KB, PKT, 1>(c.min_blocks);
   if (c.schedule == KDGR_SCHED_WARP_STRIPS) {
@@ -385,6 +477,19 @@ cudaError_t resident_ctas(F* fn, int* out) {
 
 }  // namespace
 
+// First group of every view and their number, for a launch of `tiles` 8x4
+// tiles in all.
+uint32_t number_groups(ViewDesc* views, int n_views, uint64_t tiles) {
+  const GroupShape gs = group_shape(tiles);
+  uint64_t base = 0;
+  for (int v = 0; v < n_views; ++v) {
+    views[v].grp_base = (uint32_t)base;
+    base += (uint64_t)((views[v].W + (16 << gs.lx) - 1) >> (4 + gs.lx)) *
+            (uint64_t)((views[v].H + (8 << gs.ly) - 1) >> (3 + gs.ly));
+  }
+  return (uint32_t)base;
+}
+
 // Host: view table and total tile count for a list of views.
 int make_view_table(const kdgr_view* views, int n_views, std::vector<ViewDesc>& out, uint32_t totals[3]) {
   out.resize(n_views);
@@ -411,7 +516,7 @@ int fill_view_table(const kdgr_view* views, int n_views, ViewDesc* out, uint32_t
     d.cb_base = (uint32_t)cbase;
     d.out_off = kv.out_offset;
     d.scene = 0;
-    d.pad = 0;
+    d.grp_base = 0;
     wbase += (uint64_t)d.wt_x * (uint64_t)((kv.height + kTileH - 1) / kTileH);
     cbase += (uint64_t)d.cb_x * (uint64_t)((kv.height + kBlockH - 1) / kBlockH);
     if (wbase > 0xF0000000ull) {
@@ -421,7 +526,7 @@ int fill_view_table(const kdgr_view* views, int n_views, ViewDesc* out, uint32_t
   }
   totals[0] = (uint32_t)wbase;
   totals[1] = (uint32_t)cbase;
-  totals[2] = 0;
+  totals[2] = number_groups(out, n_views, wbase);
   return KDGR_OK;
 }
 
@@ -488,7 +593,8 @@ int check_batch_config(kdgr_scene_t s, const kdgr_batch_config& c) {
 constexpr uint64_t kFewRays = 30000, kSomeRays = 250000, kSomeRaysDense = 1200000;
 
 // The configuration a launch runs with: a caller's own choice as it is; the
-// default one (precision apart) with the walk that suits the number of rays.
+// default one (precision apart) by groups, with the walk that suits the number
+// of rays.
 // Every walk gives the same pixels bit for bit.
 kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64_t rays) {
   kdgr_batch_config d;
@@ -496,11 +602,15 @@ kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64
   d.precision = c.precision;
   if (memcmp(&d, &c, sizeof d) != 0) return c;
   const bool dense = s->n_pair_entries / 64u > s->n_gauss;
-  if (rays >= (dense ? kSomeRaysDense : kSomeRays)) return c;
-  d.schedule = KDGR_SCHED_WARP_STRIPS;
+  d.schedule = kSchedGroups;
+  if (rays >= (dense ? kSomeRaysDense : kSomeRays)) return d;
   d.min_blocks = 6;
-  if (rays < kFewRays) d.rays_per_warp = 4;
-  else d.traversal = KDGR_TRAV_RAY;
+  if (rays < kFewRays) {
+    d.schedule = KDGR_SCHED_WARP_STRIPS;  // the finest shares: 10k rays 210 us, in groups 275
+    d.rays_per_warp = 4;
+  } else {
+    d.traversal = KDGR_TRAV_RAY;
+  }
   return d;
 }
 
@@ -509,6 +619,7 @@ cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& cc, const View
                          const uint32_t totals[3], float* rgb, float* alpha, float* depth, uint32_t* queue,
                          cudaStream_t st) {
   const kdgr_batch_config c = choose_walk(s, cc, 32ull * totals[0]);
+  const bool by_groups = c.schedule == kSchedGroups;
   const uint32_t total_tiles = totals[0], total_blocks = totals[1];
   KernelFn fn = pick_kernel(c);
   int per_sm = c.blocks_per_sm;
@@ -521,13 +632,16 @@ cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& cc, const View
   if (warp_strips && total_blocks > 0x3FFFFFFFu) return cudaErrorInvalidValue;
   const uint32_t lpr = (uint32_t)lanes_per_ray(c);
   if (warp_strips && total_blocks > 0x3FFFFFFFu / lpr) return cudaErrorInvalidValue;
-  const uint32_t total = warp_strips ? 4u * lpr * total_blocks : per_warp ? total_tiles : total_blocks;
+  const uint32_t total =
+      by_groups ? totals[2] : warp_strips ? 4u * lpr * total_blocks : per_warp ? total_tiles : total_blocks;
   // SM strips: the kernel's `chunk` argument carries the number of strips
-  const bool strips = c.schedule == KDGR_SCHED_SM_STRIPS || warp_strips;
-  const int chunk = strips ? std::min(num_sms(), kMaxStrips) : c.chunk;
+  const bool strips = c.schedule == KDGR_SCHED_SM_STRIPS || warp_strips || by_groups;
+  const GroupShape gs = group_shape(total_tiles);
+  int chunk = strips ? std::min(num_sms(), kMaxStrips) : c.chunk;
+  if (by_groups) chunk = group_arg(chunk, gs);
   uint64_t blocks = (uint64_t)num_sms() * per_sm;
   const uint64_t grabs = strips ? total : ((uint64_t)total + chunk - 1) / chunk;
-  const uint64_t cap = per_warp ? (grabs + kWarps - 1) / kWarps : grabs;
+  const uint64_t cap = by_groups ? ((uint64_t)lpr << (gs.lx + gs.ly)) * total : per_warp ? (grabs + kWarps - 1) / kWarps : grabs;
   if (blocks > cap) blocks = cap > 0 ? cap : 1;
   fn<<<(unsigned)blocks, kThreads, 0, st>>>(s->fast_view(c.precision != 0), d_views, n_views, total, rgb, alpha,
                                             depth, queue, s->d_status, chunk, c.tile_shape);
@@ -678,8 +792,8 @@ cudaError_t stage_views(const ViewDesc* views, int n_views, ViewDesc* d_views, u
 }
 
 cudaError_t launch_multi(const SceneTable& scenes, bool packed, const ViewDesc* d_views, int n_views,
-                         uint32_t total_blocks, float* const* d_outs, uint32_t* queue, uint32_t* status,
-                         cudaStream_t st) {
+                         uint32_t total_blocks, uint32_t total_groups, float* const* d_outs, uint32_t* queue,
+                         uint32_t* status, cudaStream_t st) {
   // the walk by the number of rays, as choose_walk (the scenes may differ)
   const uint64_t rays = (uint64_t)kBlockW * kBlockH * total_blocks;
   const uint32_t lpr = rays < kFewRays ? 8 : 1;
@@ -690,12 +804,14 @@ cudaError_t launch_multi(const SceneTable& scenes, bool packed, const ViewDesc* 
   cudaError_t e = resident_ctas(reinterpret_cast<const void*>(fn), &occ);
   if (e != cudaSuccess) return e;
   if (total_blocks > 0x3FFFFFFFu) return cudaErrorInvalidValue;
-  const uint32_t items = 4u * lpr * total_blocks;
+  const GroupShape gs = group_shape(4ull * total_blocks);
+  const int sms = std::min(num_sms(), kMaxStrips);
+  const uint32_t total = lpr == 8 ? 4u * lpr * total_blocks : total_groups;
+  const int share = lpr == 8 ? sms : group_arg(sms, gs);
   uint64_t blocks = (uint64_t)num_sms() * (occ > 0 ? occ : 1);
-  const uint64_t cap = ((uint64_t)items + kWarps - 1) / kWarps;
+  const uint64_t cap = (uint64_t)lpr * total_blocks;  // four items to a block, four warps to a CTA
   if (blocks > cap) blocks = cap > 0 ? cap : 1;
-  fn<<<(unsigned)blocks, kThreads, 0, st>>>(scenes, d_views, n_views, items, d_outs, queue, status,
-                                            std::min(num_sms(), kMaxStrips));
+  fn<<<(unsigned)blocks, kThreads, 0, st>>>(scenes, d_views, n_views, total, d_outs, queue, status, share);
   return cudaGetLastError();
 }
 

@@ -985,11 +985,14 @@ __device__ __forceinline__ void trace_packets(const SceneOf<FORM>& S, Ray& R, bo
   }
 }
 
+constexpr int kSchedGroups = 4;  // the groups schedule (render_fast.cu); not a KDGR_SCHED_* value
 __device__ __forceinline__ int find_view(const ViewDesc* views, int n_views, uint32_t item, int sched) {
   int lo = 0, hi = n_views - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    const uint32_t b = sched == KDGR_SCHED_WARP_TILES ? __ldg(&views[mid].wt_base) : __ldg(&views[mid].cb_base);
+    const uint32_t b = sched == kSchedGroups              ? __ldg(&views[mid].grp_base)
+                       : sched == KDGR_SCHED_WARP_TILES ? __ldg(&views[mid].wt_base)
+                                                        : __ldg(&views[mid].cb_base);
     if (b <= item) lo = mid;
     else hi = mid - 1;
   }
@@ -1036,6 +1039,13 @@ __device__ __forceinline__ void render_px(const FastView& S, const ViewDesc& V, 
     if ((tid & (LPR - 1)) != 0) return;
     store_px(V, x, y, R, rgb, alpha_out, depth_out);
   }
+}
+
+// i-th of n positions from the middle outwards: blocks are handed out in this
+// order, so that a launch ends on the image border, where rays are short.
+__device__ __forceinline__ uint32_t middle_out(uint32_t i, uint32_t n) {
+  const uint32_t m = (n - 1) / 2;
+  return (i & 1u) ? m + (i + 1) / 2 : m - i / 2;
 }
 
 // Pixel of lane `lane` in quarter q (0..3) of the 16x8 block whose top-left

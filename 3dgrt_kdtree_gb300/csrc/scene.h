@@ -178,7 +178,7 @@ cudaError_t build_flag_pairs(const uint32_t* d_gid, uint32_t n_entries, const ui
 // The FP64 factors of n flagged Gaussians (k_aniso_fp64).
 cudaError_t launch_aniso_fp64(const float* src, uint32_t n, float4* table, cudaStream_t st);
 // Batched rendering (render_fast.cu).
-// totals: 8x4 tiles, 16x8 blocks and 32x16 super-blocks over all views.
+// totals: 8x4 tiles, 16x8 blocks and groups of blocks over all views.
 int make_view_table(const kdgr_view* views, int n_views, std::vector<ViewDesc>& out, uint32_t totals[3]);
 int fill_view_table(const kdgr_view* views, int n_views, ViewDesc* out, uint32_t totals[3]);
 int check_batch_config(kdgr_scene_t s, const kdgr_batch_config& c);
@@ -190,6 +190,9 @@ cudaError_t launch_batch(kdgr_scene_t s, const kdgr_batch_config& c, const ViewD
                          const uint32_t totals[3], float* rgb, float* alpha, float* depth, uint32_t* queue,
                          cudaStream_t st);
 int batch_sms();
+// Sets every view's first group for a launch of `tiles` 8x4 tiles in all;
+// returns the number of groups.
+uint32_t number_groups(ViewDesc* views, int n_views, uint64_t tiles);
 // Writes a launch's view table to d_views and zeroes its queue words
 // (kQueueBytes at d_queue), stream-ordered: up to 256 views in the
 // parameters of one staging kernel, more by one copy from host memory that
@@ -202,11 +205,12 @@ constexpr int kSceneSlots = 64;
 struct SceneTable {
   FastView s[kSceneSlots];
 };
-// Multi-scene persistent launch (warp-strip schedule) for the serving loop;
-// views[v].scene indexes the table and d_outs[v] is view v's output base.
+// Multi-scene persistent launch for the serving loop; views[v].scene indexes
+// the table and d_outs[v] is view v's output base.  The views' groups are
+// numbered for 4 * total_blocks tiles.
 cudaError_t launch_multi(const SceneTable& scenes, bool packed, const ViewDesc* d_views, int n_views,
-                         uint32_t total_blocks, float* const* d_outs, uint32_t* queue, uint32_t* status,
-                         cudaStream_t st);
+                         uint32_t total_blocks, uint32_t total_groups, float* const* d_outs, uint32_t* queue,
+                         uint32_t* status, cudaStream_t st);
 // Scale ratio above which a Gaussian's factors come from the FP64 precompute.
 constexpr double kAnisoRatio = 1e3;
 

@@ -22,7 +22,9 @@ def scene(pkg, cuda, request):
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("sizes", [[(1, 1)], [(7, 3)], [(199, 149)], [(203, 151)], [(499, 499)], [(503, 509)],
-                                   [(64, 48)] * 9, [(160, 120), (33, 17), (250, 190)]])
+                                   [(64, 48)] * 9, [(160, 120), (33, 17), (250, 190)],
+                                   # groups of 2x2 and 2x4 blocks
+                                   [(1203, 701)], [(1920, 1088), (17, 3), (331, 77), (1919, 1089)]])
 def test_default_equals_explicit(pkg, cuda, scene, precision, sizes):
     rec, tree, S = scene
     F = pkg.renderer
@@ -48,7 +50,7 @@ def test_default_equals_explicit(pkg, cuda, scene, precision, sizes):
     assert S.status() == 0
     for a, b, c in zip(want, got, graph):
         assert torch.equal(a, b) and torch.equal(a, c)
-    srv = F.Server(hbm_budget_bytes=2 << 30, arena_bytes=64 << 20, precision=precision)
+    srv = F.Server(hbm_budget_bytes=2 << 30, arena_bytes=128 << 20, precision=precision)
     slot = srv.add_scene(tree, rec)
     out = torch.full((total * 3,), -1.0).pin_memory()
     assert srv.wait(srv.submit(slot, views, len(cams), out))[0] == 0
