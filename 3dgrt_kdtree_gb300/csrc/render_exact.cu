@@ -574,14 +574,15 @@ cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamIn
     // outgrow L2 where the records themselves do not (100k overlapping
     // Gaussians, 175 leaves each: 980 MB against 8 MB), so the walk over the
     // tree as given is the faster one unless rays are few (65k rays: 410 us,
-    // 4 lanes per ray 360; 250k rays: 540, packets 950, own walk 560).
+    // 4 lanes per ray 360; 250k rays: 540, packets 950, own walk 560) and
+    // below a full frame (2.1M rays: 1974, packets 1668).
     const bool copies = s.n_offsets / 64u > s.n_gauss;
     if (rays < 30000) return launch_plain<8, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (copies && rays < 70000) return launch_plain<4, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 60000) return launch_plain<4, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 300000) return launch_plain<1, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 1000000) return launch_plain<1, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (!copies) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies || rays >= 1500000) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
   }
   dim3 grid((W + 15) / 16, (H + 7) / 8);
   if (trace)

@@ -794,12 +794,15 @@ cudaError_t stage_views(const ViewDesc* views, int n_views, ViewDesc* d_views, u
 cudaError_t launch_multi(const SceneTable& scenes, bool packed, const ViewDesc* d_views, int n_views,
                          uint32_t total_blocks, uint32_t total_groups, float* const* d_outs, uint32_t* queue,
                          uint32_t* status, cudaStream_t st) {
-  // the walk by the number of rays, as choose_walk (the scenes may differ)
+  // The walk by the number of rays, as choose_walk (the scenes may differ), but
+  // independent rays only below 100k: other lanes' launches fill the chip, and
+  // packets take less of it (12 requests of 400x300: 1.86 to 2.05 ms, 1.95 to
+  // 2.10 with independent rays; 8 of 300x220: 1.04 to 1.28, 0.84 to 1.05).
   const uint64_t rays = (uint64_t)kBlockW * kBlockH * total_blocks;
   const uint32_t lpr = rays < kFewRays ? 8 : 1;
   auto fn = packed ? k_render_multi<true, 8, true, 1> : k_render_multi<false, 8, true, 1>;
   if (lpr == 8) fn = packed ? k_render_multi<true, 6, true, 8> : k_render_multi<false, 6, true, 8>;
-  else if (rays < kSomeRays) fn = packed ? k_render_multi<true, 6, false, 1> : k_render_multi<false, 6, false, 1>;
+  else if (rays < 100000) fn = packed ? k_render_multi<true, 6, false, 1> : k_render_multi<false, 6, false, 1>;
   int occ = 0;
   cudaError_t e = resident_ctas(reinterpret_cast<const void*>(fn), &occ);
   if (e != cudaSuccess) return e;
