@@ -42,12 +42,14 @@ constexpr uint32_t kTestWords = 5;
 // The plain form's leaf-order arrays for the packet walk: the fast form's
 // relaid tree, padded ID list and FP32 pairs, and per pair the constants of
 // the filter's tolerance (Ce lo, Ce hi, Cmu lo, Cmu hi; render_packet.cuh).
-// leaf_tol is null when they were not materialised.
+// leaf_tol is null when they were not materialised.  leaf_first: first pair of
+// each leaf of the tree as given (ExactView's nodes), for the traced walk.
 struct PlainView {
   const uint2* nodes;
   const uint32_t* offsets;
   const float4* leaf_pairs;
   const float4* leaf_tol;
+  const uint32_t* leaf_first;
   const float4* test;
   const float4* sh;
   uint32_t n_offsets, n_gauss;

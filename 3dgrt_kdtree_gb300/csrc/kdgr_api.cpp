@@ -97,6 +97,7 @@ kdgr::PlainView kdgr_scene_s::plain_view() const {
   v.offsets = d_pair_gid;
   v.leaf_pairs = d_leaf_pairs;
   v.leaf_tol = d_leaf_tol;
+  v.leaf_first = d_leaf_first;
   v.test = d_test;
   v.sh = d_sh;
   v.n_offsets = n_pair_entries;
@@ -228,6 +229,7 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     P.add(s->d_pair_gid, 2 * n_pairs + 2);
     if (fast || plain) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
     if (plain) P.add(s->d_leaf_tol, n_pairs + 1);
+    if (plain) P.add(s->d_leaf_first, n_nodes);
     return P.make(s->blocks);
   };
   Slab P;
@@ -241,6 +243,7 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
       plain = false;
       s->d_pair_gid = nullptr;
       s->d_leaf_pairs = s->d_leaf_tol = nullptr;
+      s->d_leaf_first = nullptr;
       P = Slab();
       e = fast || packed ? leaf_arrays(false, P) : cudaSuccess;
     }
@@ -254,6 +257,7 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
       e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, po.fast, s->d_leaf_pairs, W.st);
     if (e == cudaSuccess && s->d_leaf_tol)
       e = build_leaf_tol(s->d_pair_gid, s->n_pair_entries, po.tol, s->d_leaf_tol, W.st);
+    if (e == cudaSuccess && s->d_leaf_first) e = tree_leaf_first(W, L, first, s->d_leaf_first);
     if (e != cudaSuccess) return fail("leaf order", e);
   }
   Slab Q;

@@ -539,10 +539,12 @@ __device__ __forceinline__ unsigned group_mask(int LPR) {
 // Measured (GB300, 64 or 80 registers): a 1080p packet frame 2.39 ms entry by
 // entry, 2.75 ms marked (spills, 32 different records per load); a 320x240
 // frame of independent rays 391 us entry by entry, 378 us marked.
+// COUNT: *found counts the accepted hits.
 constexpr uint32_t kChunk = 16;
-template <int K, int LPR, bool PACKET>
+template <int K, int LPR, bool PACKET, bool COUNT = false>
 __device__ __forceinline__ bool scan_plain(const PlainView& S, const LeafRef& L, const Ray& R, float tn, unsigned mask,
-                                           bool have_last, float last_t, uint32_t last_i, HitBuf<K>& hb) {
+                                           bool have_last, float last_t, uint32_t last_i, HitBuf<K>& hb,
+                                           uint32_t* found = nullptr) {
   const unsigned sub = threadIdx.x & (LPR - 1u);
   bool overflow = false;
   const Ray2 w = ray2(R.o, R.d);
@@ -550,9 +552,9 @@ __device__ __forceinline__ bool scan_plain(const PlainView& S, const LeafRef& L,
   auto test = [&](uint32_t ik) {
     float t, g;
     const uint32_t gid = __ldg(S.offsets + 2ull * L.pb + ik);
-    if (gid < S.n_gauss && exact_test(R.o, R.d, S.test + kTestWords * (size_t)gid, tn, R.t_far, &t, &g) &&
-        (!have_last || t > last_t || (t == last_t && ik > last_i)))
-      overflow |= hb.insert(t, g, ik);
+    if (gid >= S.n_gauss || !exact_test(R.o, R.d, S.test + kTestWords * (size_t)gid, tn, R.t_far, &t, &g)) return;
+    if (COUNT) ++*found;
+    if (!have_last || t > last_t || (t == last_t && ik > last_i)) overflow |= hb.insert(t, g, ik);
   };
   // pair p of the leaf; a lane past its end tests the last pair again and drops it
   auto filter_t = [&](uint32_t p, PlainPair& x) {

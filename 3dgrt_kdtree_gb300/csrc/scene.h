@@ -39,6 +39,7 @@ struct kdgr_scene_s {
   uint32_t n_pair_entries = 0;     // even
   float4* d_leaf_pairs = nullptr;  // FP32 and plain forms, 6 x float4 per pair of entries
   float4* d_leaf_tol = nullptr;    // plain form, 1 x float4 per pair of entries
+  uint32_t* d_leaf_first = nullptr;  // plain form: first pair of each leaf of d_nodes
   uint4* d_leaf_packed = nullptr;  // packed form, 4 x uint4 per pair of plain entries
   // The packed form's own leaf layout: a leaf's plain entries in FP16 pairs
   // (d_leaf_packed), its flagged entries (scale ratio > 1e3 or factors beyond
@@ -136,6 +137,7 @@ int cuda_fail(cudaError_t e, const char* where);
 // reached from the root, listed level by level:
 struct TreeLists {
   uint32_t *list = nullptr, *cpos = nullptr, *ls = nullptr;  // node, list position of its left child, level starts
+  uint32_t* idx = nullptr;                                   // relaid number of each listed node (tree_relayout)
   std::vector<uint32_t> starts;                              // host copy of ls
   uint32_t n = 0, levels = 0, top_nodes = 0;
   uint32_t n_leaves = 0, max_leaf = 0;  // over all nodes given
@@ -145,13 +147,15 @@ cudaError_t tree_check(WorkMem& W, const uint2* d_nodes, uint32_t n_nodes, const
                        uint32_t n_offsets, uint32_t n_gauss, TreeLists& L);
 // Fast-form node order into out[0 .. L.n): top levels breadth-first, rest
 // depth-first; leaf words as given.
-cudaError_t tree_relayout(WorkMem& W, const uint2* d_nodes, const TreeLists& L, uint2* out);
+cudaError_t tree_relayout(WorkMem& W, const uint2* d_nodes, TreeLists& L, uint2* out);
 // First pair of every relaid leaf (exclusive sums, n + 1 of them) and the
 // number of pairs; synchronises.
 cudaError_t tree_leaf_pairs(WorkMem& W, const uint2* relaid, uint32_t n, uint64_t** first, uint64_t* n_pairs);
 // Padded leaf-order IDs; leaf word y of the relaid tree becomes its first pair.
 cudaError_t tree_leaf_gids(WorkMem& W, uint2* relaid, uint32_t n, const uint64_t* first, const uint32_t* d_offsets,
                            uint32_t* gid);
+// First pair of every leaf, at its number in the tree as given.
+cudaError_t tree_leaf_first(WorkMem& W, const TreeLists& L, const uint64_t* first, uint32_t* out);
 // Table index of every flagged Gaussian (0xFFFFFFFF for the others); n_aniso
 // is set once the stream has been synchronised.
 cudaError_t aniso_index(WorkMem& W, const uint8_t* flag, uint32_t n, uint32_t** aidx, uint32_t* n_aniso);

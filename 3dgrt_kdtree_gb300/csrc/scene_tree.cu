@@ -245,6 +245,14 @@ __global__ void k_leaf_gids(uint2* nodes, uint32_t n, const uint64_t* __restrict
   if (lane == 0) nodes[i].y = (uint32_t)p;
 }
 
+// First pair of every leaf under its number in the tree as given.
+__global__ void k_leaf_first(const uint32_t* __restrict__ list, const uint32_t* __restrict__ cpos,
+                             const uint32_t* __restrict__ idx, uint32_t n, const uint64_t* __restrict__ first,
+                             uint32_t* out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && cpos[i] == kNone) out[list[i]] = (uint32_t)first[idx[i]];
+}
+
 struct FlagOp {
   const uint8_t* flag;
   uint64_t n;
@@ -376,9 +384,9 @@ cudaError_t tree_check(WorkMem& W, const uint2* d_nodes, uint32_t n_nodes, const
   return cudaSuccess;
 }
 
-cudaError_t tree_relayout(WorkMem& W, const uint2* d_nodes, const TreeLists& L, uint2* out) {
+cudaError_t tree_relayout(WorkMem& W, const uint2* d_nodes, TreeLists& L, uint2* out) {
   uint32_t* sub = W.take<uint32_t>(L.n);
-  uint32_t* idx = W.take<uint32_t>(L.n);
+  uint32_t* idx = L.idx = W.take<uint32_t>(L.n);
   uint32_t* pair = W.take<uint32_t>(L.n);
   if (W.err != cudaSuccess) return W.err;
   auto grid = [&](int l) { return std::min(kSweep, blocks_for(L.starts[l + 1] - L.starts[l], 256)); };
@@ -401,6 +409,11 @@ cudaError_t tree_leaf_pairs(WorkMem& W, const uint2* relaid, uint32_t n, uint64_
 cudaError_t tree_leaf_gids(WorkMem& W, uint2* relaid, uint32_t n, const uint64_t* first, const uint32_t* d_offsets,
                            uint32_t* gid) {
   k_leaf_gids<<<blocks_for(n, 256 / kLeafLanes), 256, 0, W.st>>>(relaid, n, first, d_offsets, gid);
+  return cudaGetLastError();
+}
+
+cudaError_t tree_leaf_first(WorkMem& W, const TreeLists& L, const uint64_t* first, uint32_t* out) {
+  k_leaf_first<<<blocks_for(L.n, 256), 256, 0, W.st>>>(L.list, L.cpos, L.idx, L.n, first, out);
   return cudaGetLastError();
 }
 
