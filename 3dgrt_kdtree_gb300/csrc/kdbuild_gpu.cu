@@ -330,6 +330,16 @@ __global__ void k_box_decode(const uint32_t* box, float* node_lo, float* node_hi
 }
 
 // ------------------------------------------------------------ runs and nodes
+// Counters of one level: nodes listed for the 128- and 512-thread searches,
+// planar keys and scored candidates of the large nodes' search.
+enum { kCntMid, kCntBlock, kCntPlanar, kCntScored, kCounts };
+
+// Sizes of the next level, read back once per level.
+struct LevelSum {
+  unsigned long long triangles;
+  uint32_t n_split, leaf_ids, max_ids;  // max_ids: most IDs in a split node
+};
+
 struct HeadOp {  // 1 where a (node, Gaussian) run starts
   const uint32_t *tri, *node;
   uint64_t T;
@@ -339,9 +349,14 @@ struct HeadOp {  // 1 where a (node, Gaussian) run starts
   }
 };
 
+// (Zeroes the level's counters as well: a memset each was a launch each.)
 __global__ void k_run_scatter(const uint32_t* __restrict__ ridx, const uint32_t* __restrict__ node, size_t T,
-                              uint32_t* run_start, uint32_t* run_node) {
+                              uint32_t* run_start, uint32_t* run_node, uint32_t* counts, LevelSum* sum) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) {
+    for (int k = 0; k < kCounts; ++k) counts[k] = 0u;
+    *sum = LevelSum{0ull, 0u, 0u, 0u};
+  }
   if (t >= T) return;
   const uint32_t r = ridx[t];
   if (ridx[t + 1] == r) return;
@@ -368,7 +383,7 @@ constexpr uint32_t kFewNodes = 4096;
 
 // Per node: its first run, its ID count, the class lists of its split search
 // (nodes of up to kWarpIds need no list) and a leaf decision to begin with.
-// counts: [0] kMidIds nodes, [1] kBlockIds nodes, [2] larger nodes.
+// eG (levels that may hold larger nodes): their ID counts, 0 for the others.
 __global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ ridx, uint32_t N,
                              int level, int max_level, uint32_t warp_ids, uint32_t* rb, Decision* dec, uint32_t* is_split,
                              uint32_t* list_mid, uint32_t* list_block, uint32_t* counts, uint32_t* eG) {
@@ -377,19 +392,16 @@ __global__ void k_node_setup(const uint32_t* __restrict__ tb, const uint32_t* __
   rb[n] = ridx[tb[n]];
   if (n == N) {
     is_split[n] = 0u;
+    if (eG) eG[n] = 0u;
     return;
   }
   const uint32_t G = ridx[tb[n + 1]] - ridx[tb[n]];
   dec[n] = Decision{-1, 0.f, 0};
   is_split[n] = 0u;
   const bool elig = level < max_level && G > kMinPrim;
-  if (elig && G > warp_ids && G <= kMidIds) list_mid[atomicAdd(&counts[0], 1u)] = n;
-  if (elig && G > kMidIds && G <= kBlockIds) list_block[atomicAdd(&counts[1], 1u)] = n;
-  if (eG) {
-    const bool big = elig && G > kBlockIds;
-    eG[n] = big ? G : 0u;
-    if (big) atomicAdd(&counts[2], 1u);
-  }
+  if (elig && G > warp_ids && G <= kMidIds) list_mid[atomicAdd(&counts[kCntMid], 1u)] = n;
+  if (elig && G > kMidIds && G <= kBlockIds) list_block[atomicAdd(&counts[kCntBlock], 1u)] = n;
+  if (eG) eG[n] = elig && G > kBlockIds ? G : 0u;
 }
 
 // ------------------------------------------------------------ scores
@@ -1269,12 +1281,6 @@ struct Rec {
   uint32_t leaf_off, leaf_cnt;
 };
 
-// Sizes of the next level, read back once per level.
-struct LevelSum {
-  unsigned long long triangles;
-  uint32_t n_split, leaf_ids, max_ids;  // max_ids: most IDs in a split node
-};
-
 // Per node: its record, and for split nodes the children's boxes and first
 // triangles.
 __global__ void k_children(const uint32_t* __restrict__ tb, const uint32_t* __restrict__ rb, uint32_t N,
@@ -1534,20 +1540,17 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
       depth = (uint32_t)level;
       const TriView V = view(cur);
       // 1. runs of (node, ID)
-      DBuf<uint32_t> ridx(S, T + 1), run_start(S, T + 1), run_node(S, T + 1), rb(S, (size_t)N + 1);
+      DBuf<uint32_t> ridx(S, T + 1), run_start(S, T + 1), run_node(S, T + 1), rb(S, (size_t)N + 1), counts(S, kCounts);
+      DBuf<LevelSum> d_sum(S, 1);
       if (S.err != cudaSuccess) break;
       exclusive_sum_of(S, tmp, HeadOp{V.tri, V.node, T}, ridx.p, T + 1);
-      k_run_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(ridx.p, V.node, T, run_start.p, run_node.p);
+      k_run_scatter<<<grid_for(T, 256), 256, 0, S.s>>>(ridx.p, V.node, T, run_start.p, run_node.p, counts.p, d_sum.p);
       // 2. node classes and split search; large nodes can only appear below a large node
       const bool may_be_big = max_ids > kBlockIds;
       DBuf<Decision> dec(S, N);
-      DBuf<uint32_t> is_split(S, (size_t)N + 1), lists(S, 2 * (size_t)N), counts(S, 3), eG;
-      if (may_be_big) {
-        eG.alloc(S, (size_t)N + 1);
-        eG.zero();
-      }
+      DBuf<uint32_t> is_split(S, (size_t)N + 1), lists(S, 2 * (size_t)N), eG;
+      if (may_be_big) eG.alloc(S, (size_t)N + 1);
       if (S.err != cudaSuccess) break;
-      counts.zero();
       const uint32_t warp_ids = N < kFewNodes ? 0u : kWarpIds;
       k_node_setup<<<grid_for((size_t)N + 1, 128), 128, 0, S.s>>>(tb.p, ridx.p, N, level, P.max_level, warp_ids, rb.p,
                                                                   dec.p, is_split.p, lists.p, lists.p + N, counts.p,
@@ -1556,10 +1559,10 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
         k_search_warp<<<grid_for(N, kSearchWarps), 32 * kSearchWarps, 0, S.s>>>(
             P, N, level, tb.p, rb.p, ridx.p, V, nlo.p, nhi.p, dec.p, is_split.p);
       if (max_ids > std::max(warp_ids, kMinPrim))
-        launch_search_block<128, (int)kMidIds>(S, P, lists.p, counts.p, N, tb.p, rb.p, ridx.p, V, nlo.p, nhi.p, dec.p,
+        launch_search_block<128, (int)kMidIds>(S, P, lists.p, counts.p + kCntMid, N, tb.p, rb.p, ridx.p, V, nlo.p, nhi.p, dec.p,
                                                is_split.p);
       if (max_ids > kMidIds)
-        launch_search_block<512, (int)kBlockIds>(S, P, lists.p + N, counts.p + 1, N, tb.p, rb.p, ridx.p, V,
+        launch_search_block<512, (int)kBlockIds>(S, P, lists.p + N, counts.p + kCntBlock, N, tb.p, rb.p, ridx.p, V,
                                                  nlo.p, nhi.p, dec.p, is_split.p);
       if (may_be_big) {
         DBuf<uint32_t> grb(S, (size_t)N + 1);
@@ -1577,17 +1580,15 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
           while ((1ull << B.nb) < N) ++B.nb;
           DBuf<uint64_t> kmin(S, 3 * (size_t)eGT), kmax(S, 3 * (size_t)eGT), kpl(S, 3 * (size_t)eGT),
               alt(S, 3 * (size_t)eGT);
-          DBuf<uint32_t> pl_fill(S, 1), best32(S, N), hull(S, 6 * (size_t)N);
+          DBuf<uint32_t> best32(S, N), hull(S, 6 * (size_t)N);
           DBuf<unsigned long long> best64(S, 2 * (size_t)N);
           DBuf<float2> scores(S, 6 * (size_t)eGT);
           DBuf<Scored> scored(S, kScoredCap);
-          DBuf<uint32_t> n_scored(S, 1);
           if (S.err != cudaSuccess) break;
-          pl_fill.zero();
-          n_scored.zero();
+          uint32_t* const pl_fill = counts.p + kCntPlanar;
           k_run_bounds<<<grid_for(T, 128), 128, 0, S.s>>>(run_start.p, run_node.p, rb.p, N, T, V, B, kmin.p, kmax.p,
-                                                          kpl.p, pl_fill.p);
-          S.check(cudaMemcpyAsync(&B.n_pl, pl_fill.p, 4, cudaMemcpyDeviceToHost, S.s));
+                                                          kpl.p, pl_fill);
+          S.check(cudaMemcpyAsync(&B.n_pl, pl_fill, 4, cudaMemcpyDeviceToHost, S.s));
           const int end_bit = 32 + B.nb + 2;
           sort_keys(S, tmp, kmin, alt, 3 * (size_t)eGT, end_bit);
           sort_keys(S, tmp, kmax, alt, 3 * (size_t)eGT, end_bit);
@@ -1596,7 +1597,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
           B.kmin = kmin.p;
           B.kmax = kmax.p;
           B.kpl = kpl.p;
-          BigState st{best32.p, best64.p, best64.p + N, hull.p, hull.p + 3 * (size_t)N, scored.p, n_scored.p};
+          BigState st{best32.p, best64.p, best64.p + N, hull.p, hull.p + 3 * (size_t)N, scored.p, counts.p + kCntScored};
           const unsigned ge = grid_for(6 * (size_t)eGT, 256), gt = grid_for(T, 256), gn = grid_for(N, 128);
           k_big_init<<<gn, 128, 0, S.s>>>(P, B, tb.p, N, st);
           k_event_scores<<<ge, 256, 0, S.s>>>(P, B, tb.p, nlo.p, nhi.p, scores.p, st);
@@ -1614,9 +1615,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
       DBuf<Rec> rec(S, N);
       DBuf<float> clo(S, 6 * (size_t)N), chi(S, 6 * (size_t)N);
       DBuf<uint32_t> ctb(S, 2 * (size_t)N + 1);
-      DBuf<LevelSum> d_sum(S, 1);
       if (S.err != cudaSuccess) break;
-      d_sum.zero();
       exclusive_sum_of(S, tmp, NodeOp{is_split.p, rb.p, N}, nsc.p, (size_t)N + 1);
       exclusive_sum_of(S, tmp, SideOp{V, dec.p, T}, sc.p, T + 1);
       k_children<<<grid_for(N, 128), 128, 0, S.s>>>(tb.p, rb.p, N, dec.p, nsc.p, sc.p, (uint32_t)pool_used, nlo.p,
