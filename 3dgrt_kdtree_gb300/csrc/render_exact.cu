@@ -270,8 +270,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_render_plain(PlainView S, Ca
   if (depth_out) depth_out[idx] = v.w;
 }
 
-template <int K, bool TRACE, bool LEAF>
-__global__ void __launch_bounds__(kBlock) k_render_exact(ExactView S, PlainView L, CamInfo C, int W, int H, float* __restrict__ rgb,
+template <int K, bool TRACE, bool LEAF, int MINB = 0>
+__global__ void __launch_bounds__(kBlock, MINB) k_render_exact(ExactView S, PlainView L, CamInfo C, int W, int H, float* __restrict__ rgb,
                                                          float* __restrict__ alpha_out, float* __restrict__ depth_out,
                                                          kdgr_ray_trace* __restrict__ trace, uint32_t* status) {
   __shared__ uint32_t s_id[kStack][kBlock];
@@ -432,8 +432,8 @@ __device__ __forceinline__ SecHit intersect_secondary(const HybridView& M, const
 // the bounces; a lane whose ray has ended only waits.  What a pass does not
 // need (the running colour, throughput and the hit) waits in shared memory
 // meanwhile: in registers it spilled 600 bytes around the walk.
-template <int WALK>
-__global__ void __launch_bounds__(kBlock, WALK == 0 ? 0 : 6)
+template <int WALK, int MINB>
+__global__ void __launch_bounds__(kBlock, MINB)
     k_render_hybrid(ExactView S, PlainView L, CamInfo C, int W, int H, HybridView M, float* __restrict__ rgb,
                     uint32_t* status) {
   __shared__ uint32_t s_id[kStack][kBlock];
@@ -558,29 +558,40 @@ cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamIn
     //   110k rays  246 / 547 / 726   1 lane, own walk  178 / 405 / 475   (packets 233 / 633 / 572)
     //   400k rays  477 / 1215 / 1472 packets           305 / 757 / 880   (own walk 281 / 821 / 1011)
     //   2.1M rays  (1M Gaussians) 4260, packets 2504, with 64 registers 2394
+    // The lines over several scenes: at 36k rays 8 lanes and 4-lane packets
+    // meet; at 65k packets take 240 (uniform 40k Gaussians) and 413 (cluster
+    // 100k), own walks 264 and 366, but uniform scenes would lose against one
+    // thread per ray (276); at 307k own walks take 398 / 740, packets 392 / 765.
+    // Own walks of one lane have 96 registers: the 80 that 6 blocks leave spill
+    // (90k rays, cluster 100k: 409 against 391), 128 leave too few warps (307k:
+    // 804 against 740).
     const uint64_t rays = (uint64_t)W * H;
     // Gaussians that sit in more than 64 leaves each: their leaf-order copies
     // outgrow L2 where the records themselves do not (100k overlapping
     // Gaussians, 175 leaves each: 980 MB against 8 MB), so the walk over the
-    // tree as given is the faster one unless rays are few (65k rays: 410 us,
-    // 4 lanes per ray 360; 250k rays: 540, packets 950, own walk 560) and
-    // below a full frame (2.1M rays: 1974, packets 1668).
+    // tree as given is the faster one unless rays are few (20k rays: 427 us,
+    // 8 lanes per ray 198; 250k rays: 540, packets 950, own walk 560).
     const bool copies = s.n_offsets / 64u > s.n_gauss;
-    if (rays < 30000) return launch_plain<8, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (copies && rays < 70000) return launch_plain<4, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (!copies && rays < 60000) return launch_plain<4, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (!copies && rays < 300000) return launch_plain<1, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (rays < 36000) return launch_plain<8, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies && rays < 80000) return launch_plain<4, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies && rays < 350000) return launch_plain<1, 5, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 1000000) return launch_plain<1, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (!copies || rays >= 1500000) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
   }
-  dim3 grid((W + 15) / 16, (H + 7) / 8);
+  const dim3 grid((W + 15) / 16, (H + 7) / 8);
   // Traces filter the leaves' candidates too, unless the leaf copies are too
-  // large for L2 (see above): 640x480, 100k / 10k Gaussians 1310 -> 881 us and
-  // 503 -> 321; 256x256 496 -> 395 and 276 -> 213.
+  // large for L2 (see above): 640x480, 100k / 10k Gaussians 1310 -> 864 us and
+  // 503 -> 309; 256x256 500 -> 373 and 277 -> 199.  A bound of 4 blocks per SM
+  // leaves 128 registers and no spill; without it a 256x256 trace takes 397 / 214.
   if (trace && plain.leaf_tol && !(s.n_offsets / 64u > s.n_gauss))
-    k_render_exact<8, true, true><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
+    k_render_exact<8, true, true, 4><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
   else if (trace)
-    k_render_exact<8, true, false><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
+    k_render_exact<8, true, false, 4><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
+  // 128 registers pay while every block is resident at once (4 per SM) or
+  // nearly: overlapping 100k, 65k / 120k rays 444 / 500 us -> 382 / 432; at
+  // 307k rays the blocks wait for each other instead (571 -> 604).
+  else if ((uint64_t)W * H < 200000)
+    k_render_exact<8, false, false, 4><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
   else
     k_render_exact<8, false, false><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
   return cudaGetLastError();
@@ -592,15 +603,23 @@ cudaError_t launch_hybrid(const ExactView& s, const PlainView& plain, const CamI
   // us with 320 triangles, 100k / 10k Gaussians, one thread per ray first:
   // 256x256 765 / 731, own walk 657 / 599; 1280x720 2352 / 1203, packets
   // 1277 / 967 (own walk 1532 / 933); without groups of triangles to skip the
-  // 1280x720 frame took 3400.
+  // 1280x720 frame took 3400.  Own walks want 128 registers: with 80 they spill
+  // and 256x256 with 80 triangles takes 20 % longer, over 20k uniform Gaussians
+  // more than the walk over the tree as given (303).  At 500k rays own walks
+  // take 523 (uniform 20k) and 1142 (cluster 100k), packets 568 and 1041.
+  // Bounced rays gain less from leaf-order pairs than primary ones, so here the
+  // tree as given is the faster one from 16 leaves per Gaussian on, for small
+  // frames (120k rays over 33k uniform Gaussians, 17 leaves each: 308 us, own
+  // walk 339; 26k, 11 leaves each, 81k rays: 256 and 244).
   const dim3 grid((W + 15) / 16, (H + 7) / 8);
-  const bool leaf = plain.leaf_tol && !(s.n_offsets / 64u > s.n_gauss);
+  const bool leaf =
+      plain.leaf_tol && !(s.n_offsets / ((uint64_t)W * H < 300000 ? 16u : 64u) > s.n_gauss);
   if (!leaf)
-    k_render_hybrid<0><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
-  else if ((uint64_t)W * H < 300000)
-    k_render_hybrid<1><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
+    k_render_hybrid<0, 0><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
+  else if ((uint64_t)W * H < 600000)
+    k_render_hybrid<1, 4><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
   else
-    k_render_hybrid<2><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
+    k_render_hybrid<2, 6><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, m, rgb, status);
   return cudaGetLastError();
 }
 

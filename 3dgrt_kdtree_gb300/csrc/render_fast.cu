@@ -589,8 +589,13 @@ int check_batch_config(kdgr_scene_t s, const kdgr_batch_config& c) {
 //   400k rays  282 / 629 / 696 / 783    own walk      282 / 650 / 748 / 521
 // A scene whose Gaussians sit in more than 64 leaves each (the last one) has
 // leaves far smaller than a tile: its rays share too few of them for packets
-// up to a full frame (1.1M rays: 924 us, own walk 850).
-constexpr uint64_t kFewRays = 30000, kSomeRays = 250000, kSomeRaysDense = 1200000;
+// up to a full frame (1.1M rays: 924 us, own walk 850).  Between 16 and 64
+// leaves each, own walks win less far up; uniform 33k / 40k / 55k Gaussians (17,
+// 22 and 40 leaves each), packets and own walk: one frame of 307k rays 264 / 284
+// / 329 and 237 / 247 / 276; 6 views of 88k rays, packed, 627 / 713 / 981 and
+// 443 / 454 / 494; one frame of 858k rays 350 / 381 / 441 and 390 / 398 / 439.
+// At 11 leaves each one frame is as fast either way (233, 217).
+constexpr uint64_t kFewRays = 30000, kSomeRays = 250000, kSomeRaysMid = 600000, kSomeRaysDense = 1200000;
 
 // The configuration a launch runs with: a caller's own choice as it is; the
 // default one (precision apart) by groups, with the walk that suits the number
@@ -601,9 +606,9 @@ kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64
   kdgr_batch_config_default(&d);
   d.precision = c.precision;
   if (memcmp(&d, &c, sizeof d) != 0) return c;
-  const bool dense = s->n_pair_entries / 64u > s->n_gauss;
+  const bool mid = s->n_pair_entries / 16u > s->n_gauss, dense = s->n_pair_entries / 64u > s->n_gauss;
   d.schedule = kSchedGroups;
-  if (rays >= (dense ? kSomeRaysDense : kSomeRays)) return d;
+  if (rays >= (dense ? kSomeRaysDense : mid ? kSomeRaysMid : kSomeRays)) return d;
   d.min_blocks = 6;
   if (rays < kFewRays) {
     d.schedule = KDGR_SCHED_WARP_STRIPS;  // the finest shares: 10k rays 210 us, in groups 275

@@ -25,14 +25,17 @@ def _ball(n, radius, at):
     return (t * radius + np.asarray(at)).reshape(-1, 9).astype(np.float32)
 
 
-@pytest.mark.parametrize("mesh", ["none", "one", "ball8", "ball9", "ball64", "ball65", "ball330", "wall"])
-@pytest.mark.parametrize("w,h", [(120, 90), (643, 479)])
+@pytest.mark.parametrize("mesh", ["none", "one", "ball8", "ball9", "ball64", "ball65", "ball330", "mid_ball65", "wall"])
+@pytest.mark.parametrize("w,h", [(120, 90), (643, 479), (1011, 601)])
 def test_hybrid_matches_oracle(pkg, O, cuda, mesh, w, h):
     F = pkg.renderer
-    if mesh != "ball330" and w > 200:
+    if mesh not in ("ball330", "mid_ball65")[:2 if w < 900 else 1] and w > 200:
         pytest.skip("one mesh at the larger size")
-    rec = sc.cluster_shell(2500, seed=6, n_clusters=5)
+    mid = mesh.startswith("mid_")  # more than 16 leaves per Gaussian: small frames walk the tree as given
+    rec = sc.uniform_cube(2500, seed=9, scale=0.025) if mid else sc.cluster_shell(2500, seed=6, n_clusters=5)
     tree = pkg.kdtree.build(rec)
+    assert (tree.offsets.size > 16 * len(rec)) == mid
+    mesh = mesh.removeprefix("mid_")
     tris = {"none": np.zeros((0, 9), np.float32), "one": _ball(8, 0.5, (0, 0, 0.3))[:1],
             "wall": np.array([[-9, -9, -0.5, 9, -9, -0.5, 9, 9, -0.5], [-9, -9, -0.5, 9, 9, -0.5, -9, 9, -0.5]],
                              np.float32)}.get(mesh)

@@ -33,7 +33,7 @@ def walk_scene(pkg, cuda, request):
     return request.param, F.Scene(tree, rec, forms=F.FORM_EXACT), F.Scene(tree, rec)
 
 
-@pytest.mark.parametrize("w,h", [(1, 1), (9, 5), (173, 171), (251, 161), (263, 229), (331, 239), (641, 479), (1013, 991)])
+@pytest.mark.parametrize("w,h", [(1, 1), (9, 5), (191, 188), (251, 161), (331, 239), (331, 243), (641, 479), (701, 501), (1013, 991)])
 def test_walks_match_the_trace_kernel(pkg, cuda, walk_scene, w, h):
     name, exact_only, both = walk_scene
     if name == "many" and w * h > 200_000:

@@ -11,17 +11,19 @@ pytestmark = pytest.mark.gpu
 sc = importlib.import_module("3dgrt_kdtree_gb300.scenes")
 
 
-@pytest.fixture(scope="module", params=["few", "many"])
+@pytest.fixture(scope="module", params=["few", "mid", "many"])
 def scene(pkg, cuda, request):
     rec = (sc.cluster_shell(6000, seed=8, n_clusters=6) if request.param == "few"
-           else sc.uniform_cube(2500, seed=9, scale=0.12))
+           else sc.uniform_cube(2500, seed=9, scale=0.12 if request.param == "many" else 0.027))
     tree = pkg.kdtree.build(rec)
+    dup = tree.offsets.size / len(rec)
+    assert {"few": dup < 14, "mid": 18 < dup < 50, "many": dup > 64}[request.param]
     F = pkg.renderer
     return rec, tree, F.Scene(tree, rec, forms=F.FORM_FAST | F.FORM_PACKED)
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("sizes", [[(1, 1)], [(7, 3)], [(199, 149)], [(203, 151)], [(499, 499)], [(503, 509)],
+@pytest.mark.parametrize("sizes", [[(1, 1)], [(7, 3)], [(199, 149)], [(203, 151)], [(499, 499)], [(503, 509)], [(773, 773), (71, 9)], [(787, 781)],
                                    [(64, 48)] * 9, [(160, 120), (33, 17), (250, 190)],
                                    # groups of 2x2 and 2x4 blocks
                                    [(1203, 701)], [(1920, 1088), (17, 3), (331, 77), (1919, 1089)]])
