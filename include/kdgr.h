@@ -278,9 +278,11 @@ typedef struct {
                             small batches); needs KDGR_SCHED_WARP_STRIPS, warp packets and 8x4 tiles */
 } kdgr_batch_config;
 
-/* The defaults.  A launch with exactly these (precision apart) and fewer than
- * 250,000 rays is walked in the way that suits its size (independent rays, or
- * packets of four rays shared by eight lanes); the pixels are the same. */
+/* The defaults.  A launch with exactly these (precision apart) is dealt in
+ * groups of neighbouring blocks from the middle of each view outwards, and
+ * walked in the way that suits its size (packets of four rays shared by eight
+ * lanes, independent rays, packets of 32); any other configuration runs as it
+ * is written.  The pixels are the same. */
 void kdgr_batch_config_default(kdgr_batch_config* cfg);
 
 /* Render all views in one persistent launch.  Output pixel p of view v is at
