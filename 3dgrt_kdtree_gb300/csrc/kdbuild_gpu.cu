@@ -788,9 +788,10 @@ __device__ __forceinline__ void search_node(SearchMem<NT, CAP>& S, int tid, cons
     for (uint32_t i = tid; i < m; i += NT) same = same && S.cand[i] == c0;
     same = NT == 32 ? __all_sync(0xFFFFFFFFu, same) : __syncthreads_and(same);
     const Counts k0 = counts_at(a, ordz(p));
-    if (same && k0.planar == 0 && (double)score32(P, c, a, p, k0) * (1.0 + kMargin) < init) {
+    if (P.filter && same && k0.planar == 0 && (double)score32(P, c, a, p, k0) * (1.0 + kMargin) < init) {
       // one position is left and it certainly beats the leaf: its cost decides
-      // nothing more, and without planar IDs both sides score the same
+      // nothing more, and without planar IDs both sides score the same (the
+      // margin bounds positive scores only: other costs go to FP64)
       best_k = cand_key(a, p, 0);
     } else {
       for (uint32_t i = tid; i < m; i += NT) {
