@@ -89,6 +89,10 @@ constexpr uint32_t kFaces = 20;      // triangles per proxy: triangle t belongs 
 // 1e-6 of the FP64 one: a candidate that is not worse than the best in FP64 is
 // at most 2e-6 above it in FP32.  Twice that is allowed.
 constexpr float kMargin = 4e-6f;
+// That needs products clear of the denormals: a node of half surface area A
+// and N IDs takes an error of up to N * 2^-149 / A, below 1e-7 for any N that
+// fits 32 bits of triangles when A is at least this.
+constexpr float kThinArea = 1e-28f;
 
 struct Params {
   int max_level;
@@ -430,7 +434,9 @@ __device__ __forceinline__ Cell make_cell(const Params& P, const float* __restri
     ext[d] = c.hi[d] - c.lo[d];
   }
   const float area = (ext[0] * ext[1]) + (ext[1] * ext[2]) + (ext[0] * ext[2]);
-  c.rcp = 1.0f / area;
+  // below kThinArea the FP32 products round on the denormals' grid, outside
+  // kMargin: NaN scores discard nothing, FP64 decides
+  c.rcp = area < kThinArea ? __int_as_float(0x7fc00000) : 1.0f / area;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     c.am[a] = ext[(a + 1) % 3] + ext[(a + 2) % 3];

@@ -48,3 +48,19 @@ def test_last_position_close_to_the_leaf_cost(pkg, cuda):
     for bits in [few - 9, few - 3, few - 1, few, many, many + 1, many + 9]:
         cost = float(np.uint32(bits).view(np.float32))
         _same(pkg.kdtree.build(rec, device="cuda", isect_cost=cost, **flags), host(bits))
+
+
+@pytest.mark.parametrize("n,cost,free", [(1000, 10, 8), (3000, 40, 30)])
+@pytest.mark.parametrize("thin", [2e-39, 5e-39, 1e-38, 1e-33, 1e-30, 1e-26])
+def test_thin_scenes(pkg, cuda, n, cost, free, thin):
+    """Points along x whose SAH costs are equal to 1e-7 by construction (the
+    position of the k-th solves k p + (n - k)(1 - p) = cost), in a box `thin`
+    wide on the other axes: 4e-6 of FP32 slack is not enough where the half
+    area is a denormal's size."""
+    k = np.arange(n - cost + 1, n - cost + 1 + free)
+    x = np.concatenate([np.zeros(n - cost), (cost - n + k) / (2.0 * k - n), np.ones(cost - free)])
+    rec = _records(n)
+    rec[:, 0] = x.astype(np.float32)
+    rec[-1, 1:3] = np.float32(thin)
+    flags = dict(sah_mode=0)
+    _same(pkg.kdtree.build(rec, device="cuda", **flags), pkg.kdtree.build(rec, **flags))
