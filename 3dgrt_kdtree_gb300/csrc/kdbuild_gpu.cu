@@ -106,11 +106,27 @@ struct Params {
 // ------------------------------------------------------------ device buffers
 // Work memory comes from the library's pool of the device (device_pool.h): it
 // keeps what it has mapped while a build runs, where the device's default
-// pool hands memory back at every synchronisation of the level loop.
+// pool hands memory back at every synchronisation of the level loop.  The
+// stream and the entry into the pool end with the object, on every way out.
 struct Stream {
   cudaStream_t s = nullptr;
   cudaMemPool_t pool = nullptr;
+  int dev = -1;
   cudaError_t err = cudaSuccess;
+  Stream() {
+    check(cudaGetDevice(&dev));
+    if (err == cudaSuccess) check(work_pool_enter(dev, &pool));
+    if (err == cudaSuccess) check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  }
+  ~Stream() {
+    if (s) {
+      cudaStreamSynchronize(s);
+      cudaStreamDestroy(s);
+    }
+    if (pool) work_pool_leave(dev);
+  }
+  Stream(const Stream&) = delete;
+  Stream& operator=(const Stream&) = delete;
   void check(cudaError_t e) {
     if (err == cudaSuccess && e != cudaSuccess) err = e;
   }
@@ -1489,12 +1505,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
     return KDGR_ERR_LIMIT;
   }
   bool limit_hit = false;
-  Stream S;
-  int dev = 0;
-  S.check(cudaGetDevice(&dev));
-  if (S.err == cudaSuccess) S.check(work_pool_enter(dev, &S.pool));
-  const bool in_pool = S.pool != nullptr;
-  if (in_pool) S.check(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
+  Stream S;  // after the host arrays that its copies read and write: it ends before them
   const Params P{bp.max_level,  bp.force_split, bp.isect_cost,
                  bp.sah_mode,   bp.sort_cost,   (bp.isect_cost >= 0.0f && bp.sort_cost >= 0.0f) ? 1 : 0};
   uint32_t depth = 0, n_leaves = 0, max_leaf = 0, n_nodes = 0;
@@ -1718,11 +1729,6 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
     }
     S.check(cudaStreamSynchronize(S.s));
   }  // device buffers are returned to the pool here
-  if (S.s) {
-    cudaStreamSynchronize(S.s);
-    cudaStreamDestroy(S.s);
-  }
-  if (in_pool) work_pool_leave(dev);
   const cudaError_t e = S.err;
   if (limit_hit && e == cudaSuccess) return KDGR_ERR_LIMIT;
   if (e != cudaSuccess) {
