@@ -62,6 +62,7 @@
 #include <chrono>
 #include <cstdint>
 #include <cstring>
+#include <new>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -1425,11 +1426,12 @@ constexpr uint32_t kHostThreads = 8;
 template <typename F>
 void host_parallel(uint32_t n, F fn) {
   std::vector<std::thread> t;
-  t.reserve(n);
   uint32_t r = 1;
   try {
+    t.reserve(n);
     for (; r < n; ++r) t.emplace_back(fn, r);
   } catch (const std::system_error&) {  // no more threads: the rest runs here
+  } catch (const std::bad_alloc&) {     // nor memory for one
   }
   fn(0u);
   for (uint32_t k = r; k < n; ++k) fn(k);

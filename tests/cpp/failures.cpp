@@ -117,6 +117,7 @@ static int build_alloc(uint32_t n) {
 int main(int argc, char** argv) {
   const char* c = argc > 1 ? argv[1] : "";
   if (!std::strcmp(c, "build_alloc")) return build_alloc(2000);
+  if (!std::strcmp(c, "build_alloc_threads")) return build_alloc(70000);  // four host ranges
   std::fprintf(stderr, "unknown case %s\n", c);
   return 2;
 }

@@ -34,6 +34,6 @@ def program(pkg, tmp_path_factory):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("case", ["build_alloc"])
+@pytest.mark.parametrize("case", ["build_alloc", "build_alloc_threads"])
 def test_device_build_allocations(program, cuda, case):
     program(case)
