@@ -1456,7 +1456,6 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
                    std::string& err) {
   using clk = std::chrono::steady_clock;
   auto t0 = clk::now();
-  memset(out, 0, sizeof(*out));
   // the host arrays of the result: released on every exit but the last
   struct HostArrays {
     void *nodes = nullptr, *offsets = nullptr, *valid = nullptr;
@@ -1739,6 +1738,7 @@ int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_t
     return e == cudaErrorMemoryAllocation ? KDGR_ERR_OUT_OF_MEMORY : KDGR_ERR_CUDA;
   }
   if (!H.nodes || !H.offsets) throw std::bad_alloc();
+  memset(out, 0, sizeof(*out));
   out->nodes = static_cast<uint32_t*>(H.nodes);
   out->offsets = static_cast<uint32_t*>(H.offsets);
   out->valid = valid;

@@ -43,7 +43,7 @@ bool proxy_kiso(const float* g, float* k_iso);
 extern const float kIcosaVerts[12][3];
 extern const int kIcosaFaces[20][3];
 // The same build on the current CUDA device (kdbuild_gpu.cu); the arrays of
-// `out` are malloc'd on success and null otherwise.
+// `out` are malloc'd; `out` is written on success only.
 int build_tree_gpu(const float* gauss, uint32_t n, const BuildParams& bp, kdgr_tree* out, BuildStats* stats,
                    std::string& err);
 
