@@ -54,11 +54,17 @@ void work_pool_leave(int dev) {
   if (--P.users[dev] == 0) cudaMemPoolTrimTo(P.pool[dev], P.keep[dev]);
 }
 
-void work_pool_trim(int dev) {
-  if (dev < 0 || dev >= kMaxDevices) return;
+cudaError_t work_pool_release() {
   Pools& P = pools();
   std::lock_guard<std::mutex> lk(P.mu);
-  if (P.pool[dev] && P.users[dev] == 0) cudaMemPoolTrimTo(P.pool[dev], 0);
+  cudaError_t first = cudaSuccess;
+  for (int dev = 0; dev < kMaxDevices; ++dev) {
+    if (!P.pool[dev] || P.users[dev] != 0) continue;
+    const cudaError_t e = cudaMemPoolDestroy(P.pool[dev]);
+    if (first == cudaSuccess) first = e;
+    P.pool[dev] = nullptr;
+  }
+  return first;
 }
 
 }  // namespace kdgr

@@ -20,7 +20,8 @@ constexpr size_t kWorkPoolShare = 64;
 // so calls on several threads and streams may share the pool.
 cudaError_t work_pool_enter(int dev, cudaMemPool_t* out);
 void work_pool_leave(int dev);
-// Hand back what the pool of `dev` keeps (kdgr_shutdown).
-void work_pool_trim(int dev);
+// Hand back the pools that no call is in, on every device (kdgr_shutdown); the
+// next call on a device makes a new one.
+cudaError_t work_pool_release();
 
 }  // namespace kdgr

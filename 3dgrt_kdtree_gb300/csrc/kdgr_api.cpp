@@ -314,10 +314,8 @@ int kdgr_init(int device) {
 
 int kdgr_shutdown(void) {
   cudaError_t e = cudaDeviceSynchronize();
-  int dev = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = work_pool_release();
   if (e != cudaSuccess) return cuda_fail(e, "kdgr_shutdown");
-  work_pool_trim(dev);
   return KDGR_OK;
 }
 

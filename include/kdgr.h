@@ -174,7 +174,9 @@ typedef struct {
 
 /* Select the device the calling thread uses (initCuda, cudaRenderer.cu:2445). */
 int kdgr_init(int device);
-/* Synchronise the device; scenes must be destroyed by the caller. */
+/* Synchronise the device and give back the work memory that tree builds and
+ * scene uploads keep mapped between calls (at most 1/64 of a device's memory
+ * each, on every device); scenes must be destroyed by the caller. */
 int kdgr_shutdown(void);
 
 /* renderGaussianWithCudaSetup (cudaRenderer.cu:2557-2703): upload a tree in

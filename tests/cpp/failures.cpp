@@ -45,6 +45,53 @@ cudaError_t __wrap_cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t poo
   if (e == cudaSuccess) ++g_pool_blocks;
   return e;
 }
+// stand-ins for memory pools on devices that this machine need not have
+struct FakePool {
+  int dev;
+  size_t mapped;  // what the pool holds of its device
+};
+static bool g_fake_pools = false;
+static int g_device = 0;
+static std::vector<FakePool*> g_pools;
+cudaError_t __real_cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* props);
+cudaError_t __wrap_cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* props) {
+  if (!g_fake_pools) return __real_cudaMemPoolCreate(p, props);
+  FakePool* f = new FakePool{props->location.id, 1u << 20};
+  g_pools.push_back(f);
+  *p = reinterpret_cast<cudaMemPool_t>(f);
+  return cudaSuccess;
+}
+cudaError_t __real_cudaMemPoolSetAttribute(cudaMemPool_t p, cudaMemPoolAttr a, void* v);
+cudaError_t __wrap_cudaMemPoolSetAttribute(cudaMemPool_t p, cudaMemPoolAttr a, void* v) {
+  return g_fake_pools ? cudaSuccess : __real_cudaMemPoolSetAttribute(p, a, v);
+}
+cudaError_t __real_cudaMemPoolTrimTo(cudaMemPool_t p, size_t keep);
+cudaError_t __wrap_cudaMemPoolTrimTo(cudaMemPool_t p, size_t keep) {
+  if (!g_fake_pools) return __real_cudaMemPoolTrimTo(p, keep);
+  FakePool* f = reinterpret_cast<FakePool*>(p);
+  if (f->mapped > keep) f->mapped = keep;
+  return cudaSuccess;
+}
+cudaError_t __real_cudaMemPoolDestroy(cudaMemPool_t p);
+cudaError_t __wrap_cudaMemPoolDestroy(cudaMemPool_t p) {
+  if (!g_fake_pools) return __real_cudaMemPoolDestroy(p);
+  reinterpret_cast<FakePool*>(p)->mapped = 0;
+  return cudaSuccess;
+}
+cudaError_t __real_cudaMemGetInfo(size_t* free_bytes, size_t* total);
+cudaError_t __wrap_cudaMemGetInfo(size_t* free_bytes, size_t* total) {
+  if (!g_fake_pools) return __real_cudaMemGetInfo(free_bytes, total);
+  *free_bytes = *total = size_t(1) << 32;
+  return cudaSuccess;
+}
+cudaError_t __real_cudaGetDevice(int* dev);
+cudaError_t __wrap_cudaGetDevice(int* dev) {
+  if (!g_fake_pools) return __real_cudaGetDevice(dev);
+  *dev = g_device;
+  return cudaSuccess;
+}
+cudaError_t __real_cudaDeviceSynchronize();
+cudaError_t __wrap_cudaDeviceSynchronize() { return g_fake_pools ? cudaSuccess : __real_cudaDeviceSynchronize(); }
 cudaError_t __real_cudaFreeAsync(void* p, cudaStream_t s);
 cudaError_t __wrap_cudaFreeAsync(void* p, cudaStream_t s) {
   --g_pool_blocks;
@@ -114,10 +161,30 @@ static int build_alloc(uint32_t n) {
   return 0;
 }
 
+// kdgr_shutdown gives back every device's work pool, except one in use.
+static int shutdown_pools() {
+  g_fake_pools = true;
+  cudaMemPool_t p = nullptr;
+  for (int dev : {0, 1, 5}) REQUIRE(kdgr::work_pool_enter(dev, &p) == cudaSuccess);
+  kdgr::work_pool_leave(0);
+  kdgr::work_pool_leave(1);
+  REQUIRE(g_pools.size() == 3);
+  REQUIRE(kdgr_shutdown() == KDGR_OK);
+  REQUIRE(g_pools[0]->mapped == 0 && g_pools[1]->mapped == 0 && g_pools[2]->mapped > 0);
+  kdgr::work_pool_leave(5);
+  g_device = 1;
+  REQUIRE(kdgr_shutdown() == KDGR_OK);
+  for (const FakePool* f : g_pools) REQUIRE(f->mapped == 0);
+  REQUIRE(kdgr::work_pool_enter(1, &p) == cudaSuccess);
+  kdgr::work_pool_leave(1);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* c = argc > 1 ? argv[1] : "";
   if (!std::strcmp(c, "build_alloc")) return build_alloc(2000);
   if (!std::strcmp(c, "build_alloc_threads")) return build_alloc(70000);  // four host ranges
+  if (!std::strcmp(c, "shutdown_pools")) return shutdown_pools();
   std::fprintf(stderr, "unknown case %s\n", c);
   return 2;
 }

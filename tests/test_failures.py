@@ -10,7 +10,9 @@ import pytest
 
 from conftest import REPO
 
-WRAPPED = ["cudaStreamCreateWithFlags", "cudaStreamDestroy", "cudaMallocFromPoolAsync", "cudaFreeAsync"]
+WRAPPED = ["cudaStreamCreateWithFlags", "cudaStreamDestroy", "cudaMallocFromPoolAsync", "cudaFreeAsync",
+           "cudaMemPoolCreate", "cudaMemPoolSetAttribute", "cudaMemPoolTrimTo", "cudaMemPoolDestroy",
+           "cudaMemGetInfo", "cudaGetDevice", "cudaDeviceSynchronize"]
 
 
 @pytest.fixture(scope="module")
@@ -37,3 +39,7 @@ def program(pkg, tmp_path_factory):
 @pytest.mark.parametrize("case", ["build_alloc", "build_alloc_threads"])
 def test_device_build_allocations(program, cuda, case):
     program(case)
+
+
+def test_shutdown_gives_back_every_pool(program):
+    program("shutdown_pools")
