@@ -11,6 +11,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -195,53 +197,54 @@ int kdgr_secondary_create(const kdgr_sphere* spheres, int n_spheres, const float
     set_error("kdgr_secondary_create: at most 4096 spheres");
     return KDGR_ERR_LIMIT;
   }
-  std::vector<float> sph(10 * (size_t)n_spheres);
-  for (int i = 0; i < n_spheres; ++i) {
-    const kdgr_sphere& s = spheres[i];
-    if (!material_ok(s.material) || !(s.radius > 0.f)) {
-      set_error("kdgr_secondary_create: sphere " + std::to_string(i) + " has a bad radius or material");
-      return KDGR_ERR_INVALID_ARG;
-    }
-    memcpy(&sph[10 * i], s.center, 12);
-    sph[10 * i + 3] = s.radius;
-    material_words(s.material, &sph[10 * i + 4]);
-  }
+  // every host allocation before the first device one: a failure leaves nothing behind
+  std::vector<float> sph, groups;
+  std::unique_ptr<kdgr_secondary_s> s;
   float tm[6] = {0, 0, 0, 0, 0, 0};
-  if (n_tris > 0) {
-    if (!material_ok(*tri_material)) {
-      set_error("kdgr_secondary_create: bad mesh material");
-      return KDGR_ERR_INVALID_ARG;
+  try {
+    sph.resize(10 * (size_t)n_spheres);
+    for (int i = 0; i < n_spheres; ++i) {
+      const kdgr_sphere& sp = spheres[i];
+      if (!material_ok(sp.material) || !(sp.radius > 0.f)) {
+        set_error("kdgr_secondary_create: sphere " + std::to_string(i) + " has a bad radius or material");
+        return KDGR_ERR_INVALID_ARG;
+      }
+      memcpy(&sph[10 * i], sp.center, 12);
+      sph[10 * i + 3] = sp.radius;
+      material_words(sp.material, &sph[10 * i + 4]);
     }
-    material_words(*tri_material, tm);
+    if (n_tris > 0) {
+      if (!material_ok(*tri_material)) {
+        set_error("kdgr_secondary_create: bad mesh material");
+        return KDGR_ERR_INVALID_ARG;
+      }
+      material_words(*tri_material, tm);
+      groups = tri_groups(tri_verts, n_tris);
+    }
+    s.reset(new kdgr_secondary_s);
+  } catch (const std::bad_alloc&) {
+    set_error("kdgr_secondary_create: host allocation failed");
+    return KDGR_ERR_OUT_OF_MEMORY;
   }
-  kdgr_secondary_s* s = new kdgr_secondary_s;
   s->n_spheres = n_spheres;
   s->n_tris = n_tris;
+  auto upload = [](float** d, const float* h, size_t floats) {
+    const cudaError_t e = cudaMalloc(d, 4 * floats);
+    return e == cudaSuccess ? cudaMemcpy(*d, h, 4 * floats, cudaMemcpyHostToDevice) : e;
+  };
   cudaError_t e = cudaSuccess;
-  if (n_spheres > 0) {
-    e = cudaMalloc(&s->d_spheres, sph.size() * 4);
-    if (e == cudaSuccess) e = cudaMemcpy(s->d_spheres, sph.data(), sph.size() * 4, cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess && n_tris > 0) {
-    e = cudaMalloc(&s->d_tris, 36ull * n_tris);
-    if (e == cudaSuccess) e = cudaMemcpy(s->d_tris, tri_verts, 36ull * n_tris, cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess && n_tris > 0) {
-    const std::vector<float> groups = tri_groups(tri_verts, n_tris);
-    e = cudaMalloc(&s->d_groups, groups.size() * 4);
-    if (e == cudaSuccess) e = cudaMemcpy(s->d_groups, groups.data(), groups.size() * 4, cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&s->d_tri_material, sizeof tm);
-  if (e == cudaSuccess) e = cudaMemcpy(s->d_tri_material, tm, sizeof tm, cudaMemcpyHostToDevice);
+  if (n_spheres > 0) e = upload(&s->d_spheres, sph.data(), sph.size());
+  if (e == cudaSuccess && n_tris > 0) e = upload(&s->d_tris, tri_verts, 9ull * n_tris);
+  if (e == cudaSuccess && n_tris > 0) e = upload(&s->d_groups, groups.data(), groups.size());
+  if (e == cudaSuccess) e = upload(&s->d_tri_material, tm, 6);
   if (e != cudaSuccess) {
     cudaFree(s->d_spheres);
     cudaFree(s->d_tris);
     cudaFree(s->d_groups);
     cudaFree(s->d_tri_material);
-    delete s;
     return cuda_fail(e, "kdgr_secondary_create");
   }
-  *out = s;
+  *out = s.release();
   return KDGR_OK;
 }
 

@@ -45,6 +45,33 @@ cudaError_t __wrap_cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t poo
   if (e == cudaSuccess) ++g_pool_blocks;
   return e;
 }
+// device memory from the host (for cases that launch nothing), counted
+static bool g_fake_memory = false;
+static long g_blocks = 0;
+cudaError_t __real_cudaMalloc(void** p, size_t n);
+cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
+  if (!g_fake_memory) {
+    const cudaError_t e = __real_cudaMalloc(p, n);
+    if (e == cudaSuccess) ++g_blocks;
+    return e;
+  }
+  ++g_blocks;
+  *p = std::malloc(n);
+  return cudaSuccess;
+}
+cudaError_t __real_cudaFree(void* p);
+cudaError_t __wrap_cudaFree(void* p) {
+  if (p) --g_blocks;
+  if (!g_fake_memory) return __real_cudaFree(p);
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t __real_cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k);
+cudaError_t __wrap_cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
+  if (!g_fake_memory) return __real_cudaMemcpy(d, s, n, k);
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
 // stand-ins for memory pools on devices that this machine need not have
 struct FakePool {
   int dev;
@@ -180,11 +207,41 @@ static int shutdown_pools() {
   return 0;
 }
 
+// Every `new` of a secondary scene's creation fails once.
+static int secondary_alloc() {
+  g_fake_memory = true;
+  std::vector<float> tris(9 * 700);
+  for (size_t i = 0; i < tris.size(); ++i) tris[i] = (float)(i % 11) * 0.1f + (float)(i % 9 == 4);
+  kdgr_sphere sp[2];
+  REQUIRE(kdgr_demo_spheres(sp) == KDGR_OK);
+  int failed = 0;
+  for (long k = 0;; ++k) {
+    kdgr_secondary_t sec = nullptr;
+    int rc = -1;
+    g_new_left = k;
+    try {
+      rc = kdgr_secondary_create(sp, 2, tris.data(), 700, &sp[0].material, &sec);
+    } catch (...) {
+      rc = -2;
+    }
+    const bool fired = g_new_left.exchange(-1) < 0;
+    REQUIRE(rc != -2);  // an exception left the C entry
+    REQUIRE(rc == (fired ? KDGR_ERR_OUT_OF_MEMORY : KDGR_OK));
+    failed += fired;
+    if (rc == KDGR_OK) REQUIRE(kdgr_secondary_destroy(sec) == KDGR_OK);
+    REQUIRE(g_blocks == 0);
+    if (!fired) break;
+  }
+  REQUIRE(failed >= 3);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* c = argc > 1 ? argv[1] : "";
   if (!std::strcmp(c, "build_alloc")) return build_alloc(2000);
   if (!std::strcmp(c, "build_alloc_threads")) return build_alloc(70000);  // four host ranges
   if (!std::strcmp(c, "shutdown_pools")) return shutdown_pools();
+  if (!std::strcmp(c, "secondary_alloc")) return secondary_alloc();
   std::fprintf(stderr, "unknown case %s\n", c);
   return 2;
 }

@@ -12,7 +12,7 @@ from conftest import REPO
 
 WRAPPED = ["cudaStreamCreateWithFlags", "cudaStreamDestroy", "cudaMallocFromPoolAsync", "cudaFreeAsync",
            "cudaMemPoolCreate", "cudaMemPoolSetAttribute", "cudaMemPoolTrimTo", "cudaMemPoolDestroy",
-           "cudaMemGetInfo", "cudaGetDevice", "cudaDeviceSynchronize"]
+           "cudaMalloc", "cudaFree", "cudaMemcpy", "cudaMemGetInfo", "cudaGetDevice", "cudaDeviceSynchronize"]
 
 
 @pytest.fixture(scope="module")
@@ -43,3 +43,7 @@ def test_device_build_allocations(program, cuda, case):
 
 def test_shutdown_gives_back_every_pool(program):
     program("shutdown_pools")
+
+
+def test_secondary_scene_allocations(program):
+    program("secondary_alloc")
