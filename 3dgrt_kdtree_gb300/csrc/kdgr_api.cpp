@@ -128,10 +128,15 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   const bool exact = (forms & KDGR_FORM_EXACT) != 0, fast = (forms & KDGR_FORM_FAST) != 0,
              packed = (forms & KDGR_FORM_PACKED) != 0;
 
-  std::unique_ptr<kdgr_scene_s> s(new kdgr_scene_s);
+  struct Discard {  // a scene that is not handed out gives its arrays back
+    void operator()(kdgr_scene_s* p) const {
+      for (void* b : p->blocks) cudaFree(b);
+      delete p;
+    }
+  };
+  std::unique_ptr<kdgr_scene_s, Discard> s(new kdgr_scene_s);
   WorkMem W(nullptr);
   auto fail = [&](const char* where, cudaError_t e) {
-    for (void* p : s->blocks) cudaFree(p);
     return cuda_fail(e != cudaSuccess ? e : cudaErrorUnknown, (w + ": " + where).c_str());
   };
   auto host_check = [&]() {  // names what is wrong with the tree
@@ -220,7 +225,6 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   if (e != cudaSuccess) return fail("tree relayout", e);
   const bool fits = 2 * n_pairs <= 0xFFFFFFF0ull;
   if ((fast || packed) && !fits) {
-    for (void* p : s->blocks) cudaFree(p);
     set_error(w + ": more than 2^32 leaf entries after pair padding");
     return KDGR_ERR_LIMIT;
   }
@@ -328,16 +332,18 @@ int kdgr_scene_create(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   *out = nullptr;
   // the records go to the device as they are; the device packs every form
   float* d_rec = nullptr;
-  const int rc = scene_create_impl(
-      nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
-      [&](const float** d) {
-        cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d_rec, g, 256ull * n, cudaMemcpyHostToDevice, nullptr);
-        if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create: record upload");
-        *d = d_rec;
-        return (int)KDGR_OK;
-      },
-      out, "kdgr_scene_create");
+  const int rc = host_guard("kdgr_scene_create", [&] {
+    return scene_create_impl(
+        nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
+        [&](const float** d) {
+          cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
+          if (e == cudaSuccess) e = cudaMemcpyAsync(d_rec, g, 256ull * n, cudaMemcpyHostToDevice, nullptr);
+          if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create: record upload");
+          *d = d_rec;
+          return (int)KDGR_OK;
+        },
+        out, "kdgr_scene_create");
+  });
   if (d_rec) cudaFree(d_rec);
   return rc;
 }
@@ -349,13 +355,15 @@ int kdgr_scene_create_device(const uint32_t* nodes, uint32_t n_nodes, const uint
     return KDGR_ERR_INVALID_ARG;
   }
   *out = nullptr;
-  return scene_create_impl(
-      nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
-      [&](const float** d) {
-        *d = d_g;
-        return (int)KDGR_OK;
-      },
-      out, "kdgr_scene_create_device");
+  return host_guard("kdgr_scene_create_device", [&] {
+    return scene_create_impl(
+        nodes, n_nodes, offsets, n_offsets, aabb, n, flags,
+        [&](const float** d) {
+          *d = d_g;
+          return (int)KDGR_OK;
+        },
+        out, "kdgr_scene_create_device");
+  });
 }
 
 int kdgr_scene_destroy(kdgr_scene_t s) {

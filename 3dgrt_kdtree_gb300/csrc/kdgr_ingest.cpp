@@ -352,33 +352,31 @@ extern "C" int kdgr_scene_create_from_files(const char* ply_path, const char* kd
     return KDGR_ERR_INVALID_ARG;
   }
   *out = nullptr;
-  std::string err;
-  HostTree t;
-  int rc = read_kdt(kdt_path, t, err);
-  if (rc != KDGR_OK) {
-    set_error("kdgr_scene_create_from_files: " + err);
-    return rc;
-  }
-  uint32_t n = 0;
-  rc = read_ply_device(ply_path, nullptr, 0, &n, nullptr, err);  // vertex count from the header
-  if (rc != KDGR_OK) {
-    set_error("kdgr_scene_create_from_files: " + err);
-    return rc;
-  }
-  const uint32_t n_nodes = (uint32_t)(t.nodes.size() / 2), n_offsets = (uint32_t)t.offsets.size();
   float* d_rec = nullptr;
-  rc = scene_create_impl(
-      t.nodes.data(), n_nodes, t.offsets.data(), n_offsets, t.aabb, n, flags,
-      [&](const float** d) {
-        const cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
-        if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create_from_files: cudaMalloc");
-        uint32_t n2 = 0;
-        const int prc = read_ply_device(ply_path, d_rec, n, &n2, nullptr, err);
-        if (prc != KDGR_OK) set_error("kdgr_scene_create_from_files: " + err);
-        *d = d_rec;
-        return prc;
-      },
-      out, "kdgr_scene_create_from_files");
+  const int rc = host_guard("kdgr_scene_create_from_files", [&] {
+    std::string err;
+    HostTree t;
+    int rc = read_kdt(kdt_path, t, err);
+    uint32_t n = 0;
+    if (rc == KDGR_OK) rc = read_ply_device(ply_path, nullptr, 0, &n, nullptr, err);  // vertex count from the header
+    if (rc != KDGR_OK) {
+      set_error("kdgr_scene_create_from_files: " + err);
+      return rc;
+    }
+    const uint32_t n_nodes = (uint32_t)(t.nodes.size() / 2), n_offsets = (uint32_t)t.offsets.size();
+    return scene_create_impl(
+        t.nodes.data(), n_nodes, t.offsets.data(), n_offsets, t.aabb, n, flags,
+        [&](const float** d) {
+          const cudaError_t e = cudaMalloc(&d_rec, 256ull * n);
+          if (e != cudaSuccess) return cuda_fail(e, "kdgr_scene_create_from_files: cudaMalloc");
+          uint32_t n2 = 0;
+          const int prc = read_ply_device(ply_path, d_rec, n, &n2, nullptr, err);
+          if (prc != KDGR_OK) set_error("kdgr_scene_create_from_files: " + err);
+          *d = d_rec;
+          return prc;
+        },
+        out, "kdgr_scene_create_from_files");
+  });
   if (d_rec) cudaFree(d_rec);
   return rc;
 }

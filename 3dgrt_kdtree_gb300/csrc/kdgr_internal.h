@@ -2,6 +2,7 @@
 // of libkdgr (not part of the public C ABI; that is include/kdgr.h).
 #pragma once
 #include <cstdint>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -59,5 +60,16 @@ int validate_tree(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* offse
 
 // Thread-local last-error text behind kdgr_last_error().
 void set_error(const std::string& msg);
+
+// A C entry's body: a failed host allocation becomes its status.
+template <typename F>
+int host_guard(const char* who, F body) {
+  try {
+    return body();
+  } catch (const std::bad_alloc&) {
+    set_error(std::string(who) + ": host allocation failed");
+    return KDGR_ERR_OUT_OF_MEMORY;
+  }
+}
 
 }  // namespace kdgr

@@ -93,6 +93,7 @@ struct Slab {
   }
   cudaError_t make(std::vector<void*>& blocks) {
     void* base = nullptr;
+    blocks.reserve(blocks.size() + 1);
     const cudaError_t e = cudaMalloc(&base, bytes ? bytes : 256);
     if (e != cudaSuccess) return e;
     blocks.push_back(base);
@@ -123,6 +124,7 @@ struct WorkMem {
   T* take(size_t count) {
     if (err != cudaSuccess) return nullptr;
     void* p = nullptr;
+    ptrs.reserve(ptrs.size() + 1);
     err = cudaMallocFromPoolAsync(&p, count * sizeof(T) + 16, pool, st);
     if (err != cudaSuccess) return nullptr;
     ptrs.push_back(p);

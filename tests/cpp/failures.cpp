@@ -188,6 +188,43 @@ static int build_alloc(uint32_t n) {
   return 0;
 }
 
+// Every `new` of a scene's creation, in all forms, fails once.
+static int scene_alloc() {
+  const uint32_t n = 3000;
+  std::vector<float> g = records(n);
+  for (uint32_t i = 0; i < n; i += 16) g[64ull * i + 4] = 1e-6f;  // flagged in the packed form
+  kdgr_tree t;
+  REQUIRE(kdgr_init(0) == KDGR_OK);
+  REQUIRE(kdgr_build_tree(g.data(), n, nullptr, &t, nullptr) == KDGR_OK);
+  const long blocks = g_blocks, pool_blocks = g_pool_blocks;
+  int failed = 0;
+  for (long k = 0;; ++k) {
+    kdgr_scene_t scene = nullptr;
+    int rc = -1;
+    g_new_left = k;
+    try {
+      rc = kdgr_scene_create(t.nodes, t.n_nodes, t.offsets, t.n_offsets, t.aabb, g.data(), n,
+                             KDGR_FORM_EXACT | KDGR_FORM_FAST | KDGR_FORM_PACKED, &scene);
+    } catch (...) {
+      rc = -2;
+    }
+    const bool fired = g_new_left.exchange(-1) < 0;
+    REQUIRE(rc != -2);  // an exception left the C entry
+    REQUIRE(rc == (fired ? KDGR_ERR_OUT_OF_MEMORY : KDGR_OK));
+    failed += fired;
+    if (rc == KDGR_OK) REQUIRE(kdgr_scene_destroy(scene) == KDGR_OK);
+    REQUIRE(g_blocks == blocks && g_pool_blocks == pool_blocks);
+    if (!fired) break;
+  }
+  REQUIRE(failed > 10);
+  REQUIRE(kdgr_shutdown() == KDGR_OK);
+  uint64_t reserved = 1;
+  REQUIRE(pool_reserved(&reserved) == 0);
+  REQUIRE(reserved == 0);
+  kdgr_tree_free(&t);
+  return 0;
+}
+
 // kdgr_shutdown gives back every device's work pool, except one in use.
 static int shutdown_pools() {
   g_fake_pools = true;
@@ -242,6 +279,7 @@ int main(int argc, char** argv) {
   if (!std::strcmp(c, "build_alloc_threads")) return build_alloc(70000);  // four host ranges
   if (!std::strcmp(c, "shutdown_pools")) return shutdown_pools();
   if (!std::strcmp(c, "secondary_alloc")) return secondary_alloc();
+  if (!std::strcmp(c, "scene_alloc")) return scene_alloc();
   std::fprintf(stderr, "unknown case %s\n", c);
   return 2;
 }

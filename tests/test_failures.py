@@ -47,3 +47,8 @@ def test_shutdown_gives_back_every_pool(program):
 
 def test_secondary_scene_allocations(program):
     program("secondary_alloc")
+
+
+@pytest.mark.gpu
+def test_scene_allocations(program, cuda):
+    program("scene_alloc")
