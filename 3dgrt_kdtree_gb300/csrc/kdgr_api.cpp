@@ -111,6 +111,16 @@ kdgr::PlainView kdgr_scene_s::plain_view() const {
 
 namespace kdgr {
 
+// Whether the plain form's leaf order may take `bytes` of the current device:
+// above 64 MB at most an eighth of what is free, so that a scene does not fill
+// the device with arrays that it can render without (the 1M cluster scene:
+// 0.37 GB without them, 1.9 with).
+static bool plain_order_fits(size_t bytes) {
+  if (bytes <= (64u << 20)) return true;
+  size_t free_bytes = 0, total = 0;
+  return cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes <= free_bytes / 8;
+}
+
 // renderGaussianWithCudaSetup (cudaRenderer.cu:2557-2703) from device-resident
 // 64-float records: the tree is copied to the device as given, checked,
 // relaid out and expanded into padded leaf order there (scene_tree.cu), and
@@ -188,7 +198,7 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     A.add(s->d_nodes, n_nodes);
     A.add(s->d_test, kTestWords * (size_t)n);
   }
-  A.add(s->d_nodes_fast, n_nodes);
+  if (fast || packed) A.add(s->d_nodes_fast, n_nodes);
   if (fast || packed) A.add(s->d_opacity, n);
   if (packed) {
     A.add(s->d_sh_bf16, 6 * (size_t)n);
@@ -203,25 +213,12 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
   if (e == cudaSuccess) e = cudaMemsetAsync(s->d_status, 0, 4, W.st);
   if (e != cudaSuccess) return fail("tree arrays", e);
 
-  // per-Gaussian arrays, packed on the device
-  PackOut po{};
-  po.sh = s->d_sh;
-  po.test = s->d_test;
-  po.opacity = s->d_opacity;
-  po.sh_bf16 = s->d_sh_bf16;
-  if (packed) po.giscl = W.take<float>(3 * (size_t)n);
-  if (fast || exact) po.fast = W.take<float4>(3 * (size_t)n);
-  if (exact) po.tol = W.take<float2>(n);
-  if (packed) po.packed = W.take<uint32_t>(8 * (size_t)n);
-  if (packed) po.aniso = W.take<uint8_t>(n);
-  if (W.err != cudaSuccess) return fail("cudaMalloc (staging)", W.err);
-  e = launch_pack(d_g, n, inverted, po, W.st);
-  if (e != cudaSuccess) return fail("packing kernel", e);
-
-  // the relaid tree and its padded leaf order
+  // the relaid tree and its leaves' pairs
+  uint2* const relaid = fast || packed ? s->d_nodes_fast : W.take<uint2>(n_nodes);
   uint64_t *first = nullptr, n_pairs = 0;
-  e = tree_relayout(W, d_raw, L, s->d_nodes_fast);
-  if (e == cudaSuccess) e = tree_leaf_pairs(W, s->d_nodes_fast, L.n, &first, &n_pairs);
+  e = W.err;
+  if (e == cudaSuccess) e = tree_relayout(W, d_raw, L, relaid);
+  if (e == cudaSuccess) e = tree_leaf_pairs(W, relaid, L.n, &first, &n_pairs);
   if (e != cudaSuccess) return fail("tree relayout", e);
   const bool fits = 2 * n_pairs <= 0xFFFFFFF0ull;
   if ((fast || packed) && !fits) {
@@ -229,39 +226,48 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     return KDGR_ERR_LIMIT;
   }
   if (fast || packed) s->top_nodes = L.top_nodes;
-  auto leaf_arrays = [&](bool plain, Slab& P) {
-    P.add(s->d_pair_gid, 2 * n_pairs + 2);
-    if (fast || plain) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
-    if (plain) P.add(s->d_leaf_tol, n_pairs + 1);
-    if (plain) P.add(s->d_leaf_first, n_nodes);
-    return P.make(s->blocks);
-  };
-  Slab P;
-  bool plain = exact && fits;
-  if (plain || fast || packed) {
-    e = leaf_arrays(plain, P);
-    if (e != cudaSuccess && plain) {
-      // no room for the plain form's leaf order: its frames are then walked
-      // one thread per ray over the tree as given
-      cudaGetLastError();
-      plain = false;
-      s->d_pair_gid = nullptr;
-      s->d_leaf_pairs = s->d_leaf_tol = nullptr;
-      s->d_leaf_first = nullptr;
-      P = Slab();
-      e = fast || packed ? leaf_arrays(false, P) : cudaSuccess;
-    }
-    if (e != cudaSuccess) return fail("cudaMalloc (leaf order)", e);
+
+  // The plain form's leaf order only makes it faster: it is taken last, never
+  // at the cost of what a form cannot do without, and within bounds.
+  Slab X;
+  if (!(fast || packed)) {
+    X.add(s->d_nodes_fast, n_nodes);
+    X.add(s->d_pair_gid, 2 * n_pairs + 2);
   }
-  if (plain || fast || packed) {
+  if (!fast) X.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
+  X.add(s->d_leaf_tol, n_pairs + 1);
+  X.add(s->d_leaf_first, n_nodes);
+  bool plain = exact && fits && plain_order_fits(X.bytes);
+
+  // per-Gaussian arrays, packed on the device
+  PackOut po{};
+  po.sh = s->d_sh;
+  po.test = s->d_test;
+  po.opacity = s->d_opacity;
+  po.sh_bf16 = s->d_sh_bf16;
+  if (packed) po.giscl = W.take<float>(3 * (size_t)n);
+  if (fast) po.fast = W.take<float4>(3 * (size_t)n);
+  if (packed) po.packed = W.take<uint32_t>(8 * (size_t)n);
+  if (packed) po.aniso = W.take<uint8_t>(n);
+  if (W.err != cudaSuccess) return fail("cudaMalloc (staging)", W.err);
+  if (plain && !fast) po.fast = W.try_take<float4>(3 * (size_t)n);
+  if (plain) po.tol = W.try_take<float2>(n);
+  plain = plain && po.fast && po.tol;
+  e = launch_pack(d_g, n, inverted, po, W.st);
+  if (e != cudaSuccess) return fail("packing kernel", e);
+
+  // the fast forms' padded leaf order; the per-Gaussian rows are staging, the
+  // kernels read the leaf-order pairs
+  Slab P;
+  if (fast || packed) {
+    P.add(s->d_pair_gid, 2 * n_pairs + 2);
+    if (fast) P.add(s->d_leaf_pairs, 6 * (n_pairs + 1));
+    e = P.make(s->blocks);
+    if (e != cudaSuccess) return fail("cudaMalloc (leaf order)", e);
     s->n_pair_entries = (uint32_t)(2 * n_pairs);
-    e = tree_leaf_gids(W, s->d_nodes_fast, L.n, first, s->d_offsets, s->d_pair_gid);
-    // the per-Gaussian rows are staging: the kernels read the leaf-order pairs
-    if (e == cudaSuccess && s->d_leaf_pairs)
+    e = tree_leaf_gids(W, relaid, L.n, first, s->d_offsets, s->d_pair_gid);
+    if (e == cudaSuccess && fast)
       e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, po.fast, s->d_leaf_pairs, W.st);
-    if (e == cudaSuccess && s->d_leaf_tol)
-      e = build_leaf_tol(s->d_pair_gid, s->n_pair_entries, po.tol, s->d_leaf_tol, W.st);
-    if (e == cudaSuccess && s->d_leaf_first) e = tree_leaf_first(W, L, first, s->d_leaf_first);
     if (e != cudaSuccess) return fail("leaf order", e);
   }
   Slab Q;
@@ -297,9 +303,29 @@ int scene_create_impl(const uint32_t* nodes, uint32_t n_nodes, const uint32_t* o
     }
     if (e != cudaSuccess) return fail("packed upload", e);
   }
+  // without room for its leaf order the plain form walks one thread per ray
+  // over the tree as given
+  if (plain && X.make(s->blocks) != cudaSuccess) {
+    cudaGetLastError();
+    plain = false;
+  }
+  if (plain) {
+    e = cudaSuccess;
+    if (!(fast || packed)) {
+      s->n_pair_entries = (uint32_t)(2 * n_pairs);
+      e = tree_leaf_gids(W, relaid, L.n, first, s->d_offsets, s->d_pair_gid);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s->d_nodes_fast, relaid, 8ull * L.n, cudaMemcpyDeviceToDevice, W.st);
+    }
+    if (e == cudaSuccess && !fast)
+      e = build_leaf_pairs(s->d_pair_gid, s->n_pair_entries, po.fast, s->d_leaf_pairs, W.st);
+    if (e == cudaSuccess) e = build_leaf_tol(s->d_pair_gid, s->n_pair_entries, po.tol, s->d_leaf_tol, W.st);
+    if (e == cudaSuccess) e = tree_leaf_first(W, L, first, s->d_leaf_first);
+    if (e != cudaSuccess) return fail("plain leaf order", e);
+  }
   e = cudaStreamSynchronize(W.st);
   if (e != cudaSuccess) return fail("upload", e);
-  s->device_bytes = A.bytes + P.bytes + Q.bytes;
+  s->device_bytes = A.bytes + P.bytes + Q.bytes + (plain ? X.bytes : 0);
   *out = s.release();
   return KDGR_OK;
 }

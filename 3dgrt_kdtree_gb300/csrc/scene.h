@@ -130,6 +130,16 @@ struct WorkMem {
     ptrs.push_back(p);
     return static_cast<T*>(p);
   }
+  // null without memory for it, with no error left behind
+  template <typename T>
+  T* try_take(size_t count) {
+    T* const p = take<T>(count);
+    if (!p) {
+      err = cudaSuccess;
+      cudaGetLastError();
+    }
+    return p;
+  }
   WorkMem(const WorkMem&) = delete;
   WorkMem& operator=(const WorkMem&) = delete;
 };

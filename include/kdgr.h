@@ -162,6 +162,13 @@ typedef struct kdgr_scene_s* kdgr_scene_t;
 #define KDGR_FORM_FAST 0x20u      /* FP32 fast arrays (kdgr_render_fast, batches) */
 #define KDGR_FORM_PACKED 0x40u    /* BF16 SH + FP16 shape arrays (precision form) */
 /* flags without any KDGR_FORM_* bit materialise EXACT | FAST */
+/* KDGR_FORM_EXACT also keeps a leaf-order copy of what its candidate filter
+ * reads: 60 bytes per leaf entry (padded to pairs) and 12 per node, or 8 per
+ * entry and 4 per node beside KDGR_FORM_FAST, whose copy it shares (56 and 4
+ * beside KDGR_FORM_PACKED alone).  Above 64 MB it is made only within an eighth
+ * of the device's free memory, and only after everything else has been
+ * allocated; without it kdgr_render gives the same pixels, up to twice as slow.
+ * kdgr_scene_info.device_bytes tells what a scene took. */
 
 typedef struct {
   uint32_t n_nodes, n_offsets, n_gaussians;

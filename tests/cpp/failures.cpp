@@ -7,6 +7,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <cstdint>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -45,14 +46,32 @@ cudaError_t __wrap_cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t poo
   if (e == cudaSuccess) ++g_pool_blocks;
   return e;
 }
-// device memory from the host (for cases that launch nothing), counted
+// device memory, counted: from the host for cases that launch nothing, or from
+// a device that says it has no more than g_capacity bytes
 static bool g_fake_memory = false;
 static long g_blocks = 0;
+static size_t g_capacity = SIZE_MAX, g_taken = 0, g_free_reported = 0;
+static struct {
+  void* p;
+  size_t n;
+} g_sizes[64];  // the blocks handed out (no container: its own new would be counted)
+static void note_block(void* key, void* p, size_t n) {
+  for (auto& b : g_sizes)
+    if (b.p == key) {
+      g_taken += n - b.n;
+      b = {p, n};
+      return;
+    }
+}
 cudaError_t __real_cudaMalloc(void** p, size_t n);
 cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
   if (!g_fake_memory) {
+    if (n > g_capacity - g_taken) return cudaErrorMemoryAllocation;
     const cudaError_t e = __real_cudaMalloc(p, n);
-    if (e == cudaSuccess) ++g_blocks;
+    if (e == cudaSuccess) {
+      ++g_blocks;
+      note_block(nullptr, *p, n);
+    }
     return e;
   }
   ++g_blocks;
@@ -62,7 +81,10 @@ cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
 cudaError_t __real_cudaFree(void* p);
 cudaError_t __wrap_cudaFree(void* p) {
   if (p) --g_blocks;
-  if (!g_fake_memory) return __real_cudaFree(p);
+  if (!g_fake_memory) {
+    if (p) note_block(p, nullptr, 0);
+    return __real_cudaFree(p);
+  }
   std::free(p);
   return cudaSuccess;
 }
@@ -107,7 +129,11 @@ cudaError_t __wrap_cudaMemPoolDestroy(cudaMemPool_t p) {
 }
 cudaError_t __real_cudaMemGetInfo(size_t* free_bytes, size_t* total);
 cudaError_t __wrap_cudaMemGetInfo(size_t* free_bytes, size_t* total) {
-  if (!g_fake_pools) return __real_cudaMemGetInfo(free_bytes, total);
+  if (!g_fake_pools) {
+    const cudaError_t e = __real_cudaMemGetInfo(free_bytes, total);
+    if (g_free_reported) *free_bytes = g_free_reported;
+    return e;
+  }
   *free_bytes = *total = size_t(1) << 32;
   return cudaSuccess;
 }
@@ -225,6 +251,88 @@ static int scene_alloc() {
   return 0;
 }
 
+// One 96x64 frame of the plain form.
+static int frame(kdgr_scene_t scene, std::vector<float>& out) {
+  const kdgr_camera cam = {{0.f, 0.f, 1.6f}, {1.f, 0.f, 0.f}, {0.f, 1.f, 0.f}, {0.f, 0.f, 1.f}, 50.0, 1.5, 0.01};
+  float* d = nullptr;
+  out.assign(96 * 64 * 3, -1.f);
+  REQUIRE(cudaMalloc(&d, out.size() * 4) == cudaSuccess);
+  REQUIRE(kdgr_render(scene, &cam, 96, 64, d, nullptr, nullptr, nullptr, nullptr) == KDGR_OK);
+  REQUIRE(cudaMemcpy(out.data(), d, out.size() * 4, cudaMemcpyDeviceToHost) == cudaSuccess);
+  REQUIRE(cudaFree(d) == cudaSuccess);
+  return 0;
+}
+
+static int scene_bytes(const kdgr_tree& t, const std::vector<float>& g, uint32_t forms, uint64_t* bytes,
+                       std::vector<float>* img) {
+  kdgr_scene_t s = nullptr;
+  REQUIRE(kdgr_scene_create(t.nodes, t.n_nodes, t.offsets, t.n_offsets, t.aabb, g.data(), (uint32_t)(g.size() / 64),
+                            forms, &s) == KDGR_OK);
+  kdgr_scene_info i;
+  REQUIRE(kdgr_scene_info_get(s, &i) == KDGR_OK);
+  *bytes = i.device_bytes;
+  if (img && (forms & KDGR_FORM_EXACT) && frame(s, *img)) return 1;
+  REQUIRE(kdgr_scene_destroy(s) == KDGR_OK);
+  return 0;
+}
+
+// On a device with room for what a scene's forms cannot do without, the scene
+// is made whatever part of the plain form's leaf order would fit too.
+static int scene_room() {
+  const uint32_t n = 4000;
+  const std::vector<float> g = records(n);
+  kdgr_tree t;
+  REQUIRE(kdgr_init(0) == KDGR_OK);
+  REQUIRE(kdgr_build_tree(g.data(), n, nullptr, &t, nullptr) == KDGR_OK);
+  for (uint32_t other : {0u, KDGR_FORM_FAST, KDGR_FORM_PACKED, KDGR_FORM_FAST | KDGR_FORM_PACKED}) {
+    uint64_t without = 8ull * t.n_nodes + 80ull * n, full = 0, bytes = 0;
+    std::vector<float> want, got;
+    if (other) {
+      if (scene_bytes(t, g, other, &bytes, nullptr)) return 1;
+      without += bytes;
+    } else {
+      without += 4ull * t.n_offsets + 192ull * n + 4;
+    }
+    if (scene_bytes(t, g, KDGR_FORM_EXACT | other, &full, &want)) return 1;
+    const uint64_t besides = 256ull * n + 96 * 64 * 12 + 8192;  // records, frame, rounding of the arrays
+    REQUIRE(full > without + 100000);
+    for (int k = 0; k <= 8; ++k) {
+      g_capacity = without + besides + (full - without) * k / 8;
+      if (scene_bytes(t, g, KDGR_FORM_EXACT | other, &bytes, &got)) {
+        std::fprintf(stderr, "forms %x, step %d: %zu of %zu..%zu bytes\n", other, k, g_capacity, (size_t)without, (size_t)full);
+        return 1;
+      }
+      REQUIRE(bytes <= g_capacity && got == want);
+      REQUIRE(k < 8 || bytes == full);
+    }
+    g_capacity = SIZE_MAX;
+  }
+  kdgr_tree_free(&t);
+  return 0;
+}
+
+// A large leaf order stays within an eighth of the free memory.
+static int scene_share() {
+  const uint32_t n = 20000;
+  const std::vector<float> g = records(n);
+  std::vector<float> want, got;
+  kdgr_tree t;
+  REQUIRE(kdgr_init(0) == KDGR_OK);
+  REQUIRE(kdgr_build_tree_gpu(g.data(), n, nullptr, &t, nullptr) == KDGR_OK);
+  uint64_t full = 0, bytes = 0;
+  if (scene_bytes(t, g, KDGR_FORM_EXACT, &full, &want)) return 1;
+  const uint64_t order = 60ull * t.n_offsets;  // at least
+  REQUIRE(order > (100u << 20) && full > order);
+  g_free_reported = 8 * order - 1;
+  if (scene_bytes(t, g, KDGR_FORM_EXACT, &bytes, &got)) return 1;
+  REQUIRE(bytes < full - order && got == want);
+  g_free_reported = 12 * order;
+  if (scene_bytes(t, g, KDGR_FORM_EXACT, &bytes, &got)) return 1;
+  REQUIRE(bytes == full && got == want);
+  kdgr_tree_free(&t);
+  return 0;
+}
+
 // kdgr_shutdown gives back every device's work pool, except one in use.
 static int shutdown_pools() {
   g_fake_pools = true;
@@ -280,6 +388,8 @@ int main(int argc, char** argv) {
   if (!std::strcmp(c, "shutdown_pools")) return shutdown_pools();
   if (!std::strcmp(c, "secondary_alloc")) return secondary_alloc();
   if (!std::strcmp(c, "scene_alloc")) return scene_alloc();
+  if (!std::strcmp(c, "scene_room")) return scene_room();
+  if (!std::strcmp(c, "scene_share")) return scene_share();
   std::fprintf(stderr, "unknown case %s\n", c);
   return 2;
 }

@@ -52,3 +52,9 @@ def test_secondary_scene_allocations(program):
 @pytest.mark.gpu
 def test_scene_allocations(program, cuda):
     program("scene_alloc")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["scene_room", "scene_share"])
+def test_plain_leaf_order_takes_spare_memory_only(program, cuda, case):
+    program(case)
