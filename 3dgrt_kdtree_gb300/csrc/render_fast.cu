@@ -605,7 +605,10 @@ kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64
   kdgr_batch_config d;
   kdgr_batch_config_default(&d);
   d.precision = c.precision;
-  if (memcmp(&d, &c, sizeof d) != 0) return c;
+  kdgr_batch_config n = c;  // with the values that 0 stands for
+  if (n.hit_buffer == 0) n.hit_buffer = 4;
+  if (n.rays_per_warp == 0) n.rays_per_warp = 32;
+  if (memcmp(&d, &n, sizeof d) != 0) return c;
   const bool mid = s->n_pair_entries / 16u > s->n_gauss, dense = s->n_pair_entries / 64u > s->n_gauss;
   d.schedule = kSchedGroups;
   if (rays >= (dense ? kSomeRaysDense : mid ? kSomeRaysMid : kSomeRays)) return d;

@@ -198,6 +198,8 @@ cudaError_t launch_aniso_fp64(const float* src, uint32_t n, float4* table, cudaS
 int make_view_table(const kdgr_view* views, int n_views, std::vector<ViewDesc>& out, uint32_t totals[3]);
 int fill_view_table(const kdgr_view* views, int n_views, ViewDesc* out, uint32_t totals[3]);
 int check_batch_config(kdgr_scene_t s, const kdgr_batch_config& c);
+// The configuration a launch over `rays` rays runs with.
+kdgr_batch_config choose_walk(kdgr_scene_t s, const kdgr_batch_config& c, uint64_t rays);
 // Work-queue words of a batched launch: word 0 the global counter, words
 // 1..kMaxStrips the per-SM strip counters (zero before every launch).
 constexpr int kMaxStrips = 255;

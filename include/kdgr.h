@@ -287,8 +287,9 @@ typedef struct {
                             small batches); needs KDGR_SCHED_WARP_STRIPS, warp packets and 8x4 tiles */
 } kdgr_batch_config;
 
-/* The defaults.  A launch with exactly these (precision apart) is dealt in
- * groups of neighbouring blocks from the middle of each view outwards, and
+/* The defaults.  A launch with exactly these (precision apart; a 0 that stands
+ * for a default value is that value) is dealt in groups of neighbouring blocks
+ * from the middle of each view outwards, whatever its `schedule` says, and
  * walked in the way that suits its size (packets of four rays shared by eight
  * lanes, independent rays, packets of 32); any other configuration runs as it
  * is written.  The pixels are the same. */

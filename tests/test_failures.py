@@ -15,21 +15,26 @@ WRAPPED = ["cudaStreamCreateWithFlags", "cudaStreamDestroy", "cudaMallocFromPool
            "cudaMalloc", "cudaFree", "cudaMemcpy", "cudaMemGetInfo", "cudaGetDevice", "cudaDeviceSynchronize"]
 
 
-@pytest.fixture(scope="module")
-def program(pkg, tmp_path_factory):
+def link(source, exe, wrapped=()):
+    """A program of tests/cpp, linked with the library's objects."""
     B = importlib.import_module("3dgrt_kdtree_gb300.build")
-    units = [*B.CU_UNITS, *B.CPP_UNITS]
-    objs = [os.path.join(B.OUT_DIR, u + ".o") for u in units]
+    objs = [os.path.join(B.OUT_DIR, u + ".o") for u in [*B.CU_UNITS, *B.CPP_UNITS]]
     if not all(os.path.exists(o) for o in objs):
         B.build()
-    exe = tmp_path_factory.mktemp("failures") / "failures"
     home = B._cuda_home()
-    subprocess.run([os.path.join(home, "bin", "nvcc"), *B.ARCH, "-std=c++17", "-O1", "-I" + os.path.join(REPO, "include"),
-                    "-I" + B.CSRC, os.path.join(REPO, "tests", "cpp", "failures.cpp"), *objs,
-                    "-Xlinker", ",".join("--wrap=" + w for w in WRAPPED), "-lpthread", "-o", str(exe)], check=True)
+    wrap = ["-Xlinker", ",".join("--wrap=" + w for w in wrapped)] if wrapped else []
+    subprocess.run([os.path.join(home, "bin", "nvcc"), *B.ARCH, "-std=c++17", "-O1",
+                    "-I" + os.path.join(REPO, "include"), "-I" + B.CSRC,
+                    os.path.join(REPO, "tests", "cpp", source), *objs, *wrap, "-lpthread", "-o", str(exe)], check=True)
+    return str(exe)
+
+
+@pytest.fixture(scope="module")
+def program(pkg, tmp_path_factory):
+    exe = link("failures.cpp", tmp_path_factory.mktemp("failures") / "failures", WRAPPED)
 
     def run(case):
-        r = subprocess.run([str(exe), case], capture_output=True, text=True, timeout=300)
+        r = subprocess.run([exe, case], capture_output=True, text=True, timeout=300)
         assert r.returncode == 0, f"{case}: exit {r.returncode}\n{r.stdout}{r.stderr}"
 
     return run
