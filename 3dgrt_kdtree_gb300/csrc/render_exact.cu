@@ -570,13 +570,17 @@ cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamIn
     // outgrow L2 where the records themselves do not (100k overlapping
     // Gaussians, 175 leaves each: 980 MB against 8 MB), so the walk over the
     // tree as given is the faster one unless rays are few (20k rays: 427 us,
-    // 8 lanes per ray 198; 250k rays: 540, packets 950, own walk 560).
+    // 8 lanes per ray 198; 250k rays: 540, packets 950, own walk 560) or so many
+    // that a packet's rays share most leaves: 2.1M / 3.7M / 8.3M rays over 80k,
+    // 100k and 140k overlapping Gaussians (102, 176 and 371 leaves each) 1172 /
+    // 1826 / 3598, 1407 / 2190 / 4272 and 1989 / 3058 / 5967 us, packets 1185 /
+    // 1588 / 2760, 1471 / 1997 / 3423 and 2322 / 2996 / 4779.
     const bool copies = s.n_offsets / 64u > s.n_gauss;
     if (rays < 36000) return launch_plain<8, 6, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 80000) return launch_plain<4, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 350000) return launch_plain<1, 5, false>(plain, cam, W, H, rgb, alpha, depth, status, st);
     if (!copies && rays < 1000000) return launch_plain<1, 6, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
-    if (!copies) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
+    if (!copies || rays >= 3000000) return launch_plain<1, 8, true>(plain, cam, W, H, rgb, alpha, depth, status, st);
   }
   const dim3 grid((W + 15) / 16, (H + 7) / 8);
   // Traces filter the leaves' candidates too, unless the leaf copies are too
