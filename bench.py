@@ -214,6 +214,15 @@ def load_capture(key: str):
     return None
 
 
+def capture_key(config: str, cfg, default) -> str:
+    """Key of the capture that counts for a launch with `cfg`: the captures are
+    of the default configuration (precision apart); any other runs another
+    kernel and has none."""
+    key = f"{config}:{'packed' if cfg.precision else 'fp32'}"
+    a, b = cfg.as_dict(), default.as_dict()
+    return key if all(a[k] == b[k] for k in a if k != "precision") else key + ":other configuration"
+
+
 def roofline(key: str, ms_step: float, clk: dict, sms: int, alg_bytes: float, rays: int) -> dict:
     """Issue-rate bound of the batched kernel, plus its memory figures."""
     pk = peaks()
@@ -443,7 +452,7 @@ def run_ours(args, rank: int, world: int):
         "form": "batched persistent kernel, CUDA graph", "autotuned": cfg.as_dict(),
         "autotune_reranked": reranked,
         "e2e": {k: (round(v, 4) if isinstance(v, float) else v) for k, v in e2e.items()},
-        "roofline": roofline(f"{args.config}:{'packed' if precision else 'fp32'}", ms_step, clk, sms, alg_bytes,
+        "roofline": roofline(capture_key(args.config, cfg, F.BatchConfig.default()), ms_step, clk, sms, alg_bytes,
                              rays),
         "gpu_launches": args.steps,
         "clocks": clk,
