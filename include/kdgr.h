@@ -166,8 +166,8 @@ typedef struct kdgr_scene_s* kdgr_scene_t;
  * reads: 60 bytes per leaf entry (padded to pairs) and 12 per node, or 8 per
  * entry and 4 per node beside KDGR_FORM_FAST, whose copy it shares (56 and 4
  * beside KDGR_FORM_PACKED alone).  Above 64 MB it is made only within an eighth
- * of the device's free memory, and only after everything else has been
- * allocated; without it kdgr_render gives the same pixels, up to twice as slow.
+ * of the device's free memory, and only in what the rest of the scene leaves;
+ * without it kdgr_render gives the same pixels, up to twice as slow.
  * kdgr_scene_info.device_bytes tells what a scene took. */
 
 typedef struct {
