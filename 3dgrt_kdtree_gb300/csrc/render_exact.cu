@@ -13,17 +13,18 @@
 //
 // Two walks give these results:
 //   * over the tree as given, one thread per ray (k_render_exact), for traces,
-//     bounced rays and scenes without the leaf-order arrays: a warp covers an
-//     8x4 pixel tile; the 12-entry ring short stack (cudaRenderer.cu:184-210,
-//     restart from the root when it runs dry, :1694-1708) lives in shared
-//     memory laid out [slot][thread]; Gaussians are an 80-byte test record
+//     for scenes without the leaf-order arrays and for most frames over scenes
+//     whose leaf copies outgrow L2: a warp covers an 8x4 pixel tile; the
+//     12-entry ring short stack (cudaRenderer.cu:184-210, restart from the root
+//     when it runs dry, :1694-1708) lives in shared memory laid out
+//     [slot][thread]; Gaussians are an 80-byte test record
 //     (reciprocal scale and rotation rows precomputed by the same operations)
 //     and a separate 192-byte SH record read only for composited hits;
 //   * over the fast form's relaid tree and leaf-order pairs (k_render_plain,
 //     render_packet.cuh), as warp packets, independent rays or rays shared by
-//     lanes: candidates that certainly miss are discarded two at a time in
-//     FP32x2 arithmetic with a proven tolerance, the others take the same
-//     test as above.  What bounds it is the issue rate, as in the fast form:
+//     lanes, and by bounced rays (k_render_hybrid): candidates that certainly
+//     miss are discarded two at a time in FP32x2 arithmetic with a proven
+//     tolerance, the others take the same test as above.  What bounds it is the issue rate, as in the fast form:
 //     of 65.1k warp instructions per 8x4 tile (1280x720, 300k Gaussians) the
 //     filter on t* leaves 44k and that on the response 34k; 1080p on the 1M
 //     scene 4.26 -> 2.39 ms.
@@ -431,7 +432,8 @@ __device__ __forceinline__ SecHit intersect_secondary(const HybridView& M, const
 // packets, bounced ones independently.  A warp's lanes stay together through
 // the bounces; a lane whose ray has ended only waits.  What a pass does not
 // need (the running colour, throughput and the hit) waits in shared memory
-// meanwhile: in registers it spilled 600 bytes around the walk.
+// meanwhile: in registers it spilled 600 bytes around the walk (WALK 2 with its
+// 80 registers still spills 408 / 320 B of stores / loads).
 template <int WALK, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB)
     k_render_hybrid(ExactView S, PlainView L, CamInfo C, int W, int H, HybridView M, float* __restrict__ rgb,
@@ -586,7 +588,8 @@ cudaError_t launch_exact(const ExactView& s, const PlainView& plain, const CamIn
   // Traces filter the leaves' candidates too, unless the leaf copies are too
   // large for L2 (see above): 640x480, 100k / 10k Gaussians 1310 -> 864 us and
   // 503 -> 309; 256x256 500 -> 373 and 277 -> 199.  A bound of 4 blocks per SM
-  // leaves 128 registers and no spill; without it a 256x256 trace takes 397 / 214.
+  // leaves 128 registers (44 B of spills with the filter); without it a 256x256
+  // trace takes 397 / 214.
   if (trace && plain.leaf_tol && !(s.n_offsets / 64u > s.n_gauss))
     k_render_exact<8, true, true, 4><<<grid, kBlock, 0, st>>>(s, plain, cam, W, H, rgb, alpha, depth, trace, status);
   else if (trace)

@@ -25,8 +25,8 @@
 //     (fma/mul/add/sub.rn.f32x2), half the arithmetic instructions per test;
 //   * warp packets (the default traversal): the 32 rays of a warp tile walk
 //     the tree together, each with its own interval and decisions, so a
-//     leaf's records are warp-uniform loads (pkt_trace below);
-//   * lane groups (16 or 8 rays per warp): 2 or 4 lanes hold each ray and
+//     leaf's records are warp-uniform loads (pkt_trace in render_packet.cuh);
+//   * lane groups (16, 8 or 4 rays per warp): 2, 4 or 8 lanes hold each ray and
 //     split its leaves' candidate pairs, the group taking its hits in key
 //     order from the lanes' buffers -- shorter rays and more warps in flight
 //     for small batches, the same pixels bit for bit;
@@ -117,10 +117,16 @@ __device__ __forceinline__ uint32_t next_open_strip(const uint32_t* queue, uint3
 // contiguous strip of the block list per SM: every SM gets its share of the
 // expensive middle, the packets that start last are the short ones at the
 // border, and an SM's resident warps share a squarer piece of the image.  us
-// on a GB300, strips first: 640x480 of 100k Gaussians 628 -> 544, 1080p of 1M
-// 1768 -> 1693, 16 mixed views of 300k 10991 -> 10416, packed 4x1080p 7085 ->
-// 6926; smaller groups balance small launches better, larger ones share more
-// of the L1 (640x480: 2x1 541, 2x2 574, 2x4 592; mixed: 10582, 10453, 10393).
+// on a GB300, strips first, over cluster scenes: 640x480 of 100k Gaussians 613
+// -> 570, 1080p of 1M 1632 -> 1586, 16 mixed views of 300k 10989 -> 10491, packed
+// 4x1080p 6884 -> 6777.  One view of 270k to 1M rays over uniform scenes of 3k to
+// 20k Gaussians takes 0.87 to 0.93 of the strips' time (geometric means), of 60k
+// 1.00, cluster ones 0.92 to 1.01.  Two to nine views gain or lose by how their
+// blocks fall on the SMs, single launches between 0.74 and 1.32, on average 0.98
+// (cluster) and 1.02 (uniform); eleven other deals (group sizes, raster order,
+// contiguous runs) spread as much.  Smaller groups balance small launches
+// better, larger ones share more of the L1 (640x480: 2x1 541, 2x2 574, 2x4 592;
+// mixed: 10582, 10453, 10393).
 struct GroupShape {
   uint32_t lx, ly;  // blocks of a group, as powers of two
 };

@@ -499,7 +499,7 @@ __device__ __forceinline__ bool ray_init_plain(const PlainView& S, const F3 o, c
 
 // ------------------------------------------------------------ lane groups
 // With fewer than 32 rays per warp, each ray is held by a group of LPR
-// consecutive lanes (LPR = 2 or 4).  The lanes of a group hold the same ray
+// consecutive lanes (LPR = 2, 4 or 8).  The lanes of a group hold the same ray
 // state and take the same decisions; lane `sub` of the group tests pairs
 // sub, sub + LPR, ... of each leaf, and the group takes its hits in key
 // order from the lanes' buffers.  `mask` names the lanes that make the

@@ -333,7 +333,8 @@ int kdgr_batch_destroy(kdgr_batch_t batch);
  * configuration (pixel schedule, register cap, work items per queue
  * operation).
  * d_rgb must hold the views' pixels.  report (may be null) receives a JSON
- * line per variant. */
+ * line per variant: its configuration's fields and time.  The variant that
+ * equals the default is timed as the default runs (kdgr_batch_config_default). */
 int kdgr_autotune(kdgr_scene_t scene, const kdgr_view* views, int n_views, int precision, float* d_rgb,
                   kdgr_batch_config* best, char* report, int report_len);
 
@@ -347,7 +348,8 @@ int kdgr_autotune(kdgr_scene_t scene, const kdgr_view* views, int n_views, int p
 typedef struct kdgr_server_s* kdgr_server_t;
 
 typedef struct {
-  uint64_t hbm_budget_bytes;     /* resident scenes + output arena may not exceed this */
+  uint64_t hbm_budget_bytes;     /* resident scenes + output arena may not exceed this; the work memory that
+                                    the library keeps between uploads (kdgr_shutdown) is besides */
   uint64_t arena_bytes;          /* device output arena shared by in-flight requests */
   int32_t max_views_per_launch;  /* views per persistent launch (and per request) */
   int32_t lanes;                 /* launches in flight at once (streams), 1..8 */
